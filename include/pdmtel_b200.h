@@ -365,9 +365,9 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
 /* ---- Tuning options (no counterpart in the reference) ----
  * None of them changes a result (PD_OPT_STATIC_PRECOND: beyond the solve's
  * tolerance); they change launch shapes only.
- * PD_OPT_F64_LANES_BELOW: the FP64 Gauss-point force runs eight lanes per
- *   node (same arithmetic, same order) when the problem has fewer nodes than
- *   this, one thread per node otherwise.  Default 131072.
+ * PD_OPT_F64_LANES_BELOW: the FP64 force runs a warp per node (same
+ *   arithmetic, same order) when the problem has fewer nodes than this and
+ *   than 12288, eight lanes per node otherwise.  Default 131072.
  * PD_OPT_TILE: the node work order walks lattice tiles of 2^bx x 2^by x 2^bz
  *   nodes, value = bx | by << 8 | bz << 16 (1 <= bx <= 6, by, bz <= 6).
  *   Default 8 x 4 x 4.

@@ -526,6 +526,9 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
     for (int k = 0; k < P->num_materials; ++k) d.hasfail |= !(P->materials[k].ecrit >= 1e10);
     c->gch = hg;
     d.gc_host = c->gch.data();
+    d.gc_uniform = 1;
+    for (const pd::GaussConst& G : hg)
+        d.gc_uniform &= G.W == hg[0].W && G.dxe == hg[0].dxe && G.pw3 == hg[0].pw3;
     c->bdry_host.assign(N, 1.0);
     for (int k = 0; k < P->num_materials; ++k) c->mat_spring.push_back(P->materials[k].spring);
     d.nblk = nblk;

@@ -11,9 +11,11 @@
 #include <cmath>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "pd_internal.cuh"
+#include "pd_rn.cuh"
 #include "pd_stage.cuh"
 
 namespace pd {
@@ -54,190 +56,261 @@ __device__ __forceinline__ double extension(double x0, double x1, double x2, dou
     return q / (p + r);
 }
 
-// One thread per node.  FGI: the Gauss-point summation branch of
+// The force of one Gauss point on node i (CalcBondForceCCI, pdDataManager2.cpp:
+// 1293-1351) with the compiler's IEEE square roots and divisions: any operands.
+struct PointIn {
+    double bE, c, ecrit, delta, dxe, pw3;
+    bool cci_orig;
+};
+template <bool CCI, bool ENERGY, bool ACC>
+__device__ __noinline__ void point_any(const PointIn& P, double vol, double x0, double x1, double x2, double e0,
+                                       double e1, double e2, double* f) {
+    const double r = sqrt(x0 * x0 + x1 * x1 + x2 * x2);
+    const double y0 = x0 + e0, y1 = x1 + e1, y2 = x2 + e2;
+    const double pl = sqrt(y0 * y0 + y1 * y1 + y2 * y2);
+    const double beta = beta_factor(r, P.delta, P.dxe, P.cci_orig);
+    const double u = ACC ? extension(x0, x1, x2, e0, e1, e2, r, pl) : pl - r;
+    const double s = u / r;
+    f[0] = f[1] = f[2] = f[3] = 0.0;
+    if (u <= 0.0 || (u > 0.0 && s <= P.ecrit)) {
+        const double t = CCI ? P.bE * vol * beta * P.c * s : P.bE * beta * P.c * s;
+        f[0] = t * y0 / pl;
+        f[1] = t * y1 / pl;
+        f[2] = t * y2 / pl;
+        if (ENERGY) f[3] = P.bE * 0.5 * (0.5 * beta * (P.c / r) * u * u) * P.pw3;
+    }
+}
+
+// The limits of beta_factor and the reciprocal of its divisor.
+struct BetaIn {
+    double inner, outer, top, dxe, ydxe;  // ydxe = 1 / dxe rounded to nearest
+};
+__device__ __forceinline__ BetaIn beta_in(double delta, double dxe, bool cci_orig) {
+    BetaIn B;
+    B.inner = delta - 0.5 * dxe;
+    B.outer = cci_orig ? delta : delta + 0.5 * dxe;
+    B.top = delta + 0.5 * dxe;
+    B.dxe = dxe;
+    B.ydxe = 1.0 / dxe;
+    return B;
+}
+
+// v <= w for v, w >= 0 (finite): their bit patterns compare as integers, off
+// the FP64 pipe
+__device__ __forceinline__ bool le_pos(double v, double w) {
+    return __double_as_longlong(v) <= __double_as_longlong(w);
+}
+
+// point_any's arithmetic in the same order, straight-line: the square roots,
+// the two reciprocals and the six quotients of pd_rn.cuh.  ecp: the critical
+// stretch, +0 where it is negative or NaN.  False when an operand is outside
+// the range those are exact in (the caller then takes point_any).
+template <bool CCI, bool ENERGY, bool ACC>
+__device__ __forceinline__ bool point_rn(const BetaIn& B, double bE, double c, double ecp, double vol, double pw3,
+                                         double x0, double x1, double x2, double r2, double e0, double e1, double e2,
+                                         double& f0, double& f1, double& f2, double& el) {
+    const double y0 = x0 + e0, y1 = x1 + e1, y2 = x2 + e2;
+    const double p2 = y0 * y0 + y1 * y1 + y2 * y2;
+    double r, yr, pl, yp;
+    rn_sqrt_rcp(r2, r, yr);
+    rn_sqrt_rcp(p2, pl, yp);
+    const double u = ACC ? extension(x0, x1, x2, e0, e1, e2, r, pl) : pl - r;
+    const double s = rn_div(u, r, yr);
+    double beta = rn_div(B.top - r, B.dxe, B.ydxe);
+    beta = le_pos(r, B.outer) ? beta : 0.0;
+    beta = le_pos(r, B.inner) ? 1.0 : beta;
+    const double t = CCI ? bE * vol * beta * c * s : bE * beta * c * s;
+    const double n0 = t * y0, n1 = t * y1, n2 = t * y2;
+    // s <= ecrit as signed integers: true for every negative s
+    const bool on = __double_as_longlong(s) <= __double_as_longlong(ecp);
+    f0 = on ? (CCI ? rn_div_signed(n0, pl, yp) : rn_div(n0, pl, yp)) : 0.0;
+    f1 = on ? (CCI ? rn_div_signed(n1, pl, yp) : rn_div(n1, pl, yp)) : 0.0;
+    f2 = on ? (CCI ? rn_div_signed(n2, pl, yp) : rn_div(n2, pl, yp)) : 0.0;
+    if (ENERGY) el = on ? bE * 0.5 * (0.5 * beta * rn_div(c, r, yr) * u * u) * pw3 : 0.0;
+    const unsigned far = max(max(rn_dividend(n0), rn_dividend(n1)), max(rn_dividend(n2), ACC ? rn_dividend(u) : 0u));
+    return rn_range(r2) && rn_range(p2) && far < rn_span;
+}
+
+// L lanes per node.  FGI: the Gauss-point summation branch of
 // CalcBondBasedMotionRK4 (pdDataManager.cpp:1917-1962) with the per-point
 // CalcBondForceCCI (pdDataManager2.cpp:1293-1351).  CCI: the one-point
 // branch (pdDataManager.cpp:1818-1866).
-// Eight blocks per SM (64 registers, ~200 bytes of spill to L1): the
-// evaluation is a chain of IEEE square roots and divisions, so more resident
-// warps hide more of it (plate step 77 -> 64.5 ms; 6 blocks 70, 12 blocks 67).
-template <bool CCI, bool ENERGY, bool SFAC, bool ACC>
-__global__ void __launch_bounds__(128, 8) k_force_f64(Dev d, double dts) {
-    extern __shared__ GaussConst sg[];
-    for (int g = threadIdx.x; g < d.npt; g += blockDim.x) sg[g] = d.gc[g];
-    __syncthreads();
+//
+// Each lane evaluates one bond of its node (all its points, in point order)
+// and leaves the velocity increment (F + b) dt / rho, and the points' energy
+// terms, in shared memory; three lanes of the group (a fourth for the energy)
+// then add the round's L bonds in family order, so every sum has the
+// reference's terms in the reference's order, bit for bit.  Lanes past the
+// family's end store -0.0, which changes no sum.  UNI: the 2x2x2 rule with
+// equal weights, four points unrolled (their offsets are two per axis, so they
+// share squares), twice; else any rule, point by point.
+//
+// Bound by the FP64 pipe and the latency of its chains: 146 instructions per
+// evaluation, about 71 of them FP64 (pipe 53 % busy at 168 registers and three
+// blocks per SM; four blocks at 128 registers measured 1.54-1.57 ms, two at
+// 196 1.82, all eight points unrolled 1.67-1.91).  200x200x4 cracked plate, per
+// launch: 3.86 -> 1.50 ms against one thread per node with the compiler's
+// square roots and divisions (474 instructions); 20x10x10 bar with energies
+// 560 -> 62 us, 10x10x10 CCI cube 568 -> 17 us, where one thread (or eight
+// lanes) per node left a serial chain of 250 bonds on a few SMs.
+template <bool CCI, bool ENERGY, bool SFAC, bool ACC, bool UNI, int L>
+__global__ void __launch_bounds__(128, 3) k_force_f64(Dev d, double dts) {
+    constexpr int GS = 3 * L + 4;  // shared doubles per group: 4 more than its bonds, so that groups differ in bank
+    constexpr int G = 32 / L;
+    extern __shared__ double sh64[];
     const int64_t N = d.n;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (tid >= N) return;
-    const int64_t i = d.order[tid];
+    const int npt = CCI ? 1 : (UNI ? 8 : d.npt);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ql = lane % L, grp = lane / L;
+    const int ES = ENERGY ? L * npt + 2 : 0;  // shared doubles of a group's energy terms
+    double* sw = sh64 + warp * (G * (GS + ES)) + grp * GS;
+    double* se = sh64 + warp * (G * (GS + ES)) + G * GS + grp * ES;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
+    const bool live = slot < N;
+    const int64_t i = live ? d.order[slot] : 0;
     const MatDev Mi = d.mats[d.mat[i]];
-    const double rho = Mi.density;
+    const double rho = Mi.density, yrho = 1.0 / rho;
+    const bool rho_ok = rn_range(rho);
     const double b0 = Mi.grav[0] * rho, b1 = Mi.grav[1] * rho, b2 = Mi.grav[2] * rho;
-    const bool bci = d.bc[i] >= 0;
-    const double* src = bci ? d.U : d.us;
+    const double* src = (d.bc[i] >= 0) ? d.U : d.us;
     const double ui0 = src[i], ui1 = src[N + i], ui2 = src[2 * N + i];
     const double xi0 = d.x[i], xi1 = d.x[N + i], xi2 = d.x[2 * N + i];
     const double bEi = d.bdry[i];
     const double sfi = SFAC ? d.sfac[i] : 0.0;
-    double v0 = d.vbuf[i], v1 = d.vbuf[N + i], v2 = d.vbuf[2 * N + i];
-    double eacc = ENERGY ? d.eed[i] : 0.0;
-    const bool cci_orig = d.cci && !d.cci_mdf;
-    const int64_t pe = d.arow[i + 1];
-    for (int64_t p = d.arow[i]; p < pe; ++p) {
-        const int64_t j = d.acol[p];
-        const MatDev& Mj = d.mats[d.mat[j]];
-        const double ecrit = dmin(Mi.ecrit, Mj.ecrit);
-        double c = dmin(Mi.spring, Mj.spring);
-        if (SFAC) c = c * (0.5 * (sfi + d.sfac[j]));
-        const double bE = 0.5 * (bEi + d.bdry[j]);
-        const double xj0 = d.x[j], xj1 = d.x[N + j], xj2 = d.x[2 * N + j];
-        double F0 = 0.0, F1 = 0.0, F2 = 0.0;
-        if (CCI) {
-            const double* sj = (d.bc[j] >= 0) ? d.U : d.us;
-            const double xv0 = xj0 - xi0, xv1 = xj1 - xi1, xv2 = xj2 - xi2;
-            const double ev0 = sj[j] - ui0, ev1 = sj[N + j] - ui1, ev2 = sj[2 * N + j] - ui2;
-            const double r = sqrt(xv0 * xv0 + xv1 * xv1 + xv2 * xv2);
-            const double y0 = xv0 + ev0, y1 = xv1 + ev1, y2 = xv2 + ev2;
-            const double pl = sqrt(y0 * y0 + y1 * y1 + y2 * y2);
-            const double dxe = 2.0 * d.dx / 2.0;
-            const double beta = beta_factor(r, d.delta, dxe, cci_orig);
-            const double u = ACC ? extension(xv0, xv1, xv2, ev0, ev1, ev2, r, pl) : pl - r;
-            const double s = u / r;
-            if (u <= 0.0 || (u > 0.0 && s <= ecrit)) {
-                const double t = bE * d.vol_cci * beta * c * s;
-                F0 = t * y0 / pl;
-                F1 = t * y1 / pl;
-                F2 = t * y2 / pl;
-                if (ENERGY) eacc += bE * 0.5 * (0.5 * beta * (c / r) * u * u) * 1.0;
-            } else if (ENERGY) {
-                eacc += 0.0;
+    // lane ql < 3 sums component ql of the velocity, lane 3 the energy
+    double acc = -0.0;
+    if (live && ql < 3) acc = d.vbuf[(int64_t)ql * N + i];
+    if (ENERGY && live && ql == 3) acc = d.eed[i];
+    const int64_t row = d.arow[i];
+    const int cnt = live ? (int)(d.arow[i + 1] - row) : 0;
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    BetaIn B = beta_in(d.delta, CCI ? 2.0 * d.dx / 2.0 : d.gc[0].dxe, CCI && !d.cci_mdf);
+    double hlo = 0.0, hhi = 0.0, W = 0.0, pw3 = 1.0;
+    if (UNI) {
+        hlo = d.gc[0].hg[2];
+        hhi = d.gc[1].hg[2];
+        W = d.gc[0].W;
+        pw3 = d.gc[0].pw3;
+    }
+    for (int base = 0; base < most; base += L) {
+        const bool valid = base + ql < cnt;
+        double w0 = -0.0, w1 = -0.0, w2 = -0.0;
+        if (valid) {
+            const int64_t j = d.acol[row + base + ql];
+            double ecrit = Mi.ecrit, c = Mi.spring;
+            if (d.nmat > 1) {
+                const MatDev& Mj = d.mats[d.mat[j]];
+                ecrit = dmin(Mi.ecrit, Mj.ecrit);
+                c = dmin(Mi.spring, Mj.spring);
             }
-        } else {
-            for (int g = 0; g < d.npt; ++g) {
-                const GaussConst& G = sg[g];
-                const double xv0 = (G.hg[0] + xj0) - xi0;
-                const double xv1 = (G.hg[1] + xj1) - xi1;
-                const double xv2 = (G.hg[2] + xj2) - xi2;
-                const double* ugp = d.ug + (int64_t)(3 * g) * N + j;
-                const double ev0 = ugp[0] - ui0, ev1 = ugp[N] - ui1, ev2 = ugp[2 * N] - ui2;
-                const double r = sqrt(xv0 * xv0 + xv1 * xv1 + xv2 * xv2);
-                const double y0 = xv0 + ev0, y1 = xv1 + ev1, y2 = xv2 + ev2;
-                const double pl = sqrt(y0 * y0 + y1 * y1 + y2 * y2);
-                const double beta = beta_factor(r, d.delta, G.dxe, false);
-                const double u = ACC ? extension(xv0, xv1, xv2, ev0, ev1, ev2, r, pl) : pl - r;
-                const double s = u / r;
-                double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-                if (u <= 0.0 || (u > 0.0 && s <= ecrit)) {
-                    const double t = bE * beta * c * s;
-                    f0 = t * y0 / pl;
-                    f1 = t * y1 / pl;
-                    f2 = t * y2 / pl;
-                    if (ENERGY) eacc += bE * 0.5 * (0.5 * beta * (c / r) * u * u) * G.pw3;
-                } else if (ENERGY) {
-                    eacc += 0.0;
+            if (SFAC) c = c * (0.5 * (sfi + d.sfac[j]));
+            const double bE = 0.5 * (bEi + d.bdry[j]);
+            const double xj0 = d.x[j], xj1 = d.x[N + j], xj2 = d.x[2 * N + j];
+            const double ecp = ecrit > 0.0 ? ecrit : 0.0;
+            const bool c_ok = !ENERGY || rn_quotient_ok(c);
+            double F0 = 0.0, F1 = 0.0, F2 = 0.0;
+            if (CCI) {
+                const double* sj = (d.bc[j] >= 0) ? d.U : d.us;
+                const double x0 = xj0 - xi0, x1 = xj1 - xi1, x2 = xj2 - xi2;
+                const double e0 = sj[j] - ui0, e1 = sj[N + j] - ui1, e2 = sj[2 * N + j] - ui2;
+                double el = 0.0;
+                if (!point_rn<true, ENERGY, ACC>(B, bE, c, ecp, d.vol_cci, 1.0, x0, x1, x2, x0 * x0 + x1 * x1 + x2 * x2,
+                                                 e0, e1, e2, F0, F1, F2, el) || !c_ok) {
+                    double f[4];
+                    const PointIn P{bE, c, ecrit, d.delta, B.dxe, 1.0, !d.cci_mdf};
+                    point_any<true, ENERGY, ACC>(P, d.vol_cci, x0, x1, x2, e0, e1, e2, f);
+                    F0 = f[0];
+                    F1 = f[1];
+                    F2 = f[2];
+                    el = f[3];
                 }
-                F0 += G.W * f0;
-                F1 += G.W * f1;
-                F2 += G.W * f2;
-            }
-        }
-        v0 += (F0 + b0) * dts / rho;
-        v1 += (F1 + b1) * dts / rho;
-        v2 += (F2 + b2) * dts / rho;
-    }
-    d.vbuf[i] = v0;
-    d.vbuf[N + i] = v1;
-    d.vbuf[2 * N + i] = v2;
-    if (ENERGY) d.eed[i] = eacc;
-}
-
-// FGI with eight lanes per node: lane l evaluates the Gauss points l, l+8,
-// ... of every bond; the bond's force is then summed point by point in the
-// reference's order (F += W_g f_g for g = 0, 1, ...) by passing each lane's
-// product along the group with shuffles, so every lane holds the same F and
-// the velocity update (F + b) dt/rho per bond is the reference's, bit for bit.
-// More threads than k_force_f64 for the same work: the choice for lattices
-// too small to fill the GPU with one thread per node.
-template <bool ENERGY, bool SFAC, bool ACC>
-__global__ void __launch_bounds__(128) k_force_f64_lanes(Dev d, double dts) {
-    extern __shared__ GaussConst sg[];
-    for (int g = threadIdx.x; g < d.npt; g += blockDim.x) sg[g] = d.gc[g];
-    __syncthreads();
-    const int64_t N = d.n;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t slot = t >> 3;
-    const int lane = threadIdx.x & 7;
-    if (slot >= N) return;  // whole groups of 8 leave together
-    const unsigned gmask = 0xffu << (threadIdx.x & 24);
-    const int64_t i = d.order[slot];
-    const MatDev Mi = d.mats[d.mat[i]];
-    const double rho = Mi.density;
-    const double b0 = Mi.grav[0] * rho, b1 = Mi.grav[1] * rho, b2 = Mi.grav[2] * rho;
-    const bool bci = d.bc[i] >= 0;
-    const double* src = bci ? d.U : d.us;
-    const double ui0 = src[i], ui1 = src[N + i], ui2 = src[2 * N + i];
-    const double xi0 = d.x[i], xi1 = d.x[N + i], xi2 = d.x[2 * N + i];
-    const double bEi = d.bdry[i];
-    const double sfi = SFAC ? d.sfac[i] : 0.0;
-    double v0 = d.vbuf[i], v1 = d.vbuf[N + i], v2 = d.vbuf[2 * N + i];
-    double eacc = ENERGY ? d.eed[i] : 0.0;
-    const int npt = d.npt;
-    const int64_t pe = d.arow[i + 1];
-    for (int64_t p = d.arow[i]; p < pe; ++p) {
-        const int64_t j = d.acol[p];
-        const MatDev& Mj = d.mats[d.mat[j]];
-        const double ecrit = dmin(Mi.ecrit, Mj.ecrit);
-        double c = dmin(Mi.spring, Mj.spring);
-        if (SFAC) c = c * (0.5 * (sfi + d.sfac[j]));
-        const double bE = 0.5 * (bEi + d.bdry[j]);
-        const double xj0 = d.x[j], xj1 = d.x[N + j], xj2 = d.x[2 * N + j];
-        double F0 = 0.0, F1 = 0.0, F2 = 0.0;
-        for (int base = 0; base < npt; base += 8) {
-            const int g = base + lane;
-            double w0 = 0.0, w1 = 0.0, w2 = 0.0, el = 0.0;
-            if (g < npt) {
-                const GaussConst& G = sg[g];
-                const double xv0 = (G.hg[0] + xj0) - xi0;
-                const double xv1 = (G.hg[1] + xj1) - xi1;
-                const double xv2 = (G.hg[2] + xj2) - xi2;
-                const double* ugp = d.ug + (int64_t)(3 * g) * N + j;
-                const double ev0 = ugp[0] - ui0, ev1 = ugp[N] - ui1, ev2 = ugp[2 * N] - ui2;
-                const double r = sqrt(xv0 * xv0 + xv1 * xv1 + xv2 * xv2);
-                const double y0 = xv0 + ev0, y1 = xv1 + ev1, y2 = xv2 + ev2;
-                const double pl = sqrt(y0 * y0 + y1 * y1 + y2 * y2);
-                const double beta = beta_factor(r, d.delta, G.dxe, false);
-                const double u = ACC ? extension(xv0, xv1, xv2, ev0, ev1, ev2, r, pl) : pl - r;
-                const double s = u / r;
-                double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-                if (u <= 0.0 || (u > 0.0 && s <= ecrit)) {
-                    const double tt = bE * beta * c * s;
-                    f0 = tt * y0 / pl;
-                    f1 = tt * y1 / pl;
-                    f2 = tt * y2 / pl;
-                    if (ENERGY) el = bE * 0.5 * (0.5 * beta * (c / r) * u * u) * G.pw3;
+                if (ENERGY) se[ql] = el;
+            } else if (UNI) {
+                const double xa[2] = {(hlo + xj0) - xi0, (hhi + xj0) - xi0};
+                const double xb[2] = {(hlo + xj1) - xi1, (hhi + xj1) - xi1};
+                const double xc[2] = {(hlo + xj2) - xi2, (hhi + xj2) - xi2};
+                bool ok = c_ok;
+#pragma unroll 1
+                for (int a = 0; a < 2; ++a) {
+                    const double x0 = a ? xa[1] : xa[0];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int g = 4 * a + q;
+                        const double x1 = xb[q >> 1], x2 = xc[q & 1];
+                        const double* ugp = d.ug + (int64_t)(3 * g) * N + j;
+                        double f0, f1, f2, el;
+                        ok &= point_rn<false, ENERGY, ACC>(B, bE, c, ecp, 0.0, pw3, x0, x1, x2,
+                                                           x0 * x0 + x1 * x1 + x2 * x2, ugp[0] - ui0, ugp[N] - ui1,
+                                                           ugp[2 * N] - ui2, f0, f1, f2, el);
+                        F0 += W * f0;
+                        F1 += W * f1;
+                        F2 += W * f2;
+                        if (ENERGY) se[ql * 8 + g] = el;
+                    }
                 }
-                w0 = G.W * f0;
-                w1 = G.W * f1;
-                w2 = G.W * f2;
+                if (!ok) {
+                    const PointIn P{bE, c, ecrit, d.delta, B.dxe, pw3, false};
+                    F0 = F1 = F2 = 0.0;
+                    for (int g = 0; g < 8; ++g) {
+                        const double* ugp = d.ug + (int64_t)(3 * g) * N + j;
+                        double f[4];
+                        point_any<false, ENERGY, ACC>(P, 0.0, (d.gc[g].hg[0] + xj0) - xi0, (d.gc[g].hg[1] + xj1) - xi1,
+                                                      (d.gc[g].hg[2] + xj2) - xi2, ugp[0] - ui0, ugp[N] - ui1,
+                                                      ugp[2 * N] - ui2, f);
+                        F0 += W * f[0];
+                        F1 += W * f[1];
+                        F2 += W * f[2];
+                        if (ENERGY) se[ql * 8 + g] = f[3];
+                    }
+                }
+            } else {
+                for (int g = 0; g < npt; ++g) {
+                    const GaussConst& Gc = d.gc[g];
+                    const double x0 = (Gc.hg[0] + xj0) - xi0, x1 = (Gc.hg[1] + xj1) - xi1, x2 = (Gc.hg[2] + xj2) - xi2;
+                    const double* ugp = d.ug + (int64_t)(3 * g) * N + j;
+                    const double e0 = ugp[0] - ui0, e1 = ugp[N] - ui1, e2 = ugp[2 * N] - ui2;
+                    if (Gc.dxe != B.dxe) B = beta_in(d.delta, Gc.dxe, false);
+                    double f[4];
+                    f[3] = 0.0;
+                    if (!point_rn<false, ENERGY, ACC>(B, bE, c, ecp, 0.0, Gc.pw3, x0, x1, x2,
+                                                      x0 * x0 + x1 * x1 + x2 * x2, e0, e1, e2, f[0], f[1], f[2], f[3]) ||
+                        !c_ok) {
+                        const PointIn P{bE, c, ecrit, d.delta, Gc.dxe, Gc.pw3, false};
+                        point_any<false, ENERGY, ACC>(P, 0.0, x0, x1, x2, e0, e1, e2, f);
+                    }
+                    F0 += Gc.W * f[0];
+                    F1 += Gc.W * f[1];
+                    F2 += Gc.W * f[2];
+                    if (ENERGY) se[ql * npt + g] = f[3];
+                }
             }
-            const int cnt = npt - base < 8 ? npt - base : 8;
-            for (int l = 0; l < cnt; ++l) {
-                F0 += __shfl_sync(gmask, w0, l, 8);
-                F1 += __shfl_sync(gmask, w1, l, 8);
-                F2 += __shfl_sync(gmask, w2, l, 8);
-                if (ENERGY) eacc += __shfl_sync(gmask, el, l, 8);
+            const double n0 = (F0 + b0) * dts, n1 = (F1 + b1) * dts, n2 = (F2 + b2) * dts;
+            if (rho_ok && max(max(rn_dividend(n0), rn_dividend(n1)), rn_dividend(n2)) < rn_span) {
+                w0 = rn_div_signed(n0, rho, yrho);
+                w1 = rn_div_signed(n1, rho, yrho);
+                w2 = rn_div_signed(n2, rho, yrho);
+            } else {
+                w0 = n0 / rho;
+                w1 = n1 / rho;
+                w2 = n2 / rho;
             }
+        } else if (ENERGY) {
+            for (int g = 0; g < npt; ++g) se[ql * npt + g] = -0.0;
         }
-        v0 += (F0 + b0) * dts / rho;
-        v1 += (F1 + b1) * dts / rho;
-        v2 += (F2 + b2) * dts / rho;
+        sw[3 * ql] = w0;
+        sw[3 * ql + 1] = w1;
+        sw[3 * ql + 2] = w2;
+        __syncwarp();
+        if (ql < 3) {
+#pragma unroll 8
+            for (int q = 0; q < L; ++q) acc += sw[3 * q + ql];
+        } else if (ENERGY && ql == 3) {
+#pragma unroll 8
+            for (int q = 0; q < L * npt; ++q) acc += se[q];
+        }
+        __syncwarp();
     }
-    if (lane == 0) {
-        d.vbuf[i] = v0;
-        d.vbuf[N + i] = v1;
-        d.vbuf[2 * N + i] = v2;
-        if (ENERGY) d.eed[i] = eacc;
-    }
+    if (live && ql < 3) d.vbuf[(int64_t)ql * N + i] = acc;
+    if (ENERGY && live && ql == 3) d.eed[i] = acc;
 }
 
 // ----------------------------------------------------------------- gather
@@ -410,35 +483,43 @@ void launch_force_f64(const Dev& d, double dts, cudaStream_t s) {
         launch_ai_force(d, dts, s);
         return;
     }
-    const int bs = 128;
-    size_t sh = (size_t)d.npt * sizeof(GaussConst);
-    unsigned nb = blocks_for(d.n, bs);
+    // The 2x2x2 rule with equal weights takes the unrolled form.  A small
+    // problem gives a node a whole warp, so that the SMs fill; a larger one
+    // eight lanes, which waste fewer on a family's last round and add its bonds
+    // in fewer steps.  Measured, 8 against 32 lanes: 2,000 nodes 80 / 39 us,
+    // 8,192 145 / 119, 16,384 234 / 234, 32,768 424 / 458, 160,000 1501 / 1791;
+    // with energies 113 / 62 us at 2,000 and 563 / 743 at 32,768; the lighter
+    // CCI points 33 / 17 us at 1,000 and 78 / 94 at 19,800.
+    constexpr int64_t kWarpPerNodeBelow = 12288;
+    const bool uni = !d.cci && d.npt == 8 && d.gc_uniform;
+    const int lanes = d.n < std::min(d.f64_lanes_below, kWarpPerNodeBelow) ? 32 : 8;
+    const size_t warp_bytes =
+        sizeof(double) * (32 / lanes) * (3 * lanes + 4 + (d.energy ? lanes * (d.cci ? 1 : d.npt) + 2 : 0));
+    const int warps = std::max(1, std::min(4, (int)(200 * 1024 / warp_bytes)));
+    const unsigned nb = blocks_for(lanes * d.n, 32 * warps);
+    const size_t sh = warps * warp_bytes;
     const bool sf = d.sfac != nullptr;
-    if (!d.cci && d.npt >= 8 && d.n < d.f64_lanes_below) {
-        const unsigned nb8 = blocks_for(8 * d.n, bs);
-#define PD_FORCE_L(E, S)                                                                  \
-    do {                                                                                  \
-        if (d.acc_stretch) k_force_f64_lanes<E, S, true><<<nb8, bs, sh, s>>>(d, dts);    \
-        else k_force_f64_lanes<E, S, false><<<nb8, bs, sh, s>>>(d, dts);                 \
-    } while (0)
-        if (d.energy) { if (sf) PD_FORCE_L(true, true); else PD_FORCE_L(true, false); }
-        else { if (sf) PD_FORCE_L(false, true); else PD_FORCE_L(false, false); }
-#undef PD_FORCE_L
-        return;
-    }
-#define PD_FORCE(C, E, S)                                                     \
-    do {                                                                      \
-        if (d.acc_stretch) k_force_f64<C, E, S, true><<<nb, bs, sh, s>>>(d, dts); \
-        else k_force_f64<C, E, S, false><<<nb, bs, sh, s>>>(d, dts);          \
-    } while (0)
-    if (d.cci) {
-        if (d.energy) { if (sf) PD_FORCE(true, true, true); else PD_FORCE(true, true, false); }
-        else { if (sf) PD_FORCE(true, false, true); else PD_FORCE(true, false, false); }
-    } else {
-        if (d.energy) { if (sf) PD_FORCE(false, true, true); else PD_FORCE(false, true, false); }
-        else { if (sf) PD_FORCE(false, false, true); else PD_FORCE(false, false, false); }
-    }
-#undef PD_FORCE
+    auto go = [&](auto kernel) {
+        if (sh > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+        kernel<<<nb, 32 * warps, sh, s>>>(d, dts);
+    };
+    auto lanes_of = [&](auto C, auto E, auto S, auto A, auto Un) {
+        constexpr bool c = decltype(C)::value, e = decltype(E)::value, f = decltype(S)::value;
+        constexpr bool a = decltype(A)::value, u = decltype(Un)::value;
+        if (lanes == 32) go(k_force_f64<c, e, f, a, u, 32>);
+        else go(k_force_f64<c, e, f, a, u, 8>);
+    };
+    auto rule = [&](auto E, auto S, auto A) {
+        if (d.cci) lanes_of(std::true_type{}, E, S, A, std::false_type{});
+        else if (uni) lanes_of(std::false_type{}, E, S, A, std::true_type{});
+        else lanes_of(std::false_type{}, E, S, A, std::false_type{});
+    };
+    auto form = [&](auto E, auto S) {
+        if (d.acc_stretch) rule(E, S, std::true_type{});
+        else rule(E, S, std::false_type{});
+    };
+    if (d.energy) { if (sf) form(std::true_type{}, std::true_type{}); else form(std::true_type{}, std::false_type{}); }
+    else { if (sf) form(std::false_type{}, std::true_type{}); else form(std::false_type{}, std::false_type{}); }
 }
 
 void launch_gather_f64(const Dev& d, const double* us, cudaStream_t s) {

@@ -57,6 +57,7 @@ struct Dev {
     const double* sfac;       // [N] or nullptr
     const GaussConst* gc;     // [npt]
     const GaussConst* gc_host;  // host copy of gc (kernel-parameter constants)
+    int gc_uniform;           // every point has the same W, dxe and pw3
     // family (full) and active (unbroken) CSR
     const int64_t* frow;
     const int32_t* fcol;
@@ -102,7 +103,7 @@ struct Dev {
     const int32_t* lat;
     float c0, e0;             // spring and critical stretch when there is one material
     int acc_stretch;          // FP64 force: extension as (2 xi.eta + eta.eta)/(p + r)
-    int64_t f64_lanes_below;  // FGI FP64 force: eight lanes per node below this many nodes
+    int64_t f64_lanes_below;  // FP64 force: a warp per node below this many nodes (PD_OPT_F64_LANES_BELOW)
     int gather_per_point;     // FP32 gather: one thread per (node, point) instead of per 4 points
     // lattice box of the packed positions and the position -> node id map
     // (-1: no node); the FP32 force stages tile_x x tile_y x tile_z tiles in

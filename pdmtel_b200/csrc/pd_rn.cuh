@@ -1,0 +1,79 @@
+// Correctly rounded FP64 square root, reciprocal and quotient without
+// branches, for kernels whose results must be those of IEEE sqrt and / bit for
+// bit.  The compiler's own sequences test for special operands and branch on
+// every use, so several of them in one thread do not overlap; these are
+// straight lines of FMAs that interleave, one reciprocal serves several
+// quotients by the same divisor, and the caller tests the operands' range once
+// (rn_range, rn_quotient_ok) and takes the plain operators outside it.
+//
+// Square root: the coupled iteration of Goldschmidt (g -> sqrt a, h -> 1 / (2
+// sqrt a)) from a hardware seed of about 20 bits, twice, then one residual
+// correction g + h (a - g^2) (P. Markstein, "Software division and square
+// root using Goldschmidt's algorithms", RNC 2004).  Before the last rounding
+// the result is within 2^-100 of sqrt a (a in [1, 4)), so it can only round
+// to the wrong neighbour if a lies within 152 * 2^-106 of the square of a
+// midpoint: a finite list of operands (the solutions of m^2 = j modulo 2^54
+// for small |j|).
+//
+// Reciprocal and quotient: Newton's y + y (1 - b y) and Markstein's q + y (a -
+// b q) with q = a y (Muller et al., Handbook of Floating-Point Arithmetic,
+// section on division by Newton-Raphson with an FMA).  For b in [1, 2) the
+// reciprocal satisfies |y - 1/b| <= 2^-54 (1 + 2^-47).  If a/b is within reach
+// of a midpoint m, then q is one of the two neighbours of m because |a y -
+// a/b| < 2^-52, so |a - b q| is b 2^-53 to first order and the result before
+// rounding is within b 2^-107 of a/b, while a/b != m differs from m by at
+// least 2^-105 / b: it rounds to the right side for every b below 2 - 2^-46.
+// For b = 2 - 2^-52 the exact step from y = 1/2 ends on a tie that rounds to
+// 1/2 instead of 1/2 + 2^-53; the estimate before the last step therefore has
+// its lowest bit set.  tests/test_rn.py runs the operands that these bounds
+// leave open, and random ones, against IEEE results.
+#pragma once
+
+namespace pd {
+
+__device__ __forceinline__ double rn_pow2(double v, int e) {  // v 2^e, v and the result normal
+    return __hiloint2double(__double2hiint(v) + (e << 20), __double2loint(v));
+}
+
+// s = sqrt(a) and y = 1/s, both rounded to nearest (y: see above); a in
+// [2^-400, 2^400]
+__device__ __forceinline__ void rn_sqrt_rcp(double a, double& s, double& y) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
+    double g = a * y0, h = rn_pow2(y0, -1);
+    double e = fma(-g, h, 0.5);
+    g = fma(g, e, g);
+    h = fma(h, e, h);
+    e = fma(-g, h, 0.5);
+    g = fma(g, e, g);
+    h = fma(h, e, h);
+    s = fma(fma(-g, g, a), h, g);
+    y = __hiloint2double(__double2hiint(h) + (1 << 20), __double2loint(h) | 1);
+    y = fma(fma(-s, y, 1.0), y, y);
+}
+
+// a / b with y = 1/b; a zero or rn_quotient_ok (the quotient of a zero is +0)
+__device__ __forceinline__ double rn_div(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+// the same with the sign of a zero kept
+__device__ __forceinline__ double rn_div_signed(double a, double b, double y) {
+    const double q = rn_div(a, b, y);
+    return a == 0.0 ? a : q;
+}
+
+// whether a positive operand of rn_sqrt_rcp is in [2^-400, 2^400)
+__device__ __forceinline__ bool rn_range(double a) {
+    return (unsigned)__double2hiint(a) - (623u << 20) < (800u << 20);
+}
+// distance of |a| from the range [2^-500, 2^500) of dividends, as an unsigned
+// number: below rn_span inside; zeros count as inside
+constexpr unsigned rn_span = 1000u << 21;
+__device__ __forceinline__ unsigned rn_dividend(double a) {
+    const unsigned h = (unsigned)__double2hiint(a) << 1;
+    return (h | (unsigned)__double2loint(a)) ? h - (523u << 21) : 0u;
+}
+__device__ __forceinline__ bool rn_quotient_ok(double a) { return rn_dividend(a) < rn_span; }
+
+}  // namespace pd
