@@ -376,9 +376,9 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  * PD_OPT_PERSIST_FORCE_CHUNK / _GATHER_CHUNK: work items a block takes from
  *   the queue at a time (multiples of 128; defaults 128 and 256).
  * PD_OPT_STATIC_STENCIL: 1 (default) lets the static operator run as a
- *   lattice stencil when the problem is a complete box with one material,
- *   no broken bond and stencil-shaped families (checked); 0 keeps the
- *   family-list kernel.
+ *   lattice stencil when the problem is a complete box with one material and
+ *   stencil-shaped families (checked; broken bonds are subtracted from a list
+ *   of their own); 0 keeps the family-list kernel.
  * PD_OPT_GATHER_PER_POINT: 1 runs the FP32-form MLS gather with one thread
  *   per (node, Gauss point), 0 (default) with one per four points.
  * PD_OPT_FORCE_TILE: the FP32-form force (2x2x2 points, nodes on one

@@ -87,6 +87,10 @@ struct pd_ctx {
     int static_stencil_opt = 1;
     int static_precond = 1;        // block-Jacobi preconditioner of the static CG (PD_OPT_STATIC_PRECOND)
     double* bj_minv = nullptr;
+    double* cg_work = nullptr;     // [6][3N] vectors of pd_static_solve
+    double4 *fam_geo = nullptr, *fam_xm = nullptr;  // the family-list operator's node records
+    uint64_t fam_gen = ~0ull;
+    unsigned* dot_done = nullptr;  // finished blocks of a summing kernel (zero between launches)
     uint64_t bj_gen = ~0ull;
     int static_replacements = 0;
     bool sten_ok = false;
@@ -98,6 +102,10 @@ struct pd_ctx {
     double* sten_xm = nullptr;
     int4* sten_col = nullptr;
     double4* sten_colgeo = nullptr;
+    int32_t *sten_bnode = nullptr, *sten_bidx = nullptr;  // broken bonds of a cracked box (broken_prepare)
+    int64_t* sten_bptr = nullptr;
+    int2* sten_bent = nullptr;
+    double* sten_bfix = nullptr;
     int static_split = 4;           // split-form nodes per thread (PD_OPT_STATIC_SPLIT; 0: difference form)
     int64_t static_f32_below = 10;  // FP32 matvecs below relative residual 1/value (PD_OPT_STATIC_F32_BELOW)
     int4* nd_col = nullptr;
@@ -445,7 +453,7 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
         (rc = dalloc(c, &nblk, (size_t)N * d.bs)) || (rc = dalloc(c, &sblk, (size_t)N * 8)) ||
         (rc = dalloc(c, &order, N)) || (rc = dalloc(c, &eed, N)) ||
         (rc = dalloc(c, &red, 2 * N + 4 + 2 * 160)) || (rc = dalloc(c, &tdev, 1)) ||
-        (rc = dalloc(c, &c->dotpart, pd::kDotBlocks + 8)) || (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
+        (rc = dalloc(c, &c->dotpart, 2 * (N + 4096))) || (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
         return bail(rc);
     if (c->nslit) {
         double* sl = nullptr;
@@ -2020,8 +2028,8 @@ namespace {
 
 // Decides once per setup whether the static operator can run as a stencil:
 // every lattice position of a box holds one node, node id = x + nx (y + ny z),
-// one material, no broken family entry, and every node's family is the union
-// stencil clipped to the box (checked node by node on the downloaded family).
+// one material, and every node's family (broken entries included) is the union
+// stencil clipped to the box (checked node by node on the device).
 // The split form's tables (k_static_nd): the columns of the z-blocked
 // difference form sorted by half-height, (w, w oz spacing) per oz, and the
 // per-node diagonal blocks D_i built on the device from the same tables;
@@ -2092,71 +2100,106 @@ int split_prepare(pd_ctx* c, const std::vector<int4>& cols, const std::vector<do
     return PD_OK;
 }
 
-int static_prepare(pd_ctx* c) {
+// The broken family entries of a box whose full families are the stencil: the
+// nodes that have some, their entries as (neighbour, stencil slot; lut takes an
+// offset to its slot), and every node's place among them.
+int broken_prepare(pd_ctx* c, const int* lut) {
+    for (void* p : {(void*)c->sten_bnode, (void*)c->sten_bptr, (void*)c->sten_bent, (void*)c->sten_bidx,
+                    (void*)c->sten_bfix})
+        dfree(c, p);
+    c->sten_bnode = c->sten_bidx = nullptr;
+    c->sten_bptr = nullptr;
+    c->sten_bent = nullptr;
+    c->sten_bfix = nullptr;
+    c->sten.nbrk = 0;
+    if (c->Ha == c->H) return PD_OK;
+    const int64_t N = c->n;
+    int64_t* w = nullptr;  // [4][N + 1]: flags, counts and their scans
+    PD_TRY(dalloc(c, &w, 4 * (N + 1)));
+    int64_t *flag = w, *cnt = w + (N + 1), *fpos = w + 2 * (N + 1), *cpos = w + 3 * (N + 1);
+    auto done = [&](int rc) {
+        dfree(c, w);
+        return rc;
+    };
+    pd::launch_broken_counts(c->d, flag, cnt, c->stream);
+    if (pd::exclusive_scan_i64(flag, fpos, N, c->stream) != PD_OK ||
+        pd::exclusive_scan_i64(cnt, cpos, N, c->stream) != PD_OK)
+        return done(fail(PD_ERR_CUDA, "static operator: scan"));
+    int64_t nodes = 0;
+    if (cudaMemcpy(&nodes, fpos + N, sizeof(int64_t), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return done(fail(PD_ERR_CUDA, "static operator: broken bonds"));
+    int rc = PD_OK;
+    if ((rc = dalloc(c, &c->sten_bnode, nodes)) || (rc = dalloc(c, &c->sten_bptr, nodes + 1)) ||
+        (rc = dalloc(c, &c->sten_bent, c->H - c->Ha)) || (rc = dalloc(c, &c->sten_bidx, N)) ||
+        (rc = dalloc(c, &c->sten_bfix, 3 * nodes)))
+        return done(rc);
+    pd::launch_broken_fill(c->d, lut, flag, fpos, cpos, c->sten_bnode, c->sten_bptr, c->sten_bent, c->sten_bidx,
+                           c->stream);
+    const int64_t total = c->H - c->Ha;
+    if (cudaMemcpyAsync(c->sten_bptr + nodes, &total, sizeof(int64_t), cudaMemcpyHostToDevice, c->stream) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess)
+        return done(fail(PD_ERR_CUDA, "static operator: broken bonds"));
+    c->sten.bnode = c->sten_bnode;
+    c->sten.bptr = c->sten_bptr;
+    c->sten.bent = c->sten_bent;
+    c->sten.bidx = c->sten_bidx;
+    c->sten.bfix = c->sten_bfix;
+    c->sten.nbrk = (int)nodes;
+    return done(PD_OK);
+}
+
+int stencil_prepare(pd_ctx* c) {
     if (c->sten_gen == c->generation) return PD_OK;
     c->sten_ok = false;
     c->sten_gen = c->generation;
     if (!c->static_stencil_opt || c->d.multimat || c->d.nmat != 1 || c->n == 0) return PD_OK;
     const int64_t N = c->n;
-    std::vector<int32_t> lat;
-    if (!lattice_positions(c->coords, N, c->d.dx, lat)) return PD_OK;
-    int64_t dims[3] = {0, 0, 0};
-    for (int64_t i = 0; i < N; ++i) {
-        dims[0] = std::max<int64_t>(dims[0], (lat[i] & 2047) + 1);
-        dims[1] = std::max<int64_t>(dims[1], ((lat[i] >> 11) & 2047) + 1);
-        dims[2] = std::max<int64_t>(dims[2], (lat[i] >> 22) + 1);
-    }
-    if (dims[0] * dims[1] * dims[2] != N) return PD_OK;
-    for (int64_t i = 0; i < N; ++i) {
-        const int64_t l = (lat[i] & 2047) + dims[0] * (((lat[i] >> 11) & 2047) + dims[1] * (lat[i] >> 22));
-        if (l != i) return PD_OK;
-    }
-    if (c->Ha != c->H) return PD_OK;  // broken entries
-    std::vector<int64_t> rp(N + 1);
-    std::vector<int32_t> col(std::max<int64_t>(c->H, 1));
-    PD_CUDA_TRY(cudaMemcpy(rp.data(), c->d.frow, sizeof(int64_t) * (N + 1), cudaMemcpyDeviceToHost));
-    PD_CUDA_TRY(cudaMemcpy(col.data(), c->d.fcol, sizeof(int32_t) * c->H, cudaMemcpyDeviceToHost));
-    const int64_t nx = dims[0], ny = dims[1], nz = dims[2];
-    auto pos = [&](int64_t i, int64_t* q) {
-        q[0] = i % nx;
-        q[1] = (i / nx) % ny;
-        q[2] = i / (nx * ny);
+    const int64_t nx = c->d.lat_nx, ny = c->d.lat_ny, nz = c->d.lat_nz;
+    if (!c->d.lat || nx * ny * nz != N) return PD_OK;
+    // the offsets of all family entries over [-64, 63]^3, the numbering, and
+    // every family's size against the offsets that stay in the box
+    constexpr int kSpan = 128 * 128 * 128;
+    // map [kSpan]: seen (1) or not, then slot numbers; the error word and the
+    // number of offsets; the offset list
+    int* map = nullptr;
+    PD_TRY(dalloc(c, &map, kSpan + 4 + 4 * pd::kMaxStencil));
+    int* err = map + kSpan;
+    int4* dlist = reinterpret_cast<int4*>(map + kSpan + 4);
+    auto done = [&](int rc) {
+        dfree(c, map);
+        return rc;
     };
-    // union of the offsets, keyed (ox, oy, oz) in [-64, 63]^3
-    std::vector<uint8_t> seen(128 * 128 * 128, 0);
+    int found[2];
+    std::vector<int4> list(pd::kMaxStencil);
     std::vector<std::array<int, 3>> offs;
-    for (int64_t i = 0; i < N; ++i) {
-        int64_t qi[3], qj[3];
-        pos(i, qi);
-        for (int64_t p = rp[i]; p < rp[i + 1]; ++p) {
-            pos(col[p], qj);
-            int o[3];
-            for (int a = 0; a < 3; ++a) {
-                o[a] = (int)(qj[a] - qi[a]);
-                if (o[a] < -64 || o[a] > 63) return PD_OK;
-            }
-            const int key = ((o[0] + 64) << 14) | ((o[1] + 64) << 7) | (o[2] + 64);
-            if (!seen[key]) {
-                seen[key] = 1;
-                offs.push_back({o[0], o[1], o[2]});
-            }
-        }
-    }
-    if (offs.empty() || offs.size() > (size_t)pd::kMaxStencil) return PD_OK;
-    // every node's family has exactly the offsets that stay in the box
-    for (int64_t i = 0; i < N; ++i) {
-        int64_t qi[3];
-        pos(i, qi);
-        int64_t in = 0;
-        for (const auto& o : offs)
-            if (qi[0] + o[0] >= 0 && qi[0] + o[0] < nx && qi[1] + o[1] >= 0 && qi[1] + o[1] < ny &&
-                qi[2] + o[2] >= 0 && qi[2] + o[2] < nz)
-                ++in;
-        if (in != rp[i + 1] - rp[i]) return PD_OK;
-    }
+    if (cudaMemsetAsync(map, 0, sizeof(int) * (kSpan + 4), c->stream) != cudaSuccess)
+        return done(fail(PD_ERR_CUDA, "static operator: offsets"));
+    pd::launch_box_offsets(c->d, map, err, dlist, c->stream);
+    if (cudaMemcpyAsync(found, err, sizeof(found), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
+        cudaMemcpyAsync(list.data(), dlist, sizeof(int4) * list.size(), cudaMemcpyDeviceToHost, c->stream) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess)
+        return done(fail(PD_ERR_CUDA, "static operator: offsets"));
+    if (found[0] || found[1] > pd::kMaxStencil) return done(PD_OK);
+    for (int k = 0; k < found[1]; ++k) offs.push_back({list[k].x, list[k].y, list[k].z});
+    if (offs.empty() || offs.size() > (size_t)pd::kMaxStencil) return done(PD_OK);
     std::sort(offs.begin(), offs.end(), [&](const std::array<int, 3>& a, const std::array<int, 3>& b) {
         return a[0] + nx * (a[1] + ny * a[2]) < b[0] + nx * (b[1] + ny * b[2]);
     });
+    {
+        list.clear();
+        for (const auto& o : offs) list.push_back(make_int4(o[0], o[1], o[2], 0));
+        if (cudaMemcpyAsync(dlist, list.data(), sizeof(int4) * list.size(), cudaMemcpyHostToDevice, c->stream) !=
+            cudaSuccess)
+            return done(fail(PD_ERR_CUDA, "static operator: offsets"));
+        pd::launch_box_check(c->d, dlist, (int)list.size(), map, err, c->stream);
+        int bad = 0;
+        if (cudaMemcpyAsync(&bad, err, sizeof(int), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
+            cudaStreamSynchronize(c->stream) != cudaSuccess)
+            return done(fail(PD_ERR_CUDA, "static operator: families"));
+        if (bad) return done(PD_OK);
+    }
     const int ns = (int)offs.size();
     std::vector<int4> off(ns);
     std::vector<double4> geo(ns);
@@ -2197,7 +2240,7 @@ int static_prepare(pd_ctx* c) {
     if (!c->sten_off) {
         PD_TRY(dalloc(c, &c->sten_off, pd::kMaxStencil));
         PD_TRY(dalloc(c, &c->sten_geo, pd::kMaxStencil));
-        PD_TRY(dalloc(c, &c->sten_pmask, N));
+        if (!c->sten_pmask) PD_TRY(dalloc(c, &c->sten_pmask, N));
         PD_TRY(dalloc(c, &c->sten_xm, 3 * N));
         PD_TRY(dalloc(c, &c->sten_col, pd::kMaxStencil));
         PD_TRY(dalloc(c, &c->sten_colgeo, (size_t)pd::kMaxStencil * 9));
@@ -2214,17 +2257,61 @@ int static_prepare(pd_ctx* c) {
     PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->sten = pd::StencilDev{(int)nx, (int)ny, (int)nz, ns, radius, c->sten_off, c->sten_geo, c->sten_pmask,
                              c->sten_xm, (int)cols.size(), rz, c->sten_col, c->sten_colgeo};
+    PD_TRY(broken_prepare(c, map));
     PD_TRY(split_prepare(c, cols, colgeo));
     c->sten_ok = true;
+    return done(PD_OK);
+}
+
+// The node records of the family-list operator (its matvec, and every
+// problem's right-hand side).
+int family_prepare(pd_ctx* c) {
+    if (!c->dot_done) {
+        PD_TRY(dalloc(c, &c->dot_done, 1));
+        PD_CUDA_TRY(cudaMemsetAsync(c->dot_done, 0, sizeof(unsigned), c->stream));
+    }
+    if (c->fam_gen == c->generation || c->n == 0) return PD_OK;
+    if (!c->fam_geo) PD_TRY(dalloc(c, &c->fam_geo, c->n));
+    if (!c->fam_xm) PD_TRY(dalloc(c, &c->fam_xm, c->n));
+    if (!c->sten_pmask) PD_TRY(dalloc(c, &c->sten_pmask, c->n));
+    pd::launch_family_geo(c->d, c->fam_geo, c->stream);
+    pd::launch_static_pmask(c->d, c->sten_pmask, c->stream);
+    PD_CUDA_TRY(cudaGetLastError());
+    c->fam_gen = c->generation;
     return PD_OK;
 }
 
-// y = K x: the stencil kernel when static_prepare accepted the problem, the
-// family-list kernel otherwise; f32: FP32 bond terms on FP64 vectors
-void static_apply(pd_ctx* c, double time, bool f32, const double* x, double* y) {
-    if (c->sten_ok) pd::launch_static_stencil(c->d, c->sten, f32, x, y, c->stream);
-    else if (f32) pd::launch_static_apply_f32x(c->d, time, x, y, c->stream);
-    else pd::launch_static_apply_f64(c->d, time, x, y, c->stream);
+int static_prepare(pd_ctx* c) {
+    PD_TRY(stencil_prepare(c));
+    return family_prepare(c);
+}
+
+pd::FamilyDev family_dev(const pd_ctx* c) { return pd::FamilyDev{c->fam_geo, c->fam_xm, c->sten_pmask}; }
+
+// the input of the operator static_prepare chose
+pd::StaticIn static_in(const pd_ctx* c) {
+    pd::StaticIn I{c->sten, family_dev(c)};
+    if (c->sten_ok) I.F.xm = nullptr;
+    return I;
+}
+
+// sums into the context's scalars
+pd::DotOut dot_out(const pd_ctx* c, int slot0, int slot1 = -1) {
+    return pd::DotOut{c->dotpart, c->dot_done, c->scal, slot0, slot1};
+}
+
+// y = K x from the masked copy of x that launch_static_mask or launch_cg_p
+// left: the stencil kernel when static_prepare accepted the problem, the
+// family-list kernel otherwise; f32: FP32 bond terms on FP64 vectors.  True
+// when the kernel also left x . y in D.
+bool static_masked_apply(pd_ctx* c, bool f32, const double* x, double* y, const pd::DotOut& D) {
+    if (c->sten_ok) return pd::launch_static_stencil(c->d, c->sten, f32, x, y, D, c->stream);
+    return pd::launch_static_family(c->d, family_dev(c), f32, x, y, D, c->stream);
+}
+
+void static_apply(pd_ctx* c, bool f32, const double* x, double* y) {
+    pd::launch_static_mask(c->d, static_in(c), f32, x, c->stream);
+    static_masked_apply(c, f32, x, y, pd::DotOut{});
 }
 
 }  // namespace
@@ -2244,7 +2331,7 @@ int pd_static_matvec(pd_ctx* c, double time, const double* x, double* y) {
     if (!c->have_family) return fail(PD_ERR_ARG, "pd_static_matvec: no family");
     PD_TRY(static_prepare(c));
     PD_TRY(upload_vec3(c, c->d.us, x));
-    static_apply(c, time, false, c->d.us, c->d.k1);
+    static_apply(c, false, c->d.us, c->d.k1);
     PD_CUDA_TRY(cudaGetLastError());
     return download_vec3(c, y, c->d.k1);
 }
@@ -2252,7 +2339,8 @@ int pd_static_matvec(pd_ctx* c, double time, const double* x, double* y) {
 int pd_static_rhs(pd_ctx* c, double time, double* b) {
     if (!c || !b) return fail(PD_ERR_ARG, "pd_static_rhs: null argument");
     if (!c->have_family) return fail(PD_ERR_ARG, "pd_static_rhs: no family");
-    pd::launch_static_rhs(c->d, time, c->d.k1, c->stream);
+    PD_TRY(family_prepare(c));
+    pd::launch_static_rhs(c->d, family_dev(c), time, c->d.k1, c->stream);
     PD_CUDA_TRY(cudaGetLastError());
     return download_vec3(c, b, c->d.k1);
 }
@@ -2277,14 +2365,15 @@ namespace {
 // tolerate matvec errors that grow as the residual falls: Simoncini & Szyld,
 // SIAM J. Sci. Comput. 25 (2003) 454-477).  Convergence is decided on the
 // true residual.  scal: CG_RR = r.z, CG_RRN = the next r.z, CG_RES = r.r.
-int cg_static(pd_ctx* c, double time, const double* b, double* x, double* r, double* p, double* q, double* z,
+int cg_static(pd_ctx* c, const double* b, double* x, double* r, double* p, double* q, double* z,
               const double* minv, bool f32, double f32_below, double rtol, int maxit, int* iters, double* relres,
               int* replacements) {
     const int64_t n3 = 3 * c->n;
     cudaStream_t s = c->stream;
     double* scal = c->scal;
-    auto dot = [&](const double* a, const double* bb, double* out) {
-        pd::launch_dot_f64(a, bb, n3, c->dotpart, out, s);
+    const pd::StaticIn in = static_in(c);
+    auto dot = [&](const double* a, const double* bb, int slot) {
+        pd::launch_dot_f64(a, bb, n3, dot_out(c, slot), s);
     };
     auto read = [&]() -> int {
         PD_CUDA_TRY(cudaGetLastError());
@@ -2294,18 +2383,19 @@ int cg_static(pd_ctx* c, double time, const double* b, double* x, double* r, dou
     };
     // z = M^-1 r (z aliases r without a preconditioner) and r.z into slot
     const double* zz = minv ? z : r;
-    auto precond = [&](double* slot) {
+    auto precond = [&](int slot) {
         if (minv) pd::launch_bj_apply(minv, r, z, c->n, s);
         dot(r, zz, slot);
     };
-    // true residual into r, |r|^2 into scal[CG_RES], r.z into scal[CG_RR]
+    // true residual into r, |r|^2 into scal[CG_RES], r.z into scal[rz]
+    int rz = pd::CG_RR, rzn = pd::CG_RRN;
     auto true_residual = [&]() {
-        static_apply(c, time, false, x, q);
+        static_apply(c, false, x, q);
         pd::launch_sub_f64(b, q, r, n3, s);
-        dot(r, r, scal + pd::CG_RES);
-        precond(scal + pd::CG_RR);
+        dot(r, r, pd::CG_RES);
+        precond(rz);
     };
-    dot(b, b, scal + pd::CG_BB);
+    dot(b, b, pd::CG_BB);
     true_residual();
     PD_CUDA_TRY(cudaMemcpyAsync(p, zz, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s));
     PD_TRY(read());
@@ -2316,15 +2406,13 @@ int cg_static(pd_ctx* c, double time, const double* b, double* x, double* r, dou
     const int check = 10;
     while (rel > rtol && it < maxit) {
         const bool use32 = f32 && rel < f32_below;
+        pd::launch_static_mask(c->d, in, use32, p, s);
         for (int k = 0; k < check && it < maxit; ++k, ++it) {
-            static_apply(c, time, use32, p, q);
-            dot(p, q, scal + pd::CG_PQ);
-            pd::launch_cg_update_x_f64(x, r, p, q, n3, scal, s);
-            precond(scal + pd::CG_RRN);
-            pd::launch_cg_update_p_f64(zz, p, n3, scal, s);
-            pd::launch_cg_swap(scal, s);
+            if (!static_masked_apply(c, use32, p, q, dot_out(c, pd::CG_PQ))) dot(p, q, pd::CG_PQ);
+            pd::launch_cg_x(x, r, p, q, minv, z, c->n, scal + rz, scal + pd::CG_PQ, dot_out(c, rzn, pd::CG_RES), s);
+            pd::launch_cg_p(c->d, in, use32, zz, p, scal + rzn, scal + rz, s);
+            std::swap(rz, rzn);
         }
-        dot(r, r, scal + pd::CG_RES);
         PD_TRY(read());
         rel = std::sqrt(c->hscalar[pd::CG_RES] / bb);
         if (!std::isfinite(rel)) break;
@@ -2356,30 +2444,24 @@ extern "C" int pd_static_solve(pd_ctx* c, double time, int precision, double rto
         return fail(PD_ERR_ARG, "pd_static_solve: precision");
     PD_TRY(static_prepare(c));
     const int64_t n3 = 3 * c->n;
-    double *b = nullptr, *xd = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr;
-    PD_TRY(dalloc(c, &b, n3));
-    PD_TRY(dalloc(c, &xd, n3));
-    PD_TRY(dalloc(c, &r, n3));
-    PD_TRY(dalloc(c, &p, n3));
-    PD_TRY(dalloc(c, &q, n3));
-    if (c->static_precond) PD_TRY(dalloc(c, &z, n3));
-    auto cleanup = [&]() { dfree(c, b); dfree(c, xd); dfree(c, r); dfree(c, p); dfree(c, q); dfree(c, z); };
+    // the solve's vectors stay with the context for its next solve
+    if (!c->cg_work) PD_TRY(dalloc(c, &c->cg_work, 6 * n3));
+    double *b = c->cg_work, *xd = b + n3, *r = xd + n3, *p = r + n3, *q = p + n3, *z = q + n3;
     int rc = upload_vec3(c, xd, x);
-    if (rc != PD_OK) { cleanup(); return rc; }
+    if (rc != PD_OK) return rc;
     if (c->static_precond && (!c->bj_minv || c->bj_gen != c->generation)) {
-        if (!c->bj_minv && (rc = dalloc(c, &c->bj_minv, (size_t)(6 * c->n))) != PD_OK) { cleanup(); return rc; }
+        if (!c->bj_minv && (rc = dalloc(c, &c->bj_minv, (size_t)(6 * c->n))) != PD_OK) return rc;
         pd::launch_static_bjacobi(c->d, c->bj_minv, c->stream);
         c->bj_gen = c->generation;
     }
-    pd::launch_static_rhs(c->d, time, b, c->stream);
+    pd::launch_static_rhs(c->d, family_dev(c), time, b, c->stream);
     int it = 0, nrep = 0;
     double rel = 0.0;
-    rc = cg_static(c, time, b, xd, r, p, q, z, c->static_precond ? c->bj_minv : nullptr,
+    rc = cg_static(c, b, xd, r, p, q, z, c->static_precond ? c->bj_minv : nullptr,
                    precision == PD_PREC_FP32C, c->static_f32_below > 0 ? 1.0 / c->static_f32_below : 2.0, rtol,
                    maxit, &it, &rel, &nrep);
     c->static_replacements = nrep;
     int rc2 = download_vec3(c, x, xd);
-    cleanup();
     if (iters) *iters = it;
     if (relres) *relres = rel;
     if (rc == PD_ERR_NOCONV) return fail(PD_ERR_NOCONV, "static solve did not reach the tolerance");

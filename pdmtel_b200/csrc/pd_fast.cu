@@ -1,15 +1,19 @@
 // The static operator (FP64 and FP32 matvec, right-hand side), the CG pieces,
 // scans and reductions.
+#include <algorithm>
 #include <cstdio>
 #include <type_traits>
 
 #include "pd_internal.cuh"
+#include "pd_rn.cuh"
 
 namespace pd {
 
 namespace {
 
 inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
+// blocks of a grid-stride kernel that sums
+inline unsigned sum_blocks(int64_t n, int bs) { return std::max(1u, std::min(blocks_for(n, bs), (unsigned)kSumBlocks)); }
 
 __device__ __forceinline__ double time_factor(const BcDev& b, double t) {
     if (b.type == PD_BC_VELOC) return (t <= b.end_time) ? 1.0 : 0.0;
@@ -33,84 +37,178 @@ __device__ __forceinline__ void prescribed(const Dev& d, int64_t i, double t, bo
         }
 }
 
-// y = K x on free rows (prescribed columns masked), y = x on prescribed rows.
-// One thread per node over its unbroken family; pdSolve.cpp:195-527.
-template <bool SFAC>
-__global__ void k_static_apply_f64(Dev d, double t, const double* __restrict__ x, double* __restrict__ y) {
-    const int64_t N = d.n;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    bool pi[3];
-    double pv[3];
-    prescribed(d, i, t, pi, pv);
-    const double X0 = d.x[i], X1 = d.x[N + i], X2 = d.x[2 * N + i];
-    const double xi0 = pi[0] ? 0.0 : x[i], xi1 = pi[1] ? 0.0 : x[N + i], xi2 = pi[2] ? 0.0 : x[2 * N + i];
-    const double ci = d.mats[d.mat[i]].spring;
-    const double sfi = SFAC ? d.sfac[i] : 0.0;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int64_t p = d.arow[i]; p < d.arow[i + 1]; ++p) {
-        const int64_t j = d.acol[p];
-        bool pj[3];
-        double qv[3];
-        prescribed(d, j, t, pj, qv);
-        const double e0 = d.x[j] - X0, e1 = d.x[N + j] - X1, e2 = d.x[2 * N + j] - X2;
-        const double r2 = e0 * e0 + e1 * e1 + e2 * e2;
-        const double r = sqrt(r2);
-        const double cj = d.mats[d.mat[j]].spring;
-        double c = (cj < ci) ? cj : ci;
-        if (SFAC) c = c * (0.5 * (sfi + d.sfac[j]));
-        const double w = c * d.vol / (r2 * r);
-        const double d0 = xi0 - (pj[0] ? 0.0 : x[j]);
-        const double d1 = xi1 - (pj[1] ? 0.0 : x[N + j]);
-        const double d2 = xi2 - (pj[2] ? 0.0 : x[2 * N + j]);
-        const double pr = w * (e0 * d0 + e1 * d1 + e2 * d2);
-        a0 += pr * e0;
-        a1 += pr * e1;
-        a2 += pr * e2;
+// Sums the block's values v0 and v1 and, in the last block to finish, every
+// block's sums in block order into out[slot0] and out[slot1] (slot < 0: not
+// wanted), so that the result does not depend on the order of the blocks.
+// part holds two doubles per block; done is zero before and after the launch.
+__device__ __forceinline__ void block_sums(const DotOut& D, double v0, double v1) {
+    __shared__ double sh[2][32];
+    __shared__ bool last;
+    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+    const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    auto sum = [&]() {  // over the block, in v0 and v1 of warp 0
+        for (int o = 16; o > 0; o >>= 1) {
+            v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+            v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+        }
+        if (lane == 0) sh[0][w] = v0, sh[1][w] = v1;
+        __syncthreads();
+        if (w == 0) {
+            v0 = lane < nw ? sh[0][lane] : 0.0;
+            v1 = lane < nw ? sh[1][lane] : 0.0;
+            for (int o = 16; o > 0; o >>= 1) {
+                v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+                v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+            }
+        }
+    };
+    sum();
+    if (threadIdx.x == 0) {
+        __stcg(D.part + 2 * (int64_t)bid, v0);
+        __stcg(D.part + 2 * (int64_t)bid + 1, v1);
+        __threadfence();
+        last = atomicAdd(D.done, 1u) + 1 == nb;
     }
-    y[i] = pi[0] ? x[i] : a0;
-    y[N + i] = pi[1] ? x[N + i] : a1;
-    y[2 * N + i] = pi[2] ? x[2 * N + i] : a2;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    v0 = v1 = 0.0;
+    for (unsigned k = threadIdx.x; k < nb; k += blockDim.x) {
+        v0 += __ldcg(D.part + 2 * (int64_t)k);
+        v1 += __ldcg(D.part + 2 * (int64_t)k + 1);
+    }
+    sum();
+    if (threadIdx.x == 0) {
+        if (D.slot0 >= 0) D.out[D.slot0] = v0;
+        if (D.slot1 >= 0) D.out[D.slot1] = v1;
+        *D.done = 0;
+    }
 }
 
-// The same operator with FP32 arithmetic on FP64 vectors: the per-bond
-// difference x_i - x_j is formed in FP64 and rounded once, the bond term is
-// FP32, the node sum FP64.  The matvec of the mixed-precision CG.
-template <bool SFAC>
-__global__ void k_static_apply_f32x(Dev d, double t, const double* __restrict__ x, double* __restrict__ y) {
-    const int64_t N = d.n;
+// Node data of the family-list operator as one 32-byte record per node, so
+// that a bond gathers two records instead of six words from six arrays:
+// geo = (coordinates, spring), xm = (masked input, spring factor).
+__global__ void k_family_geo(Dev d, double4* __restrict__ geo) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < d.n) geo[i] = make_double4(d.x[i], d.x[d.n + i], d.x[2 * d.n + i], d.mats[d.mat[i]].spring);
+}
+
+__global__ void k_family_mask(Dev d, const uint8_t* __restrict__ pmask, const double* __restrict__ x,
+                              double4* __restrict__ xm) {
+    const int64_t N = d.n, i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= N) return;
+    const unsigned m = pmask[i];
+    xm[i] = make_double4((m & 1) ? 0.0 : x[i], (m & 2) ? 0.0 : x[N + i], (m & 4) ? 0.0 : x[2 * N + i],
+                         d.sfac ? d.sfac[i] : 0.0);
+}
+
+// xm = the prescribed values, zero elsewhere: the right-hand side's input
+__global__ void k_family_prescribed(Dev d, double t, double4* __restrict__ xm) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= d.n) return;
+    bool pre[3];
+    double v[3];
+    prescribed(d, i, t, pre, v);
+    xm[i] = make_double4(v[0], v[1], v[2], d.sfac ? d.sfac[i] : 0.0);
+}
+
+// sum over node i's unbroken family of w xi (xi . (x_i - x_j)), w = c V / r^3,
+// L lanes per node (pdSolve.cpp:195-527).  F32: the bond difference formed in
+// FP64 and rounded once, the bond term FP32, the sums FP64.
+//
+// One thread per node walked its family as a chain of dependent loads, six of
+// them 8-byte gathers, with an IEEE root and division per bond: 198 us for
+// 28,800 nodes (225 blocks, SMs mostly waiting).  A group of lanes takes the
+// bonds side by side, gathers two 32-byte records each, and forms 1/r by the
+// unrounded iteration of pd_rn.cuh: 62 us.
+template <bool SFAC, bool F32, int L>
+__device__ __forceinline__ void family_sum(const Dev& d, const FamilyDev& F, int64_t i, int ql, double4 gi,
+                                           double4 xi, double& a0, double& a1, double& a2) {
+    a0 = a1 = a2 = 0.0;
+    const int64_t pe = d.arow[i + 1];
+#pragma unroll 2
+    for (int64_t p = d.arow[i] + ql; p < pe; p += L) {
+        const int64_t j = d.acol[p];
+        const double4 gj = F.geo[j], xj = F.xm[j];
+        double c = gj.w < gi.w ? gj.w : gi.w;
+        if (SFAC) c = c * (0.5 * (xi.w + xj.w));
+        const double e0 = gj.x - gi.x, e1 = gj.y - gi.y, e2 = gj.z - gi.z;
+        const double d0 = xi.x - xj.x, d1 = xi.y - xj.y, d2 = xi.z - xj.z;
+        if (F32) {
+            const float f0 = (float)e0, f1 = (float)e1, f2 = (float)e2;
+            const float rinv = rsqrtf(fmaf(f0, f0, fmaf(f1, f1, f2 * f2)));
+            const float w = (float)(c * d.vol) * rinv * rinv * rinv;
+            const float pr = w * fmaf(f0, (float)d0, fmaf(f1, (float)d1, f2 * (float)d2));
+            a0 += (double)(pr * f0);
+            a1 += (double)(pr * f1);
+            a2 += (double)(pr * f2);
+        } else {
+            const double r2 = e0 * e0 + e1 * e1 + e2 * e2;
+            const double ri = rn_range(r2) ? rsqrt_near(r2) : 1.0 / sqrt(r2);
+            const double pr = (c * d.vol) * (ri * ri * ri) * (e0 * d0 + e1 * d1 + e2 * d2);
+            a0 += pr * e0;
+            a1 += pr * e1;
+            a2 += pr * e2;
+        }
+    }
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    }
+}
+
+// y = K x on free rows (prescribed columns masked), y = x on prescribed rows,
+// and x . y when D.part is set.
+template <bool SFAC, bool F32, int L>
+__global__ void __launch_bounds__(256) k_family_apply(Dev d, FamilyDev F, const double* __restrict__ x,
+                                                      double* __restrict__ y, DotOut D) {
+    const int64_t N = d.n;
+    const int ql = threadIdx.x % L;
+    double dot = 0.0;
+    constexpr int64_t per = 256 / L;
+    for (int64_t base = blockIdx.x * per; base < N; base += gridDim.x * per) {
+        const int64_t i = base + threadIdx.x / L;
+        const bool live = i < N;
+        const int64_t k = live ? d.order[i] : d.order[0];
+        double a[3];
+        family_sum<SFAC, F32, L>(d, F, k, ql, F.geo[k], F.xm[k], a[0], a[1], a[2]);
+        if (live && ql < 3) {
+            const double own = x[(int64_t)ql * N + k];
+            const double s = ql == 0 ? a[0] : (ql == 1 ? a[1] : a[2]);
+            const double v = (F.pmask[k] >> ql & 1) ? own : s;
+            y[(int64_t)ql * N + k] = v;
+            dot += own * v;
+        }
+    }
+    if (D.part) block_sums(D, dot, 0.0);
+}
+
+// b = prescribed values on prescribed rows; on free rows the moved prescribed
+// columns (pdSolve.cpp:296-363 sign pattern: minus the family sum of the
+// prescribed values in F.xm) plus the traction load.
+template <bool SFAC, int L>
+__global__ void __launch_bounds__(256) k_static_rhs(Dev d, FamilyDev F, double t, double* __restrict__ out) {
+    const int64_t N = d.n;
+    const int ql = threadIdx.x % L;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
+    const int64_t i = slot < N ? slot : 0;
+    double a[3];
+    family_sum<SFAC, false, L>(d, F, i, ql, F.geo[i], F.xm[i], a[0], a[1], a[2]);
+    if (slot >= N || ql >= 3) return;
     bool pi[3];
     double pv[3];
     prescribed(d, i, t, pi, pv);
-    const double X0 = d.x[i], X1 = d.x[N + i], X2 = d.x[2 * N + i];
-    const double xi0 = pi[0] ? 0.0 : x[i], xi1 = pi[1] ? 0.0 : x[N + i], xi2 = pi[2] ? 0.0 : x[2 * N + i];
-    const double ci = d.mats[d.mat[i]].spring;
-    const double sfi = SFAC ? d.sfac[i] : 0.0;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int64_t p = d.arow[i]; p < d.arow[i + 1]; ++p) {
-        const int64_t j = d.acol[p];
-        bool pj[3];
-        double qv[3];
-        prescribed(d, j, t, pj, qv);
-        const float e0 = (float)(d.x[j] - X0), e1 = (float)(d.x[N + j] - X1), e2 = (float)(d.x[2 * N + j] - X2);
-        const double cj = d.mats[d.mat[j]].spring;
-        double c = (cj < ci) ? cj : ci;
-        if (SFAC) c = c * (0.5 * (sfi + d.sfac[j]));
-        const float rinv = rsqrtf(fmaf(e0, e0, fmaf(e1, e1, e2 * e2)));
-        const float w = (float)(c * d.vol) * rinv * rinv * rinv;
-        const float d0 = (float)(xi0 - (pj[0] ? 0.0 : x[j]));
-        const float d1 = (float)(xi1 - (pj[1] ? 0.0 : x[N + j]));
-        const float d2 = (float)(xi2 - (pj[2] ? 0.0 : x[2 * N + j]));
-        const float pr = w * fmaf(e0, d0, fmaf(e1, d1, e2 * d2));
-        a0 += (double)(pr * e0);
-        a1 += (double)(pr * e1);
-        a2 += (double)(pr * e2);
+    double load = -(ql == 0 ? a[0] : (ql == 1 ? a[1] : a[2]));
+    const int b = d.bc[i];
+    if (b >= 0) {
+        const BcDev& B = d.bcs[b];
+        if (B.type == PD_BC_TRACTION && B.dir[ql] == 1) load += B.val[ql] * time_factor(B, t) / d.dx;
     }
-    y[i] = pi[0] ? x[i] : a0;
-    y[N + i] = pi[1] ? x[N + i] : a1;
-    y[2 * N + i] = pi[2] ? x[2 * N + i] : a2;
+    out[(int64_t)ql * N + i] = (ql == 0 ? pi[0] : (ql == 1 ? pi[1] : pi[2])) ? (ql == 0 ? pv[0] : (ql == 1 ? pv[1] : pv[2]))
+                                                                         : load;
 }
 
 // prescribed directions of every node as bits 0..2 (the static operator's
@@ -145,6 +243,124 @@ __global__ void k_static_mask(const uint8_t* __restrict__ pmask, int64_t N, cons
         const double v = (m & (1u << a)) ? 0.0 : x[a * N + i];
         xm[a * N + i] = (T)v;
     }
+}
+
+// The offset key of family entry i -> j from the packed lattice positions, -1
+// outside [-64, 63]^3.
+__device__ __forceinline__ int box_key(int li, int lj) {
+    const int ox = (lj & 2047) - (li & 2047), oy = (lj >> 11 & 2047) - (li >> 11 & 2047), oz = (lj >> 22) - (li >> 22);
+    if (((unsigned)(ox + 64) | (unsigned)(oy + 64) | (unsigned)(oz + 64)) > 127u) return -1;
+    return (ox + 64) << 14 | (oy + 64) << 7 | (oz + 64);
+}
+
+// A warp per node over its full family: the check that a host loop over the
+// downloaded family used to make.
+__global__ void __launch_bounds__(256) k_box_offsets(Dev d, int* __restrict__ map, int* __restrict__ err) {
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= d.n) return;
+    const int li = d.lat[i];
+    if (lane == 0 && (li & 2047) + (int64_t)d.lat_nx * ((li >> 11 & 2047) + (int64_t)d.lat_ny * (li >> 22)) != i)
+        atomicOr(err, 1);
+    for (int64_t p = d.frow[i] + lane; p < d.frow[i + 1]; p += 32) {
+        const int k = box_key(li, d.lat[d.fcol[p]]);
+        if (k < 0) atomicOr(err, 1);
+        else if (!map[k]) map[k] = 1;  // the same value from every writer
+    }
+}
+
+__global__ void k_box_list(const int* __restrict__ map, int* __restrict__ count, int4* __restrict__ list) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!map[k]) return;
+    const int at = atomicAdd(count, 1);
+    if (at < kMaxStencil) list[at] = make_int4((k >> 14) - 64, (k >> 7 & 127) - 64, (k & 127) - 64, 0);
+}
+
+__global__ void k_box_check(Dev d, const int4* __restrict__ list, int nlist, int* __restrict__ err) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= d.n) return;
+    const int li = d.lat[i], ix = li & 2047, iy = li >> 11 & 2047, iz = li >> 22;
+    int in = 0;
+    for (int k = 0; k < nlist; ++k) {
+        const int4 o = list[k];
+        in += (unsigned)(ix + o.x) < (unsigned)d.lat_nx && (unsigned)(iy + o.y) < (unsigned)d.lat_ny &&
+              (unsigned)(iz + o.z) < (unsigned)d.lat_nz;
+    }
+    if (in != d.frow[i + 1] - d.frow[i]) atomicOr(err, 1);
+}
+
+__global__ void k_box_slots(const int4* __restrict__ list, int nlist, int* __restrict__ map) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nlist) return;
+    const int4 o = list[k];
+    map[(o.x + 64) << 14 | (o.y + 64) << 7 | (o.z + 64)] = k;
+}
+
+__global__ void k_broken_counts(Dev d, int64_t* __restrict__ flag, int64_t* __restrict__ cnt) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= d.n) return;
+    const int64_t c = (d.frow[i + 1] - d.frow[i]) - (d.arow[i + 1] - d.arow[i]);
+    cnt[i] = c;
+    flag[i] = c > 0;
+}
+
+__global__ void k_broken_fill(Dev d, const int* __restrict__ map, const int64_t* __restrict__ flag,
+                              const int64_t* __restrict__ fpos, const int64_t* __restrict__ cpos,
+                              int32_t* __restrict__ bnode, int64_t* __restrict__ bptr, int2* __restrict__ bent,
+                              int32_t* __restrict__ bidx) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= d.n) return;
+    if (!flag[i]) {
+        bidx[i] = -1;
+        return;
+    }
+    const int64_t k = fpos[i];
+    bidx[i] = (int32_t)k;
+    bnode[k] = (int32_t)i;
+    int64_t o = cpos[i];
+    bptr[k] = o;
+    for (int64_t p = d.frow[i]; p < d.frow[i + 1]; ++p)
+        if (d.fbroken[p]) bent[o++] = make_int2(d.fcol[p], map[box_key(d.lat[i], d.lat[d.fcol[p]])]);
+}
+
+// What the broken bonds of a node would add to the stencil operator, a warp
+// per node that has some; the operator kernels subtract it.  A cracked box then
+// runs on the stencil, with a list only of what the crack cut: 60x40x12 with a
+// slit, 62 us per matvec on the family lists, 7 us here and about 15 in
+// k_static_nd.
+template <typename T, bool SFAC>
+__global__ void __launch_bounds__(128) k_static_broken(Dev d, StencilDev S, const T* __restrict__ xm) {
+    const int k = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (k >= S.nbrk) return;
+    const int64_t N = d.n, i = S.bnode[k];
+    const T x0 = xm[i], x1 = xm[N + i], x2 = xm[2 * N + i];
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    for (int64_t p = S.bptr[k] + lane; p < S.bptr[k + 1]; p += 32) {
+        const int2 e = S.bent[p];
+        const int64_t j = e.x;
+        const double4 g = S.geo[e.y];
+        double w = g.w;
+        if (SFAC) w = w * (0.5 * (d.sfac[i] + d.sfac[j]));
+        const T f0 = (T)g.x, f1 = (T)g.y, f2 = (T)g.z;
+        const T pr = (T)w * (f0 * (x0 - xm[j]) + f1 * (x1 - xm[N + j]) + f2 * (x2 - xm[2 * N + j]));
+        a0 += (double)(pr * f0);
+        a1 += (double)(pr * f1);
+        a2 += (double)(pr * f2);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    }
+    if (lane < 3) S.bfix[3 * (int64_t)k + lane] = lane == 0 ? a0 : (lane == 1 ? a1 : a2);
+}
+__device__ __forceinline__ void less_broken(const StencilDev& S, int64_t i, double& a0, double& a1, double& a2) {
+    if (S.nbrk == 0) return;
+    const int k = S.bidx[i];
+    if (k < 0) return;
+    a0 -= S.bfix[3 * (int64_t)k];
+    a1 -= S.bfix[3 * (int64_t)k + 1];
+    a2 -= S.bfix[3 * (int64_t)k + 2];
 }
 
 // FP64: bond terms and sums in FP64.  FP32: bond terms in FP32 from an FP32
@@ -233,6 +449,7 @@ __global__ void __launch_bounds__(256) k_static_stencil(Dev d, StencilDev S, con
     const bool inner = ix >= R && ix < S.nx - R && iy >= R && iy < S.ny - R && iz >= R && iz < S.nz - R;
     if (inner) stencil_sum<T, SFAC, false>(d, S, sgeo, sgeof, soff, i, ix, iy, iz, xm, sfi, a0, a1, a2);
     else stencil_sum<T, SFAC, true>(d, S, sgeo, sgeof, soff, i, ix, iy, iz, xm, sfi, a0, a1, a2);
+    less_broken(S, i, a0, a1, a2);
     y[i] = (mi & 1) ? x[i] : a0;
     y[N + i] = (mi & 2) ? x[N + i] : a1;
     y[2 * N + i] = (mi & 4) ? x[2 * N + i] : a2;
@@ -382,6 +599,7 @@ __global__ void __launch_bounds__(128) k_static_zcol(Dev d, StencilDev S, const 
     for (int m = 0; m < R; ++m) {
         if (!in_xy || iz0 + m >= S.nz) continue;
         const int64_t i = i0 + m * nxy;
+        less_broken(S, i, acc[m][0], acc[m][1], acc[m][2]);
         const unsigned mi = S.pmask[i];
         y[i] = (mi & 1) ? x[i] : acc[m][0];
         y[N + i] = (mi & 2) ? x[N + i] : acc[m][1];
@@ -495,7 +713,7 @@ inline size_t nd_smem(const StencilDev& S, int R) {
 template <int R, int RH>
 __global__ void __launch_bounds__(256) k_static_nd(Dev d, StencilDev S, const __grid_constant__ NdTab tb,
                                                    const double* __restrict__ x, const double* __restrict__ xm,
-                                                   double* __restrict__ y) {
+                                                   double* __restrict__ y, DotOut D) {
     using L = NdTile<R, RH>;
     extern __shared__ double2 ndsm[];
     double* P = reinterpret_cast<double*>(ndsm);
@@ -554,30 +772,42 @@ __global__ void __launch_bounds__(256) k_static_nd(Dev d, StencilDev S, const __
             for (int a = 0; a < 3; ++a) xch[(3 * m + a) * 128] = acc[m][a];
     }
     __syncthreads();
-    if (g == 1 || ix >= S.nx || iy >= S.ny) return;
+    double dot = 0.0;
+    if (g == 0 && ix < S.nx && iy < S.ny) {
 #pragma unroll
-    for (int m = 0; m < R; ++m)
-        for (int a = 0; a < 3; ++a) acc[m][a] += xch[(3 * m + a) * 128];
-    const bool xy_inner = S.ndin && ix >= S.nrx && ix < S.nx - S.nrx && iy >= S.nry && iy < S.ny - S.nry;
-    const int64_t i0 = ix + (int64_t)S.nx * iy + nxy * z0;
+        for (int m = 0; m < R; ++m)
+            for (int a = 0; a < 3; ++a) acc[m][a] += xch[(3 * m + a) * 128];
+        const bool xy_inner = S.ndin && ix >= S.nrx && ix < S.nx - S.nrx && iy >= S.nry && iy < S.ny - S.nry;
+        const int64_t i0 = ix + (int64_t)S.nx * iy + nxy * z0;
 #pragma unroll
-    for (int m = 0; m < R; ++m) {
-        const int iz = z0 + m;
-        if (iz >= S.nz) continue;
-        const int64_t i = i0 + m * nxy;
-        const bool inner = xy_inner && iz >= S.rz && iz < S.nz - S.rz;
-        double D[6];
+        for (int m = 0; m < R; ++m) {
+            const int iz = z0 + m;
+            if (iz >= S.nz) continue;
+            const int64_t i = i0 + m * nxy;
+            const bool inner = xy_inner && iz >= S.rz && iz < S.nz - S.rz;
+            double B[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) D[k] = inner ? S.ndint[k] : S.ndiag[k * N + i];
-        const double u0 = u[m][0], u1 = u[m][1], u2 = u[m][2];
-        const double y0v = fma(D[0], u0, fma(D[3], u1, fma(D[4], u2, acc[m][0])));
-        const double y1v = fma(D[3], u0, fma(D[1], u1, fma(D[5], u2, acc[m][1])));
-        const double y2v = fma(D[4], u0, fma(D[5], u1, fma(D[2], u2, acc[m][2])));
-        const unsigned mi = S.pmask[i];
-        y[i] = (mi & 1) ? x[i] : y0v;
-        y[N + i] = (mi & 2) ? x[N + i] : y1v;
-        y[2 * N + i] = (mi & 4) ? x[2 * N + i] : y2v;
+            for (int k = 0; k < 6; ++k) B[k] = inner ? S.ndint[k] : S.ndiag[k * N + i];
+            const double u0 = u[m][0], u1 = u[m][1], u2 = u[m][2];
+            double v[3] = {fma(B[0], u0, fma(B[3], u1, fma(B[4], u2, acc[m][0]))),
+                           fma(B[3], u0, fma(B[1], u1, fma(B[5], u2, acc[m][1]))),
+                           fma(B[4], u0, fma(B[5], u1, fma(B[2], u2, acc[m][2])))};
+            less_broken(S, i, v[0], v[1], v[2]);
+            const unsigned mi = S.pmask[i];
+            if (mi) {  // prescribed rows: y = x
+                for (int a = 0; a < 3; ++a) {
+                    if (!(mi >> a & 1)) continue;
+                    v[a] = x[a * N + i];
+                    dot += v[a] * v[a];
+                }
+            }
+            dot += v[0] * u0 + v[1] * u1 + v[2] * u2;  // u is zero in prescribed directions
+            y[i] = v[0];
+            y[N + i] = v[1];
+            y[2 * N + i] = v[2];
+        }
     }
+    if (D.part) block_sums(D, dot, 0.0);
 }
 
 // D_i = sum of w xi xi^T over the stencil offsets that stay in the box, from
@@ -606,23 +836,26 @@ __global__ void k_static_ndiag(StencilDev S, int64_t N, double* __restrict__ D) 
 }
 
 template <int R, int RH>
-void launch_nd_h(const Dev& d, const StencilDev& S, const double* x, const double* xm, double* y, cudaStream_t s) {
+void launch_nd_h(const Dev& d, const StencilDev& S, const double* x, const double* xm, double* y, const DotOut& D,
+                 cudaStream_t s) {
     const dim3 grid((unsigned)((S.nx + 31) / 32), (unsigned)((S.ny + 3) / 4), (unsigned)((S.nz + R - 1) / R));
     static bool attr = false;  // once per process: the tile needs more than the 48 KB default
     if (!attr) {
-        cudaFuncSetAttribute(k_static_nd<R, RH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(k_static_nd<R, RH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(3 * NdTile<R, RH>::CS * sizeof(double)));
         attr = true;
     }
-    k_static_nd<R, RH><<<grid, 256, nd_smem(S, R), s>>>(d, S, *S.ndhost, x, xm, y);
+    k_static_nd<R, RH><<<grid, 256, nd_smem(S, R), s>>>(d, S, *S.ndhost, x, xm, y, D);
 }
 
 template <int R>
-void launch_nd(const Dev& d, const StencilDev& S, const double* x, const double* xm, double* y, cudaStream_t s) {
+void launch_nd(const Dev& d, const StencilDev& S, const double* x, const double* xm, double* y, const DotOut& D,
+               cudaStream_t s) {
     switch (nd_halo(S)) {
-        case 1: launch_nd_h<R, 1>(d, S, x, xm, y, s); break;
-        case 2: launch_nd_h<R, 2>(d, S, x, xm, y, s); break;
-        case 3: launch_nd_h<R, 3>(d, S, x, xm, y, s); break;
-        default: launch_nd_h<R, 4>(d, S, x, xm, y, s); break;
+        case 1: launch_nd_h<R, 1>(d, S, x, xm, y, D, s); break;
+        case 2: launch_nd_h<R, 2>(d, S, x, xm, y, D, s); break;
+        case 3: launch_nd_h<R, 3>(d, S, x, xm, y, D, s); break;
+        default: launch_nd_h<R, 4>(d, S, x, xm, y, D, s); break;
     }
 }
 
@@ -636,58 +869,6 @@ void launch_zcol(const Dev& d, const StencilDev& S, const double* x, const T* xm
         case 2: k_static_zcol<T, SFAC, 2, R><<<grid, 128, sh, s>>>(d, S, x, xm, y); break;
         case 3: k_static_zcol<T, SFAC, 3, R><<<grid, 128, sh, s>>>(d, S, x, xm, y); break;
         default: k_static_zcol<T, SFAC, 4, R><<<grid, 128, sh, s>>>(d, S, x, xm, y); break;
-    }
-}
-
-// b = prescribed values on prescribed rows; on free rows the moved prescribed
-// columns (pdSolve.cpp:296-363 sign pattern) plus the traction load.
-template <bool SFAC>
-__global__ void k_static_rhs(Dev d, double t, double* __restrict__ out) {
-    const int64_t N = d.n;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    bool pi[3];
-    double pv[3];
-    prescribed(d, i, t, pi, pv);
-    const double X0 = d.x[i], X1 = d.x[N + i], X2 = d.x[2 * N + i];
-    const double ci = d.mats[d.mat[i]].spring;
-    const double sfi = SFAC ? d.sfac[i] : 0.0;
-    const double m0 = pi[0] ? pv[0] : 0.0, m1 = pi[1] ? pv[1] : 0.0, m2 = pi[2] ? pv[2] : 0.0;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int64_t p = d.arow[i]; p < d.arow[i + 1]; ++p) {
-        const int64_t j = d.acol[p];
-        bool pj[3];
-        double qv[3];
-        prescribed(d, j, t, pj, qv);
-        const double e0 = d.x[j] - X0, e1 = d.x[N + j] - X1, e2 = d.x[2 * N + j] - X2;
-        const double r2 = e0 * e0 + e1 * e1 + e2 * e2;
-        const double r = sqrt(r2);
-        const double cj = d.mats[d.mat[j]].spring;
-        double c = (cj < ci) ? cj : ci;
-        if (SFAC) c = c * (0.5 * (sfi + d.sfac[j]));
-        const double w = c * d.vol / (r2 * r);
-        // -K_ii(prescribed cols) ubar_i + K_ij-part: +c xi xi^T ubar_j
-        const double d0 = (pj[0] ? qv[0] : 0.0) - m0;
-        const double d1 = (pj[1] ? qv[1] : 0.0) - m1;
-        const double d2 = (pj[2] ? qv[2] : 0.0) - m2;
-        const double pr = w * (e0 * d0 + e1 * d1 + e2 * d2);
-        a0 += pr * e0;
-        a1 += pr * e1;
-        a2 += pr * e2;
-    }
-    double acc[3] = {a0, a1, a2};
-    const int b = d.bc[i];
-    for (int a = 0; a < 3; ++a) {
-        if (pi[a]) {
-            out[a * N + i] = pv[a];
-            continue;
-        }
-        double load = acc[a];
-        if (b >= 0) {
-            const BcDev& B = d.bcs[b];
-            if (B.type == PD_BC_TRACTION && B.dir[a] == 1) load += B.val[a] * time_factor(B, t) / d.dx;
-        }
-        out[a * N + i] = load;
     }
 }
 
@@ -760,16 +941,45 @@ int exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t 
     return rc;
 }
 
-void launch_static_apply_f64(const Dev& d, double t, const double* x, double* y, cudaStream_t s) {
-    if (d.n == 0) return;
-    if (d.sfac) k_static_apply_f64<true><<<blocks_for(d.n, 128), 128, 0, s>>>(d, t, x, y);
-    else k_static_apply_f64<false><<<blocks_for(d.n, 128), 128, 0, s>>>(d, t, x, y);
+// A small problem gives a node a whole warp, so that the SMs fill; a larger one
+// eight lanes, whose families (about 170 to 250 bonds) then leave fewer lanes
+// idle in their last round.
+namespace {
+constexpr int64_t kFamilyWarpBelow = 12288;
+template <typename K>
+void family_launch(const Dev& d, K&& kernel) {
+    if (d.n < kFamilyWarpBelow) kernel(std::integral_constant<int, 32>{});
+    else kernel(std::integral_constant<int, 8>{});
+}
+}  // namespace
+
+void launch_family_geo(const Dev& d, double4* geo, cudaStream_t s) {
+    if (d.n) k_family_geo<<<blocks_for(d.n, 256), 256, 0, s>>>(d, geo);
 }
 
-void launch_static_apply_f32x(const Dev& d, double t, const double* x, double* y, cudaStream_t s) {
+void launch_static_mask(const Dev& d, const StaticIn& I, bool f32, const double* x, cudaStream_t s) {
     if (d.n == 0) return;
-    if (d.sfac) k_static_apply_f32x<true><<<blocks_for(d.n, 128), 128, 0, s>>>(d, t, x, y);
-    else k_static_apply_f32x<false><<<blocks_for(d.n, 128), 128, 0, s>>>(d, t, x, y);
+    const unsigned nb = blocks_for(d.n, 256);
+    if (I.F.xm) k_family_mask<<<nb, 256, 0, s>>>(d, I.F.pmask, x, I.F.xm);
+    else if (f32) k_static_mask<float><<<nb, 256, 0, s>>>(I.S.pmask, d.n, x, reinterpret_cast<float*>(I.S.xm));
+    else k_static_mask<double><<<nb, 256, 0, s>>>(I.S.pmask, d.n, x, I.S.xm);
+}
+
+bool launch_static_family(const Dev& d, const FamilyDev& F, bool f32, const double* x, double* y, const DotOut& D,
+                          cudaStream_t s) {
+    if (d.n == 0) return false;
+    family_launch(d, [&](auto lanes) {
+        constexpr int L = decltype(lanes)::value;
+        const unsigned nb = sum_blocks(L * d.n, 256);
+        if (f32) {
+            if (d.sfac) k_family_apply<true, true, L><<<nb, 256, 0, s>>>(d, F, x, y, D);
+            else k_family_apply<false, true, L><<<nb, 256, 0, s>>>(d, F, x, y, D);
+        } else {
+            if (d.sfac) k_family_apply<true, false, L><<<nb, 256, 0, s>>>(d, F, x, y, D);
+            else k_family_apply<false, false, L><<<nb, 256, 0, s>>>(d, F, x, y, D);
+        }
+    });
+    return D.part != nullptr;
 }
 
 size_t static_nd_smem(const StencilDev& S, int R) { return nd_smem(S, R); }
@@ -778,19 +988,42 @@ void launch_static_ndiag(const StencilDev& S, int64_t n, double* D, cudaStream_t
     if (n) k_static_ndiag<<<blocks_for(n, 128), 128, 0, s>>>(S, n, D);
 }
 
+void launch_box_offsets(const Dev& d, int* map, int* err, int4* list, cudaStream_t s) {
+    if (d.n == 0) return;
+    k_box_offsets<<<blocks_for(32 * d.n, 256), 256, 0, s>>>(d, map, err);
+    k_box_list<<<(1 << 21) / 256, 256, 0, s>>>(map, err + 1, list);
+}
+void launch_box_check(const Dev& d, const int4* list, int nlist, int* map, int* err, cudaStream_t s) {
+    if (d.n == 0) return;
+    k_box_check<<<blocks_for(d.n, 256), 256, 0, s>>>(d, list, nlist, err);
+    k_box_slots<<<blocks_for(nlist, 256), 256, 0, s>>>(list, nlist, map);
+}
+void launch_broken_counts(const Dev& d, int64_t* flag, int64_t* cnt, cudaStream_t s) {
+    if (d.n) k_broken_counts<<<blocks_for(d.n, 256), 256, 0, s>>>(d, flag, cnt);
+}
+void launch_broken_fill(const Dev& d, const int* map, const int64_t* flag, const int64_t* fpos, const int64_t* cpos,
+                        int32_t* bnode, int64_t* bptr, int2* bent, int32_t* bidx, cudaStream_t s) {
+    if (d.n) k_broken_fill<<<blocks_for(d.n, 128), 128, 0, s>>>(d, map, flag, fpos, cpos, bnode, bptr, bent, bidx);
+}
+
 void launch_static_pmask(const Dev& d, uint8_t* pm, cudaStream_t s) {
     if (d.n == 0) return;
     k_static_pmask<<<blocks_for(d.n, 256), 256, 0, s>>>(d, pm);
 }
 
-void launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const double* x, double* y, cudaStream_t s) {
-    if (d.n == 0) return;
+bool launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const double* x, double* y, const DotOut& D,
+                           cudaStream_t s) {
+    if (d.n == 0) return false;
     const size_t sh = (size_t)S.ns * (sizeof(double4) + sizeof(float4) + sizeof(int4));
     const unsigned nb = blocks_for(d.n, 256);
     const bool zcol = S.ncol > 0 && S.rz >= 1 && S.rz <= 4;
     if (f32) {
         float* xm = reinterpret_cast<float*>(S.xm);
-        k_static_mask<float><<<nb, 256, 0, s>>>(S.pmask, d.n, x, xm);
+        if (S.nbrk) {
+            const unsigned bb = blocks_for(32 * (int64_t)S.nbrk, 128);
+            if (d.sfac) k_static_broken<float, true><<<bb, 128, 0, s>>>(d, S, xm);
+            else k_static_broken<float, false><<<bb, 128, 0, s>>>(d, S, xm);
+        }
         if (zcol) {
             if (d.sfac) launch_zcol<float, true, 8>(d, S, x, xm, y, s);
             else launch_zcol<float, false, 8>(d, S, x, xm, y, s);
@@ -801,12 +1034,17 @@ void launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const do
         }
     } else {
         double* xm = S.xm;
-        k_static_mask<double><<<nb, 256, 0, s>>>(S.pmask, d.n, x, xm);
+        if (S.nbrk) {
+            const unsigned bb = blocks_for(32 * (int64_t)S.nbrk, 128);
+            if (d.sfac) k_static_broken<double, true><<<bb, 128, 0, s>>>(d, S, xm);
+            else k_static_broken<double, false><<<bb, 128, 0, s>>>(d, S, xm);
+        }
         if (S.ndcol > 0 && S.ndhost && !d.sfac && (S.ndr == 2 || S.ndr == 4 || S.ndr == 8) && nd_halo(S) > 0 &&
-            nd_smem(S, S.ndr) <= 227 * 1024) {
-            if (S.ndr == 2) launch_nd<2>(d, S, x, xm, y, s);
-            else if (S.ndr == 4) launch_nd<4>(d, S, x, xm, y, s);
-            else launch_nd<8>(d, S, x, xm, y, s);
+            nd_smem(S, S.ndr) <= 226 * 1024) {
+            if (S.ndr == 2) launch_nd<2>(d, S, x, xm, y, D, s);
+            else if (S.ndr == 4) launch_nd<4>(d, S, x, xm, y, D, s);
+            else launch_nd<8>(d, S, x, xm, y, D, s);
+            return D.part != nullptr;
         } else if (zcol) {
             if (d.sfac) launch_zcol<double, true, 4>(d, S, x, xm, y, s);
             else launch_zcol<double, false, 4>(d, S, x, xm, y, s);
@@ -816,6 +1054,7 @@ void launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const do
             k_static_stencil<double, false><<<nb, 256, sh, s>>>(d, S, x, xm, y);
         }
     }
+    return false;
 }
 
 void launch_static_bjacobi(const Dev& d, double* minv, cudaStream_t s) {
@@ -828,62 +1067,94 @@ void launch_bj_apply(const double* minv, const double* r, double* z, int64_t n, 
     if (n) k_bj_apply<<<148 * 8, 256, 0, s>>>(minv, r, z, n);
 }
 
-void launch_static_rhs(const Dev& d, double t, double* b, cudaStream_t s) {
+void launch_static_rhs(const Dev& d, const FamilyDev& F, double t, double* b, cudaStream_t s) {
     if (d.n == 0) return;
-    if (d.sfac) k_static_rhs<true><<<blocks_for(d.n, 128), 128, 0, s>>>(d, t, b);
-    else k_static_rhs<false><<<blocks_for(d.n, 128), 128, 0, s>>>(d, t, b);
+    k_family_prescribed<<<blocks_for(d.n, 256), 256, 0, s>>>(d, t, F.xm);
+    family_launch(d, [&](auto lanes) {
+        constexpr int L = decltype(lanes)::value;
+        if (d.sfac) k_static_rhs<true, L><<<blocks_for(L * d.n, 256), 256, 0, s>>>(d, F, t, b);
+        else k_static_rhs<false, L><<<blocks_for(L * d.n, 256), 256, 0, s>>>(d, F, t, b);
+    });
 }
 
 // -------------------------------------------------------------- CG pieces
 
 namespace {
 
-template <typename T>
-__global__ void k_dot_partial(const T* __restrict__ a, const T* __restrict__ b, int64_t n, double* __restrict__ part) {
-    __shared__ double sh[256];
+__global__ void __launch_bounds__(256) k_dot(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
+                                             DotOut D) {
     double acc = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        acc += (double)a[i] * (double)b[i];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-        __syncthreads();
+        acc += a[i] * b[i];
+    block_sums(D, acc, 0.0);
+}
+
+// One pass of the CG update: alpha = r.z / p.q, x += alpha p, r -= alpha q,
+// z = M^-1 r (not formed without a preconditioner: z is r), and the sums r.z
+// and r.r.  Separate kernels for the update, the preconditioner, each dot
+// product and its last sum were seven launches and 19 passes over a vector;
+// this and k_cg_p are two launches and 13.  Bound by HBM: 30.8 and 12.6 us at
+// 96^3 nodes (13 x 21 MB; 6.3 TB/s), 7 and 4 us at 29 thousand, where the
+// launches and the last block's sum are what counts.
+template <bool PRE>
+__global__ void __launch_bounds__(256) k_cg_x(double* __restrict__ x, double* __restrict__ r,
+                                              const double* __restrict__ p, const double* __restrict__ q,
+                                              const double* __restrict__ minv, double* __restrict__ z, int64_t N,
+                                              const double* __restrict__ rz, const double* __restrict__ pq, DotOut D) {
+    const double alpha = *rz / *pq;
+    double s0 = 0.0, s1 = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+        double pv[3], qv[3], rv[3], xv[3], m[6];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) pv[a] = p[a * N + i], qv[a] = q[a * N + i], rv[a] = r[a * N + i], xv[a] = x[a * N + i];
+        if (PRE) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) m[k] = minv[k * N + i];
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            x[a * N + i] = xv[a] + alpha * pv[a];
+            rv[a] = rv[a] - alpha * qv[a];
+            r[a * N + i] = rv[a];
+            s1 += rv[a] * rv[a];
+        }
+        if (PRE) {
+            const double z0 = m[0] * rv[0] + m[3] * rv[1] + m[4] * rv[2];
+            const double z1 = m[3] * rv[0] + m[1] * rv[1] + m[5] * rv[2];
+            const double z2 = m[4] * rv[0] + m[5] * rv[1] + m[2] * rv[2];
+            z[i] = z0;
+            z[N + i] = z1;
+            z[2 * N + i] = z2;
+            s0 += rv[0] * z0 + rv[1] * z1 + rv[2] * z2;
+        }
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+    block_sums(D, PRE ? s0 : s1, s1);
 }
 
-__global__ void k_dot_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-    __shared__ double sh[32];
-    double acc = 0.0;
-    for (int k = threadIdx.x; k < nb; k += 32) acc += part[k];
-    sh[threadIdx.x] = acc;
-    __syncwarp();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < 32; ++k) s += sh[k];
-        *out = s;
+// p = z + (r.z / the last r.z) p, and the operator's next input from it:
+// masked (prescribed directions zero) in FP64, in FP32, or in the records of
+// the family-list operator.
+enum { MASK_F64, MASK_F32, MASK_FAMILY };
+template <int MASK>
+__global__ void __launch_bounds__(256) k_cg_p(const double* __restrict__ z, double* __restrict__ p, Dev d,
+                                              const uint8_t* __restrict__ pmask, void* __restrict__ xm,
+                                              const double* __restrict__ rzn, const double* __restrict__ rz) {
+    const double beta = *rzn / *rz;
+    const int64_t N = d.n, i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    double v[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a] = z[a * N + i] + beta * p[a * N + i];
+    const unsigned m = pmask[i];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        p[a * N + i] = v[a];
+        if (m >> a & 1) v[a] = 0.0;
+        if (MASK == MASK_F64) static_cast<double*>(xm)[a * N + i] = v[a];
+        if (MASK == MASK_F32) static_cast<float*>(xm)[a * N + i] = (float)v[a];
     }
-}
-
-template <typename T>
-__global__ void k_cg_x(T* x, T* r, const T* p, const T* q, int64_t n, const double* scal) {
-    const double alpha = scal[CG_RR] / scal[CG_PQ];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        x[i] = (T)((double)x[i] + alpha * (double)p[i]);
-        r[i] = (T)((double)r[i] - alpha * (double)q[i]);
-    }
-}
-
-template <typename T>
-__global__ void k_cg_p(const T* r, T* p, int64_t n, const double* scal) {
-    const double beta = scal[CG_RRN] / scal[CG_RR];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = (T)((double)r[i] + beta * (double)p[i]);
-}
-
-__global__ void k_cg_swap(double* scal) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) scal[CG_RR] = scal[CG_RRN];
+    if (MASK == MASK_FAMILY)
+        static_cast<double4*>(xm)[i] = make_double4(v[0], v[1], v[2], d.sfac ? d.sfac[i] : 0.0);
 }
 
 __global__ void k_sub(const double* a, const double* b, double* o, int64_t n) {
@@ -895,18 +1166,23 @@ constexpr int kStreamBlocks = 148 * 8;
 
 }  // namespace
 
-void launch_dot_f64(const double* a, const double* b, int64_t n, double* part, double* out, cudaStream_t s) {
-    k_dot_partial<double><<<kDotBlocks, 256, 0, s>>>(a, b, n, part);
-    k_dot_final<<<1, 32, 0, s>>>(part, kDotBlocks, out);
+void launch_dot_f64(const double* a, const double* b, int64_t n, const DotOut& D, cudaStream_t s) {
+    k_dot<<<sum_blocks(n, 256), 256, 0, s>>>(a, b, n, D);
 }
-void launch_cg_update_x_f64(double* x, double* r, const double* p, const double* q, int64_t n, const double* scal,
-                            cudaStream_t s) {
-    k_cg_x<double><<<kStreamBlocks, 256, 0, s>>>(x, r, p, q, n, scal);
+void launch_cg_x(double* x, double* r, const double* p, const double* q, const double* minv, double* z, int64_t n,
+                 const double* rz, const double* pq, const DotOut& D, cudaStream_t s) {
+    const unsigned nb = sum_blocks(n, 256);
+    if (minv) k_cg_x<true><<<nb, 256, 0, s>>>(x, r, p, q, minv, z, n, rz, pq, D);
+    else k_cg_x<false><<<nb, 256, 0, s>>>(x, r, p, q, minv, z, n, rz, pq, D);
 }
-void launch_cg_update_p_f64(const double* r, double* p, int64_t n, const double* scal, cudaStream_t s) {
-    k_cg_p<double><<<kStreamBlocks, 256, 0, s>>>(r, p, n, scal);
+void launch_cg_p(const Dev& d, const StaticIn& I, bool f32, const double* z, double* p, const double* rzn,
+                 const double* rz, cudaStream_t s) {
+    if (d.n == 0) return;
+    const unsigned nb = blocks_for(d.n, 256);
+    if (I.F.xm) k_cg_p<MASK_FAMILY><<<nb, 256, 0, s>>>(z, p, d, I.F.pmask, I.F.xm, rzn, rz);
+    else if (f32) k_cg_p<MASK_F32><<<nb, 256, 0, s>>>(z, p, d, I.S.pmask, I.S.xm, rzn, rz);
+    else k_cg_p<MASK_F64><<<nb, 256, 0, s>>>(z, p, d, I.S.pmask, I.S.xm, rzn, rz);
 }
-void launch_cg_swap(double* scal, cudaStream_t s) { k_cg_swap<<<1, 32, 0, s>>>(scal); }
 void launch_sub_f64(const double* a, const double* b, double* o, int64_t n, cudaStream_t s) {
     k_sub<<<kStreamBlocks, 256, 0, s>>>(a, b, o, n);
 }

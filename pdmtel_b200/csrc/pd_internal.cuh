@@ -250,23 +250,40 @@ int persist_max_blocks(const Dev& d, int* per_sm, int* sms);
 cudaError_t launch_persist_f32c(const Dev& d, double dt, int nsteps, PersistCtl* ctl, int blocks,
                                 unsigned force_chunk, unsigned gather_chunk, PersistWait W, cudaStream_t s);
 
-// CG helpers (pd_fast.cu): slots of the device scalar array
+// CG helpers (pd_fast.cu): slots of the device scalar array.  r.z alternates
+// between CG_RR and CG_RRN.
 enum { CG_RR = 0, CG_PQ = 1, CG_RRN = 2, CG_BB = 3, CG_RES = 4, CG_NSLOT = 8 };
-void launch_dot_f64(const double* a, const double* b, int64_t n, double* part, double* out, cudaStream_t s);
-void launch_cg_update_x_f64(double* x, double* r, const double* p, const double* q, int64_t n, const double* scal, cudaStream_t s);
-void launch_cg_update_p_f64(const double* r, double* p, int64_t n, const double* scal, cudaStream_t s);
-void launch_cg_swap(double* scal, cudaStream_t s);
+// where a kernel leaves up to two sums over all its blocks: scalars
+// out[slot0], out[slot1] (slot < 0: none) through two doubles per block in
+// part and the counter done; part == nullptr: no sums
+struct DotOut {
+    double* part;
+    unsigned* done;
+    double* out;
+    int slot0, slot1;
+};
+constexpr int kSumBlocks = 148 * 8;  // most blocks of the grid-stride kernels that sum
+// the family-list static operator's node records (k_family_geo, k_family_mask)
+struct FamilyDev {
+    const double4* geo;    // [N] coordinates, spring
+    double4* xm;           // [N] masked input, spring factor
+    const uint8_t* pmask;  // [N] prescribed directions, bits 0..2
+};
+void launch_dot_f64(const double* a, const double* b, int64_t n, const DotOut& D, cudaStream_t s);
+void launch_cg_x(double* x, double* r, const double* p, const double* q, const double* minv, double* z, int64_t n,
+                 const double* rz, const double* pq, const DotOut& D, cudaStream_t s);
 void launch_sub_f64(const double* a, const double* b, double* out, int64_t n, cudaStream_t s);
-constexpr int kDotBlocks = 296;
 
 // static operator (pd_fast.cu)
-void launch_static_apply_f64(const Dev& d, double t, const double* x, double* y, cudaStream_t s);
+void launch_family_geo(const Dev& d, double4* geo, cudaStream_t s);
+// y = K x from F.xm (x masked); with D.part, x . y too.  Whether it left x . y.
+bool launch_static_family(const Dev& d, const FamilyDev& F, bool f32, const double* x, double* y, const DotOut& D,
+                          cudaStream_t s);
 // block-Jacobi preconditioner of the static operator ([6][N] symmetric
 // inverses of the 3x3 diagonal blocks) and its application z = M^-1 r
 void launch_static_bjacobi(const Dev& d, double* minv, cudaStream_t s);
 void launch_bj_apply(const double* minv, const double* r, double* z, int64_t n, cudaStream_t s);
-void launch_static_rhs(const Dev& d, double t, double* b, cudaStream_t s);
-void launch_static_apply_f32x(const Dev& d, double t, const double* x, double* y, cudaStream_t s);
+void launch_static_rhs(const Dev& d, const FamilyDev& F, double t, double* b, cudaStream_t s);
 // the static operator on a complete box lattice (node id = x + nx (y + ny z))
 // whose families are the horizon stencil clipped to the box
 constexpr int kMaxStencil = 768;  // 64 B of shared memory each: under the 48 KB default
@@ -317,6 +334,16 @@ struct StencilDev {
     const double2* ndtap;
     const double* ndiag;
     const struct NdTab* ndhost;  // host copy of the tables, passed as a kernel parameter
+    // broken bonds (a slit): the operator of the whole stencil less bfix, the
+    // broken bonds' share (k_static_broken).  bnode [nbrk] the nodes that have
+    // some, bptr / bent their entries (neighbour, slot of off / geo), bidx [N]
+    // a node's place in bnode or -1, bfix [nbrk][3]
+    int nbrk;
+    const int32_t* bnode;
+    const int64_t* bptr;
+    const int2* bent;
+    const int32_t* bidx;
+    double* bfix;
 };
 // The split form's tables as one kernel parameter (constant bank: warp-uniform
 // reads through the constant cache, no shared-memory traffic).
@@ -326,7 +353,32 @@ struct NdTab {
     int4 col[kNdMaxCol];
 };
 void launch_static_pmask(const Dev& d, uint8_t* pm, cudaStream_t s);
-void launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const double* x, double* y, cudaStream_t s);
+// setup of the stencil on a box lattice (d.lat): every full-family entry's
+// offset marked in map [128]^3 (key (ox + 64) << 14 | (oy + 64) << 7 | oz + 64)
+// and listed in any order (the first kMaxStencil; err[1] counts them all), then
+// every family's size against the nlist offsets that stay in the box and
+// map turned into list positions; err: set where a node breaks the numbering x
+// + nx (y + ny z), an offset is outside or a size differs
+void launch_box_offsets(const Dev& d, int* map, int* err, int4* list, cudaStream_t s);
+void launch_box_check(const Dev& d, const int4* list, int nlist, int* map, int* err, cudaStream_t s);
+// nodes with broken entries: flags and counts per node, and (from their scans)
+// the list that StencilDev::bnode .. bidx describe, map giving the slots
+void launch_broken_counts(const Dev& d, int64_t* flag, int64_t* cnt, cudaStream_t s);
+void launch_broken_fill(const Dev& d, const int* map, const int64_t* flag, const int64_t* fpos, const int64_t* cpos,
+                        int32_t* bnode, int64_t* bptr, int2* bent, int32_t* bidx, cudaStream_t s);
+// the operator's input: the stencil's masked vectors, or (F.xm set) the
+// family-list records
+struct StaticIn {
+    StencilDev S;
+    FamilyDev F;
+};
+void launch_static_mask(const Dev& d, const StaticIn& I, bool f32, const double* x, cudaStream_t s);
+void launch_cg_p(const Dev& d, const StaticIn& I, bool f32, const double* z, double* p, const double* rzn,
+                 const double* rz, cudaStream_t s);
+// y = K x from S.xm (x masked); with D.part, x . y too where the kernel forms
+// it (the split form).  Whether it did.
+bool launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const double* x, double* y, const DotOut& D,
+                           cudaStream_t s);
 void launch_static_ndiag(const StencilDev& S, int64_t n, double* D, cudaStream_t s);
 size_t static_nd_smem(const StencilDev& S, int R);  // shared memory of the split-form kernel
 

@@ -52,6 +52,18 @@ __device__ __forceinline__ void rn_sqrt_rcp(double a, double& s, double& y) {
     y = fma(fma(-s, y, 1.0), y, y);
 }
 
+// 1 / sqrt(a) to about 2^-51 (the iteration above without its last rounding);
+// a in rn_range
+__device__ __forceinline__ double rsqrt_near(double a) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
+    double g = a * y0, h = rn_pow2(y0, -1);
+    const double e = fma(-g, h, 0.5);
+    g = fma(g, e, g);
+    h = fma(h, e, h);
+    return rn_pow2(fma(h, fma(-g, h, 0.5), h), 1);
+}
+
 // a / b with y = 1/b; a zero or rn_quotient_ok (the quotient of a zero is +0)
 __device__ __forceinline__ double rn_div(double a, double b, double y) {
     const double q = a * y;
