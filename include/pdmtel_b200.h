@@ -116,7 +116,7 @@ int pd_ctx_destroy(pd_ctx* ctx);
 int pd_ctx_stream(pd_ctx* ctx, void** stream);
 int pd_sync(pd_ctx* ctx);
 
-/* Cell-binned, Morton-ordered family search on the device.  Replaces
+/* Cell-binned family search on the device.  Replaces
  * pdDataManager::InitBond (pdDataManager2.cpp:12-70) with its cube-distance
  * test (pdDataManager3.cpp:637-685,1573-1704); the family list of every
  * node is in ascending id order, as the reference's is.  Slit rectangles

@@ -116,7 +116,8 @@ struct pd_ctx {
     int64_t *tptr = nullptr;
     int32_t *tj = nullptr, *tpos = nullptr;
     int gpat_opt = 0;             // FP32 gather from contributor patterns (PD_OPT_GATHER_STENCIL)
-    bool have_gpat = false;       // patterns built (with the MLS data; refused when nothing repeats)
+    bool have_gpat = false;       // patterns built (refused when nothing repeats)
+    bool gpat_tried = false;      // a build was tried with the current MLS data
     int32_t* gpat_id = nullptr;
     int64_t* gpat_ptr = nullptr;
     int32_t* gpat_off = nullptr;
@@ -284,19 +285,6 @@ bool lattice_positions(const std::vector<double>& x, int64_t N, double dx, std::
         out[i] = (int32_t)(l[0] | (l[1] << 11) | (l[2] << 22));
     }
     return true;
-}
-
-uint64_t morton3(uint64_t x, uint64_t y, uint64_t z) {
-    auto spread = [](uint64_t v) {
-        v &= 0x1fffff;
-        v = (v | v << 32) & 0x1f00000000ffffull;
-        v = (v | v << 16) & 0x1f0000ff0000ffull;
-        v = (v | v << 8) & 0x100f00f00f00f00full;
-        v = (v | v << 4) & 0x10c30c30c30c30c3ull;
-        v = (v | v << 2) & 0x1249249249249249ull;
-        return v;
-    };
-    return spread(x) | spread(y) << 1 | spread(z) << 2;
 }
 
 bool ready_dynamic(pd_ctx* c) {
@@ -682,8 +670,8 @@ static int sell_prepare(pd_ctx* c) {
 // list as id offsets from the node, identical lists stored once (on a box
 // lattice numbered x + nx (y + ny z) the lists of nodes with the same
 // position relative to the boundary are translates of each other; in a
-// batch, per specimen).  Built with the MLS data (pd_set_mls), whether or not
-// a gather uses them.
+// batch, per specimen).  Built when a gather first asks for them
+// (PD_OPT_GATHER_STENCIL), and again with new MLS data while it is on.
 static void gpat_free(pd_ctx* c) {
     for (void* p : {(void*)c->gpat_id, (void*)c->gpat_ptr, (void*)c->gpat_off}) dfree(c, p);
     c->gpat_id = nullptr;
@@ -705,9 +693,21 @@ static void gpat_apply(pd_ctx* c) {
     c->generation++;
 }
 
+// The contributor ids on the host (the patterns, the adjoint's transpose and
+// pd_get_mls read them; a run that needs none of these does not copy them).
+static int mls_list_host(pd_ctx* c) {
+    const size_t T = c->cbptr_host.empty() ? 0 : (size_t)c->cbptr_host.back();
+    if (c->cbidx_host.size() == T) return PD_OK;
+    c->cbidx_host.resize(T);
+    PD_CUDA_TRY(cudaMemcpy(c->cbidx_host.data(), c->cbidx, sizeof(int32_t) * T, cudaMemcpyDeviceToHost));
+    return PD_OK;
+}
+
 static int gpat_build(pd_ctx* c) {
     gpat_free(c);
+    c->gpat_tried = true;
     if (!c->have_mls || !c->d.mls || c->n == 0) return PD_OK;
+    PD_TRY(mls_list_host(c));
     const int64_t N = c->n;
     const std::vector<int64_t>& cp = c->cbptr_host;
     const std::vector<int32_t>& ci = c->cbidx_host;
@@ -783,7 +783,9 @@ static int mls_installed(pd_ctx* c) {
     c->d.csum = c->csum;
     c->have_mls = true;
     c->generation++;
-    PD_TRY(gpat_build(c));
+    c->gpat_tried = false;
+    if (c->gpat_opt) PD_TRY(gpat_build(c));
+    else gpat_free(c);
     if (!c->have_gpat) c->gpat_opt = 0;  // the new lists do not repeat: plain lists
     gpat_apply(c);
     return sell_prepare(c);
@@ -1087,30 +1089,16 @@ int pd_bond_search(pd_ctx* c, int64_t* num_halves, int64_t* num_broken, double* 
         g.nc[a] = (int64_t)std::floor((hi[a] - lo[a]) / g.h) + 1;
         ncell *= g.nc[a];
     }
-    // Morton rank of every cell
-    std::vector<std::pair<uint64_t, int64_t>> keys(ncell);
-    for (int64_t z = 0; z < g.nc[2]; ++z)
-        for (int64_t y = 0; y < g.nc[1]; ++y)
-            for (int64_t xx = 0; xx < g.nc[0]; ++xx) {
-                int64_t lin = (z * g.nc[1] + y) * g.nc[0] + xx;
-                keys[lin] = {morton3(xx, y, z), lin};
-            }
-    std::sort(keys.begin(), keys.end());
-    std::vector<int32_t> rank(ncell);
-    for (int64_t r = 0; r < ncell; ++r) rank[keys[r].second] = (int32_t)r;
-    int32_t* drank = nullptr;
-    PD_TRY(dalloc(c, &drank, ncell));
-    int rc = upload(c, drank, rank.data(), sizeof(int32_t) * ncell);
-    if (rc != PD_OK) { dfree(c, drank); return rc; }
     double* sl = c->dslits;
     int64_t *frow, *arow;
     int32_t *fcol, *acol;
     uint8_t* fbr;
     int64_t nh = 0, nb = 0;
     double mb = 0.0;
-    rc = pd::bond_search(c->d, g, drank, ncell, c->nslit, sl, &frow, &fcol, &fbr, &arow, &acol, &nh, &nb, &mb,
-                         c->stream);
-    dfree(c, drank);
+    double reach = 0.0;
+    for (int a = 0; a < 3; ++a) reach = std::max(reach, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
+    const int rc = pd::bond_search(c->d, g, ncell, reach, c->nslit, sl, &frow, &fcol, &fbr, &arow, &acol, &nh, &nb,
+                                   &mb, c->stream);
     if (rc != PD_OK) return rc;
     install_family(c, frow, fcol, fbr, arow, acol, nh, nh - nb);
     if (num_halves) *num_halves = nh;
@@ -1268,9 +1256,8 @@ int pd_mls_setup(pd_ctx* c, double rw, const double* mls_coords, int64_t* num_co
         return fail(rc, "pd_mls_setup: device setup failed");
     }
     c->cbptr_host.resize((size_t)N + 1);
-    c->cbidx_host.resize((size_t)T);
+    c->cbidx_host.clear();  // mls_list_host copies them when something asks
     PD_CUDA_TRY(cudaMemcpy(c->cbptr_host.data(), c->cbptr, sizeof(int64_t) * (N + 1), cudaMemcpyDeviceToHost));
-    if (T) PD_CUDA_TRY(cudaMemcpy(c->cbidx_host.data(), c->cbidx, sizeof(int32_t) * T, cudaMemcpyDeviceToHost));
     if (num_contrib) *num_contrib = T;
     return mls_installed(c);
 }
@@ -1527,6 +1514,7 @@ int pd_get_mls(pd_ctx* c, int64_t* cb_ptr, int32_t* cb_idx, double* coeff) {
     const int64_t N = c->n, T = c->cbptr_host.empty() ? 0 : c->cbptr_host[N];
     const int npt = c->npt;
     std::memcpy(cb_ptr, c->cbptr_host.data(), sizeof(int64_t) * (N + 1));
+    if (cb_idx) PD_TRY(mls_list_host(c));
     if (cb_idx && T) std::memcpy(cb_idx, c->cbidx_host.data(), sizeof(int32_t) * T);
     if (coeff && T) {
         std::vector<double> co((size_t)T * npt);
@@ -1611,6 +1599,7 @@ int pd_set_option(pd_ctx* c, int option, int64_t value) {
             break;
         case PD_OPT_GATHER_STENCIL:
             if (value > 1) return fail(PD_ERR_ARG, "pd_set_option: 0 or 1");
+            if (value && !c->gpat_tried) PD_TRY(gpat_build(c));
             if (value && !c->have_gpat)
                 return fail(PD_ERR_ARG, "pd_set_option: the MLS contributor lists do not repeat (no patterns)");
             c->gpat_opt = (int)value;
@@ -2537,6 +2526,7 @@ void enqueue_step_tape(pd_ctx* c, double dt, double* tape, bool f32) {
 // transpose of the contributor lists of nodes without a boundary condition
 int build_transpose(pd_ctx* c) {
     if (c->tptr) return PD_OK;
+    PD_TRY(mls_list_host(c));
     const int64_t N = c->n;
     std::vector<int64_t> cnt(N + 1, 0);
     for (int64_t j = 0; j < N; ++j) {

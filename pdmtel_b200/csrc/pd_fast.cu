@@ -908,36 +908,59 @@ __global__ void k_scan_add(int64_t* out, int64_t n, const int64_t* __restrict__ 
     if (i < n) out[i] += boff[blockIdx.x];
 }
 
-__global__ void k_scan_total(const int64_t* in, int64_t* out, int64_t n) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) out[n] = (n > 0) ? out[n - 1] + in[n - 1] : 0;
+// One block: the blocks' offsets from their sums, and the total.
+__global__ void __launch_bounds__(kScanBlock) k_scan_sums(const int64_t* __restrict__ bsum, int64_t* __restrict__ boff,
+                                                          int64_t nb, int64_t* __restrict__ total) {
+    __shared__ int64_t wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int64_t carry = 0;
+    for (int64_t base = 0; base < nb; base += kScanBlock) {
+        const int64_t i = base + threadIdx.x;
+        const int64_t v = i < nb ? bsum[i] : 0;
+        int64_t x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[w] = x;
+        __syncthreads();
+        int64_t before = carry, all = carry;
+        for (int k = 0; k < 32; ++k) {
+            if (k < w) before += wsum[k];
+            all += wsum[k];
+        }
+        if (i < nb) boff[i] = before + x - v;
+        carry = all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *total = carry;
 }
 
 }  // namespace
 
-int exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s) {
+int64_t scan_words(int64_t n) { return 2 * (n / kScanBlock + 2); }
+
+int exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s, int64_t* scratch) {
     if (n <= 0) {
         int64_t z = 0;
         if (cudaMemcpyAsync(out, &z, sizeof(z), cudaMemcpyHostToDevice, s) != cudaSuccess) return PD_ERR_CUDA;
         return cudaStreamSynchronize(s) == cudaSuccess ? PD_OK : PD_ERR_CUDA;
     }
     const int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-    int64_t *bsum = nullptr, *boff = nullptr;
-    if (cudaMalloc(&bsum, sizeof(int64_t) * (nb + 1)) != cudaSuccess) return PD_ERR_OOM;
-    if (cudaMalloc(&boff, sizeof(int64_t) * (nb + 1)) != cudaSuccess) {
-        cudaFree(bsum);
-        return PD_ERR_OOM;
+    int64_t* own = nullptr;
+    if (!scratch) {
+        if (cudaMalloc(&own, sizeof(int64_t) * scan_words(n)) != cudaSuccess) return PD_ERR_OOM;
+        scratch = own;
     }
+    int64_t *bsum = scratch, *boff = scratch + nb;
     k_scan_block<<<(unsigned)nb, kScanBlock, 0, s>>>(in, out, n, bsum);
-    int rc = PD_OK;
-    if (nb > 1) {
-        rc = exclusive_scan_i64(bsum, boff, nb, s);
-        if (rc == PD_OK) k_scan_add<<<(unsigned)nb, kScanBlock, 0, s>>>(out, n, boff);
+    k_scan_sums<<<1, kScanBlock, 0, s>>>(bsum, boff, nb, out + n);
+    if (nb > 1) k_scan_add<<<(unsigned)nb, kScanBlock, 0, s>>>(out, n, boff);
+    int rc = cudaGetLastError() == cudaSuccess ? PD_OK : PD_ERR_CUDA;
+    if (own) {
+        if (cudaStreamSynchronize(s) != cudaSuccess) rc = PD_ERR_CUDA;
+        cudaFree(own);
     }
-    if (rc == PD_OK) k_scan_total<<<1, 32, 0, s>>>(in, out, n);
-    if (rc == PD_OK && cudaGetLastError() != cudaSuccess) rc = PD_ERR_CUDA;
-    if (cudaStreamSynchronize(s) != cudaSuccess) rc = PD_ERR_CUDA;
-    cudaFree(bsum);
-    cudaFree(boff);
     return rc;
 }
 

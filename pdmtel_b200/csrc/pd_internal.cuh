@@ -204,9 +204,10 @@ struct SearchGrid {
     double h;
     int64_t nc[3];
 };
-int bond_search(const Dev& d, const SearchGrid& g, const int32_t* cell_rank, int64_t ncell, int nslit,
-                const double* slits_dev, int64_t** frow, int32_t** fcol, uint8_t** fbroken, int64_t** arow,
-                int32_t** acol, int64_t* nh, int64_t* nb, double* min_bond, cudaStream_t s);
+// (reach: the largest |coordinate|)
+int bond_search(const Dev& d, const SearchGrid& g, int64_t ncell, double reach, int nslit, const double* slits_dev,
+                int64_t** frow, int32_t** fcol, uint8_t** fbroken, int64_t** arow, int32_t** acol, int64_t* nh,
+                int64_t* nb, double* min_bond, cudaStream_t s);
 
 // adaptive-trapezoid (AI) form (pd_ai.cu, compiled without FMA contraction):
 // the MLS table gather of a stage and the force stage
@@ -403,7 +404,10 @@ void launch_adj_stage_post(const Dev& d, double alpha, double* lk_prev, const Ad
 void launch_adj_stage1_end(const Dev& d, const AdjBuf& A, cudaStream_t s);
 
 // scans and reductions (pd_fast.cu)
-int exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s);  // out has n+1 entries
+// out has n+1 entries; scratch: scan_words(n) words of the caller's, which then
+// has to wait for the stream itself, or null
+int64_t scan_words(int64_t n);
+int exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s, int64_t* scratch = nullptr);
 
 }  // namespace pd
 
