@@ -451,19 +451,176 @@ __device__ __forceinline__ void force_pair(const Dev& d, const PointPack<8>& G, 
     force_nodes<HASFAIL, LAT, BDRY, SFAC, MULTIMAT, PERSIST, false>(d, G, dts, ia, ib, pstage, dt, t, SmemTile{});
 }
 
-template <bool HASFAIL, bool LAT, bool BDRY, bool SFAC, bool MULTIMAT>
-__global__ void __launch_bounds__(128, 4) k_force_f32c_pair(Dev d, PointPack<8> G, double dts) {
-    const int64_t t2 = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
-    if (t2 >= d.n) return;
-    force_pair<HASFAIL, LAT, BDRY, SFAC, MULTIMAT, false>(d, G, dts, t2, 0, 0.0, 0.0);
+// 16 bytes to shared memory through L1
+__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gsrc) : "memory");
+}
+
+// pt_geo for two points at once, lane by lane the operations of pt_geo.
+__device__ __forceinline__ void pt_geo2(const PointF& P0, const PointF& P1, f2 x0, f2 x1, f2 x2, f2& K, f2& r2inv) {
+    const f2 r2 = f2_fma(x0, x0, f2_fma(x1, x1, f2_mul(x2, x2)));
+    float l, h;
+    f2_split(r2, l, h);
+    const f2 rinv = f2_make(rsqrtf(l), rsqrtf(h));
+    const f2 r = f2_mul(r2, rinv);
+    const f2 t = f2_mul(f2_fma(r, f2_make(-1.f, -1.f), f2_make(P0.A, P1.A)), f2_make(P0.B, P1.B));
+    f2_split(t, l, h);
+    K = f2_mul(f2_mul(f2_make(P0.W, P1.W), f2_make(__saturatef(l), __saturatef(h))), rinv);
+    r2inv = f2_mul(rinv, rinv);
+}
+
+// A bond with a point outside the series range, from its staged block.
+template <bool HASFAIL>
+__device__ __noinline__ void bond_exact(const PointPack<8>& G, const float* blk, float x0, float x1, float x2, float u0,
+                                        float u1, float u2, float epsc, float* F) {
+    const float dx[3] = {x0, x1, x2}, du[3] = {u0, u1, u2};
+    for (int k = 0; k < 6; ++k) F[k] = 0.f;
+    for (int q = 0; q < 8; q += 4) {
+        float u4[12];
+        for (int k = 0; k < 12; ++k) u4[k] = blk[8 * (k >> 2) + q + (k & 3)];
+        bond4<HASFAIL>(G, q, u4, dx, du, epsc, F);
+    }
+}
+
+// Shared words per group of bond products: the groups' words that are read
+// together lie in different banks.
+__host__ __device__ constexpr int lane_group_words(int L) { return L == 4 ? 20 : 3 * L + 4; }
+
+// L lanes per node, each evaluating one bond of the family with the eight
+// points two per packed instruction (the even point in the low lane, the odd
+// in the high lane: the two chains of bond4); three lanes of the group then
+// add the round's bonds to the family sum in ascending order, so every sum has
+// the terms of the pair kernel in its order and the result is the same bit for
+// bit.  A round's 32 neighbour blocks (128 bytes each) are copied to shared
+// memory a round ahead, eight lanes to a block, so that a load touches four
+// lines where a lane reading its own neighbour would touch 32.
+template <bool HASFAIL, bool LAT, bool BDRY, bool SFAC, bool MULTIMAT, int L, bool CM>
+__global__ void __launch_bounds__(128, 4) k_force_f32c_lanes(Dev d, const __grid_constant__ PointPack<8> G, double dts) {
+    constexpr int GS = lane_group_words(L);
+    constexpr int kRow = kTileStride;
+    extern __shared__ float4 lane_sm[];
+    const int lane = threadIdx.x & 31, ql = lane % L, grp = lane / L;
+    float* stage = reinterpret_cast<float*>(lane_sm) + (threadIdx.x >> 5) * (2 * 32 * kRow + 32 / L * GS);
+    float* prod = stage + 2 * 32 * kRow + grp * GS;
+    const int64_t N = d.n;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
+    const bool live = slot < N;
+    const int64_t i = d.order[live ? slot : 0];
+    Own O;
+    load_own<LAT, BDRY, SFAC, MULTIMAT>(d, i, O);
+    const int64_t row = d.arow[i];
+    const int cnt = live ? (int)(d.arow[i + 1] - row) : 0;
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    const float h = (float)d.dx;
+    float sum = 0.f, comp = 0.f;  // Kahan sum of component ql of the family force (ql < 3)
+    auto neighbour = [&](int base) { return base + ql < cnt ? d.acol[row + base + ql] : (int)i; };
+    auto fetch = [&](int j, int buf) {  // the blocks of the warp's 32 neighbours
+        float* to = stage + buf * 32 * kRow + (CM ? lane * kRow : (lane >> 3) * kRow + 4 * (lane & 7));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (CM) {
+                cp_async16(to + 4 * k, d.nblk + 4 * (k * N + j));
+            } else {
+                const int jk = __shfl_sync(0xffffffffu, j, 4 * k + (lane >> 3));
+                cp_async16(to + 4 * k * kRow, d.nblk + (int64_t)jk * 32 + 4 * (lane & 7));
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // ids are loaded two rounds ahead, lattice positions and blocks one
+    int j = neighbour(0), jn = neighbour(L);
+    int lj = LAT ? d.lat[j] : 0;
+    if (most > 0) fetch(j, 0);
+    int buf = 0;
+    for (int base = 0; base < most; base += L, buf ^= 1) {
+        const int jnn = neighbour(base + 2 * L);
+        const int ljn = LAT ? d.lat[jn] : 0;
+        if (base + L < most) fetch(jn, buf ^ 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        float dx[3];
+        if (LAT) {
+            dx[0] = __fmul_rn((float)((lj & 2047) - (O.lat & 2047)), h);
+            dx[1] = __fmul_rn((float)(((lj >> 11) & 2047) - ((O.lat >> 11) & 2047)), h);
+            dx[2] = __fmul_rn((float)((lj >> 22) - (O.lat >> 22)), h);  // packed values are non-negative
+        } else {
+            const float4 s0 = ld4(d.sblk + 8 * (int64_t)j), s1 = ld4(d.sblk + 8 * (int64_t)j + 4);
+            const float pj[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
+            for (int a = 0; a < 3; ++a) dx[a] = (pj[a] - O.ph[a]) + (pj[3 + a] - O.pl[a]);
+        }
+        float c = O.c, ecrit = O.e;
+        if (MULTIMAT) {
+            const int mj = d.mat[j];
+            c = fminf(c, (float)d.mats[mj].spring);
+            ecrit = fminf(ecrit, (float)d.mats[mj].ecrit);
+        }
+        if (BDRY || SFAC) {
+            const float2 v = __ldg(reinterpret_cast<const float2*>(d.sblk + 8 * (int64_t)j + 6));
+            if (BDRY) c *= 0.5f * (O.be + v.x);
+            if (SFAC) c *= 0.5f * (O.sf + v.y);
+        }
+        const float epsc = HASFAIL ? eps_crit(ecrit) : 0.f;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const float* bj = stage + buf * 32 * kRow + lane * kRow;
+        const float4 us0 = *reinterpret_cast<const float4*>(bj + 24), us1 = *reinterpret_cast<const float4*>(bj + 28);
+        const float du[3] = {split_diff(us0.x, us0.w, O.uh[0], O.ul[0]), split_diff(us0.y, us1.x, O.uh[1], O.ul[1]),
+                             split_diff(us0.z, us1.y, O.uh[2], O.ul[2])};
+        const f2 d0 = f2_make(dx[0], dx[0]), d1 = f2_make(dx[1], dx[1]), d2 = f2_make(dx[2], dx[2]);
+        const f2 u0 = f2_make(du[0], du[0]), u1 = f2_make(du[1], du[1]), u2 = f2_make(du[2], du[2]);
+        f2 F[3] = {0ull, 0ull, 0ull};
+        bool wide = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const PointF &P0 = G.p[2 * k], &P1 = G.p[2 * k + 1];
+            const f2 x0 = f2_add(d0, f2_make(P0.hx, P1.hx)), x1 = f2_add(d1, f2_make(P0.hy, P1.hy)),
+                     x2 = f2_add(d2, f2_make(P0.hz, P1.hz));
+            f2 K, r2inv;
+            pt_geo2(P0, P1, x0, x1, x2, K, r2inv);
+            const f2 gx = *reinterpret_cast<const f2*>(bj + 2 * k), gy = *reinterpret_cast<const f2*>(bj + 8 + 2 * k),
+                     gz = *reinterpret_cast<const f2*>(bj + 16 + 2 * k);
+            pt_force2<HASFAIL, true>(x0, x1, x2, K, r2inv, f2_add(u0, gx), f2_add(u1, gy), f2_add(u2, gz), epsc, F,
+                                     &wide);
+        }
+        float F6[6];
+        f2_split(F[0], F6[0], F6[3]);
+        f2_split(F[1], F6[1], F6[4]);
+        f2_split(F[2], F6[2], F6[5]);
+        if (wide) bond_exact<HASFAIL>(G, bj, dx[0], dx[1], dx[2], du[0], du[1], du[2], epsc, F6);
+        float Fb[3];
+        chains_sum(F6, Fb);
+        prod[3 * ql] = __fmul_rn(Fb[0], c);
+        prod[3 * ql + 1] = __fmul_rn(Fb[1], c);
+        prod[3 * ql + 2] = __fmul_rn(Fb[2], c);
+        __syncwarp();
+        if (ql < 3) {
+#pragma unroll 8
+            for (int q = 0; q < L; ++q) {
+                if (base + q >= cnt) continue;
+                const float y = prod[3 * q + ql] - comp, t = sum + y;
+                comp = (t - sum) - y;
+                sum = t;
+            }
+        }
+        __syncwarp();
+        j = jn;
+        jn = jnn;
+        lj = ljn;
+    }
+    if (live && ql < 3) {
+        const MatDev& M = d.mats[O.mat];
+        const double rho = M.density;
+        const double v0 = d.vbuf[ql * N + i];
+        d.vbuf[ql * N + i] = v0 + ((double)sum - (double)comp + (double)cnt * (M.grav[ql] * rho)) * dts / rho;
+    }
 }
 
 // Four nodes per thread: the work-order slots t4 .. t4+3 (x-adjacent in a
 // node order whose tiles are at least four nodes wide) walk the merge of their
 // four ascending family lists, so a neighbour block loaded once serves up to
-// four bonds (the pair kernel: two).  Nodes on one lattice, one material, no
+// four bonds.  Nodes on one lattice, one material, no
 // failure test.  Per node the same arithmetic in the same order as
-// k_force_f32c_pair, so the same result bit for bit.
+// the lane kernel, so the same result bit for bit.
 template <bool BDRY, bool SFAC>
 __global__ void __launch_bounds__(128, 3) k_force_f32c_quad(Dev d, PointPack<8> G, double dts) {
     const int64_t N = d.n;
@@ -546,7 +703,7 @@ __global__ void __launch_bounds__(128, 3) k_force_f32c_quad(Dev d, PointPack<8> 
 // node blocks chunk-major, so that the 16 pairs of a warp row read a
 // neighbour chunk from 1 KB of contiguous memory (8 lines instead of 32).
 // Per node the same bond4 arithmetic in the same ascending neighbour order
-// as the pair kernel's lattice variants: the same result bit for bit.
+// as the lane kernel's lattice variants: the same result bit for bit.
 // (A first table of the geometric terms in global memory, read one float4
 // per point, was slower than computing them: a warp-wide broadcast from L1
 // still costs a wavefront per load.  The table below lives in shared memory,
@@ -850,7 +1007,7 @@ __global__ void k_sten_masks(Dev d, const int* __restrict__ lut, int R, uint32_t
 // where a warp's 32 loads of different nodes take a few wavefronts instead
 // of one L1 wavefront per node.  Thread t takes the x-adjacent pair of
 // positions (x0 + 2 px, x0 + 2 px + 1) of the tile.  Same arithmetic per node
-// as k_force_f32c_pair, so the same result bit for bit.
+// as the lane kernel, so the same result bit for bit.
 template <bool HASFAIL, bool BDRY, bool SFAC, bool MULTIMAT>
 __global__ void __launch_bounds__(256, 1) k_force_f32c_tiled(Dev d, PointPack<8> G, double dts) {
     extern __shared__ float4 smem4[];
@@ -1222,11 +1379,7 @@ __global__ void __launch_bounds__(256) k_gather_f32c(Dev d, const double* __rest
 
 // 16-byte copy global -> shared that the thread waits for later (L2 only:
 // the coefficient stream is read once).
-__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gsrc) : "memory");
-}
-// the same with an L2 eviction policy (the coefficient stream is read once
+// 16 bytes to shared memory with an L2 eviction policy (the coefficient stream is read once
 // per gather: evict it first, so that the node blocks the force reads next
 // stay in L2)
 __device__ __forceinline__ uint64_t l2_evict_first() {
@@ -1623,6 +1776,18 @@ void launch_blocks_to_ug(const Dev& d, double* ug, cudaStream_t s) {
     if (d.n) k_blocks_to_ug<<<blocks_for(d.n, 256), 256, 0, s>>>(d, ug);
 }
 
+// Lanes per node of k_force_f32c_lanes: a warp while nodes are too few to fill
+// the SMs (16.4 us at 1,001 nodes), eight above (26 thousand nodes 100 us, 32
+// thousand 121; four lanes 114 and 127), four for large problems, whose family
+// sums then take fewer steps (640,000 nodes 1562 -> 1421 us).
+inline int force_lanes(const Dev& d) { return d.n < 12288 ? 32 : (d.n < 131072 ? 8 : 4); }
+// With the stencil force on, a box (or batch) of fewer nodes than this takes
+// k_force_f32c_lanes on the chunk-major blocks: a stencil tile is one thread
+// per node pair walking the whole stencil, 240 to 300 us however few tiles
+// there are (5,500 nodes 296 us against 39, 50,000 238 against 167, 80,000 299
+// against 298, a batch of 97,000 375 against 432).
+constexpr int64_t kStencilFrom = 65536;
+
 void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
     if (d.n == 0) return;
     const unsigned nb = blocks_for(d.n, 128);
@@ -1632,8 +1797,29 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
         else k_force_f32c_cci<false><<<nb, 128, 0, s>>>(d, dts);
         return;
     }
+    const int lanes = force_lanes(d);
+    const unsigned nbl = blocks_for(lanes * d.n, 128);
+    const size_t shl = 4 * sizeof(float) * (2 * 32 * kTileStride + 32 / lanes * lane_group_words(lanes));
+    if (d.blk_cm && d.sten_mask && d.npt == 8 && d.gc_host && d.n < kStencilFrom) {
+        const bool bd = d.bdry_on != 0, sf = d.sfac != nullptr;
+        const PointPack<8> P = pack_points<8>(d, d.gc_host);
+#define PD_STEN_L(HF, BD, SF)                                                                                  \
+    do {                                                                                                       \
+        if (lanes == 32) k_force_f32c_lanes<HF, true, BD, SF, false, 32, true><<<nbl, 128, shl, s>>>(d, P, dts); \
+        else k_force_f32c_lanes<HF, true, BD, SF, false, 8, true><<<nbl, 128, shl, s>>>(d, P, dts);             \
+    } while (0)
+        if (d.hasfail) {
+            if (bd) { if (sf) PD_STEN_L(true, true, true); else PD_STEN_L(true, true, false); }
+            else { if (sf) PD_STEN_L(true, false, true); else PD_STEN_L(true, false, false); }
+        } else {
+            if (bd) { if (sf) PD_STEN_L(false, true, true); else PD_STEN_L(false, true, false); }
+            else { if (sf) PD_STEN_L(false, false, true); else PD_STEN_L(false, false, false); }
+        }
+#undef PD_STEN_L
+        return;
+    }
     if (d.blk_cm && d.sten_mask && d.npt == 8 && d.gc_host) {
-        // the gather stores chunk-major blocks: only this kernel reads them
+        // the gather stores chunk-major blocks
         const unsigned nbk = (unsigned)d.sten_ntiles;
         const bool bd = d.bdry_on != 0, sf = d.sfac != nullptr;
         const PointPack<8> P = pack_points<8>(d, d.gc_host);
@@ -1684,9 +1870,13 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
     }
     if (d.npt == 8 && d.gc_host) {
         const PointPack<8> P = pack_points<8>(d, d.gc_host);
-        const unsigned np = blocks_for((d.n + 1) / 2, 128);
         const bool lat = d.lat != nullptr, bd = d.bdry_on != 0, sf = d.sfac != nullptr;
-#define PD_F32(HF, LT, BD, SF, MM) k_force_f32c_pair<HF, LT, BD, SF, MM><<<np, 128, 0, s>>>(d, P, dts)
+#define PD_F32(HF, LT, BD, SF, MM)                                                         \
+    do {                                                                                   \
+        if (lanes == 32) k_force_f32c_lanes<HF, LT, BD, SF, MM, 32, false><<<nbl, 128, shl, s>>>(d, P, dts); \
+        else if (lanes == 8) k_force_f32c_lanes<HF, LT, BD, SF, MM, 8, false><<<nbl, 128, shl, s>>>(d, P, dts); \
+        else k_force_f32c_lanes<HF, LT, BD, SF, MM, 4, false><<<nbl, 128, shl, s>>>(d, P, dts); \
+    } while (0)
         if (d.hasfail || d.multimat) {
             PD_F32(true, false, true, true, true);
         } else if (lat) {
