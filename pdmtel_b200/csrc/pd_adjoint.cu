@@ -12,11 +12,15 @@
 // c_min / 2 of it.  A Gauss point whose stretch is past the critical one
 // carries no force, and none of its derivative (the test itself is a step).
 //
-// Both halves are gathers: k_vjp_own runs over node i's family and writes
-// dJ/du_i; k_vjp_partner runs over node j's family (the family relation is
-// symmetric) and writes dJ/dug of j's Gauss points.  No atomics, so the
-// gradient is deterministic.
+// Both halves are gathers without atomics, so the gradient is deterministic.
+// With 2x2x2 points every evaluation (i, j, g) serves both: k_vjp_bonds runs
+// over node j's family, sums dJ/dug of j's Gauss points in registers and leaves
+// each bond's share of dJ/du_i and dJ/dc in i's own entry of the bond, which
+// k_vjp_nodes then sums.  Other rules (and families that are not symmetric)
+// evaluate twice: k_vjp_own over node i's family for dJ/du_i, k_vjp_partner
+// over node j's for dJ/dug.
 #include "pd_internal.cuh"
+#include "pd_rn.cuh"
 
 namespace pd {
 
@@ -241,6 +245,225 @@ __global__ void __launch_bounds__(256) k_vjp_partner(Dev d, const double* __rest
     if (live && lane == 0 && d.sfac) gradf[j] += gf;
 }
 
+// 1 / v for v in rn_range, to about 2^-52
+__device__ __forceinline__ double rcp_near(double v) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    y = fma(fma(-v, y, 1.0), y, y);
+    return fma(fma(-v, y, 1.0), y, y);
+}
+
+// The place of every unbroken family entry's mirror: entry p of node j's row
+// is (j, i), mirror[p] the entry (i, j) of node i's row.  err: set where there
+// is none.
+__global__ void __launch_bounds__(256) k_mirror(Dev d, int64_t* __restrict__ mirror, int* __restrict__ err) {
+    const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (j >= d.n) return;
+    for (int64_t p = d.arow[j] + (threadIdx.x & 31); p < d.arow[j + 1]; p += 32) {
+        const int32_t i = d.acol[p];
+        int64_t lo = d.arow[i], hi = d.arow[i + 1] - 1;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (d.acol[mid] < (int32_t)j) lo = mid + 1;
+            else hi = mid;
+        }
+        const bool found = lo <= hi && d.acol[lo] == (int32_t)j;
+        mirror[p] = found ? lo : p;
+        if (!found) atomicOr(err, 1);
+    }
+}
+
+// One point of k_vjp_bonds whose lengths are outside the range of rsqrt_near:
+// (dJ/dug, its share of dJ/dc) by the general terms, out of line.
+__device__ __noinline__ double4 bond_point_any(const Dev& d, int g, double x0, double x1, double x2, double e0, double e1,
+                                               double e2, double l0, double l1, double l2, double ecrit, double bE,
+                                               double c) {
+    PointTerms T;
+    if (!point_terms(d, d.gc[g], x0, x1, x2, e0, e1, e2, l0, l1, l2, ecrit, bE, T)) return make_double4(0, 0, 0, 0);
+    const double k = T.bw * c;
+    return make_double4(k * (T.a * l0 + T.y0 * T.q), k * (T.a * l1 + T.y1 * T.q), k * (T.a * l2 + T.y2 * T.q),
+                        T.bw * T.a * (T.y0 * l0 + T.y1 * l1 + T.y2 * l2));
+}
+
+// What a bond reads of its far node, 96 bytes side by side: coordinates, the
+// displacement the stage's force used, the force's adjoint, spring factor,
+// boundary factor, and the material (as a double).
+constexpr int kVjpRec = 12;
+__global__ void k_vjp_pack(Dev d, const double* __restrict__ teU, const double* __restrict__ teus,
+                           const double* __restrict__ lamF, double* __restrict__ rec) {
+    const int64_t N = d.n, i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    double u[3];
+    ueff(d, teU, teus, i, u);
+    double* r = rec + kVjpRec * i;
+    for (int a = 0; a < 3; ++a) {
+        r[a] = d.x[a * N + i];
+        r[3 + a] = u[a];
+        r[6 + a] = lamF[a * N + i];
+    }
+    r[9] = d.sfac ? d.sfac[i] : 1.0;
+    r[10] = d.bdry[i];
+    r[11] = (double)d.mat[i];
+}
+
+// 2x2x2 points: L lanes per node j, each taking one bond (i, j) with its eight
+// points.  The cell's own data (24 point displacements, six offsets) are the
+// same for the group, a bond needs only its far node's record, copied to shared
+// memory a round ahead, and the 24 sums of dJ/dug stay in registers until the
+// lanes are added.  bond[mirror] receives the bond's (dJ/du_i, its factor
+// gradient).
+//
+// Two passes of eight lanes per node, a lane per point, evaluated every point
+// twice, gathered 24 displacements per bond in one of them and formed the roots
+// and the division with the library's routines: 0.81 + 0.66 ms for 32,768 nodes
+// (51.1M points); 0.58 ms here and 0.04 in k_vjp_nodes.  FP64 pipe 41 % busy at
+// eight warps per SM (254 registers; three blocks at 168 spill and measured the
+// same): bound by the latency of its chains.
+template <int L>
+__global__ void __launch_bounds__(128, 2) k_vjp_bonds(Dev d, const double* __restrict__ rec,
+                                                      const double* __restrict__ teug, double* __restrict__ lam_ug,
+                                                      double* __restrict__ gradf, const int64_t* __restrict__ mirror,
+                                                      double4* __restrict__ bond) {
+    constexpr int kRow = 14;  // shared doubles per record: 16-byte aligned, rows spread over the banks
+    __shared__ double su[128 / L][24];
+    __shared__ __align__(16) double sr[2][128][kRow];
+    const int64_t N = d.n;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
+    const int ql = threadIdx.x % L;
+    const bool live = slot < N;
+    const int64_t j = d.order[live ? slot : 0];
+    const double xj0 = d.x[j], xj1 = d.x[N + j], xj2 = d.x[2 * N + j];
+    const double hl = d.gc[0].hg[2], hh = d.gc[1].hg[2];
+    const MatDev Mj = d.mats[d.mat[j]];
+    const double bEj = d.bdry[j], sfj = d.sfac ? d.sfac[j] : 1.0;
+    double* u = su[threadIdx.x / L];
+    for (int k = ql; k < 24; k += L) u[k] = teug[k * N + j];
+    __syncwarp();
+    double o[24];
+#pragma unroll
+    for (int k = 0; k < 24; ++k) o[k] = 0.0;
+    double gf = 0.0;
+    const int64_t pe = live ? d.arow[j + 1] : 0;
+    const int64_t p0 = (live ? d.arow[j] : 0) + ql;
+    auto id = [&](int64_t p) { return p < pe ? d.acol[p] : (int)j; };
+    auto fetch = [&](int64_t i, int buf) {
+#pragma unroll
+        for (int k = 0; k < kVjpRec; k += 2) {
+            const unsigned sa = (unsigned)__cvta_generic_to_shared(&sr[buf][threadIdx.x][k]);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(rec + kVjpRec * i + k) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int inext = id(p0 + L);
+    fetch(id(p0), 0);
+    int buf = 0;
+    for (int64_t p = p0; p < pe; p += L, buf ^= 1) {
+        const int i2 = id(p + 2 * L);
+        fetch(inext, buf ^ 1);
+        inext = i2;
+        const int64_t mp = mirror[p];
+        asm volatile("cp.async.wait_group 1;" ::: "memory");  // a thread reads back only what it copied
+        const double* R = sr[buf][threadIdx.x];
+        const double ui[3] = {R[3], R[4], R[5]};
+        const double l0 = R[6], l1 = R[7], l2 = R[8];
+        double cmin = Mj.spring, ecrit = Mj.ecrit;
+        if (d.nmat > 1) {
+            const MatDev& Mi = d.mats[(int)R[11]];
+            cmin = Mj.spring < Mi.spring ? Mj.spring : Mi.spring;
+            ecrit = fmin(Mi.ecrit, Mj.ecrit);
+        }
+        const double c = d.sfac ? cmin * (0.5 * (R[9] + sfj)) : cmin;
+        const double bE = 0.5 * (R[10] + bEj);
+        const double dx0 = xj0 - R[0], dx1 = xj1 - R[1], dx2 = xj2 - R[2];
+        const double xa[2] = {hl + dx0, hh + dx0}, xb[2] = {hl + dx1, hh + dx1}, xc[2] = {hl + dx2, hh + dx2};
+        double w0 = 0.0, w1 = 0.0, w2 = 0.0, gc = 0.0;
+        unsigned out = 0;  // points for bond_point_any
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            const GaussConst& G = d.gc[g];
+            const double x0 = xa[g >> 2], x1 = xb[(g >> 1) & 1], x2 = xc[g & 1];
+            const double e0 = u[3 * g] - ui[0], e1 = u[3 * g + 1] - ui[1], e2 = u[3 * g + 2] - ui[2];
+            const double y0 = x0 + e0, y1 = x1 + e1, y2 = x2 + e2;
+            const double r2 = x0 * x0 + x1 * x1 + x2 * x2, p2 = y0 * y0 + y1 * y1 + y2 * y2;
+            const double rinv = rsqrt_near(r2), ip = rsqrt_near(p2);
+            const bool in = rn_range(r2) && rn_range(p2);
+            const double r = r2 * rinv, pl = p2 * ip, sum = pl + r;
+            // p - r = eta.(2 xi + eta) / (p + r)
+            const double q2 = e0 * (x0 + y0) + e1 * (x1 + y1) + e2 * (x2 + y2);
+            const double ext = q2 * rcp_near(sum);
+            const double st = ext * rinv;
+            const double beta = r <= d.delta - 0.5 * G.dxe ? 1.0
+                                : r <= d.delta + 0.5 * G.dxe ? (d.delta + 0.5 * G.dxe - r) * G.ydxe
+                                                             : 0.0;
+            const double bw = ext > 0.0 && st > ecrit ? 0.0 : bE * beta * G.W;
+            const double a = st * ip;  // 1/r - 1/p
+            const double yl = y0 * l0 + y1 * l1 + y2 * l2;
+            const double q = yl * ip * ip * ip, k = bw * c;
+            double t0 = k * (a * l0 + y0 * q), t1 = k * (a * l1 + y1 * q), t2 = k * (a * l2 + y2 * q);
+            t0 = in ? t0 : 0.0, t1 = in ? t1 : 0.0, t2 = in ? t2 : 0.0;
+            out |= in ? 0u : 1u << g;
+            o[3 * g] += t0;
+            o[3 * g + 1] += t1;
+            o[3 * g + 2] += t2;
+            w0 += t0;
+            w1 += t1;
+            w2 += t2;
+            gc += in ? bw * a * yl : 0.0;
+        }
+        if (out) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                if (!(out >> g & 1)) continue;
+                const double4 t = bond_point_any(d, g, xa[g >> 2], xb[(g >> 1) & 1], xc[g & 1], u[3 * g] - ui[0],
+                                                 u[3 * g + 1] - ui[1], u[3 * g + 2] - ui[2], l0, l1, l2, ecrit, bE, c);
+                o[3 * g] += t.x, o[3 * g + 1] += t.y, o[3 * g + 2] += t.z;
+                w0 += t.x, w1 += t.y, w2 += t.z;
+                gc += t.w;
+            }
+        }
+        gc *= 0.5 * cmin;
+        gf += gc;
+        bond[mp] = make_double4(-w0, -w1, -w2, gc);
+    }
+    gf = lane_sum<L>(gf);
+    if (live && ql == 0 && d.sfac) gradf[j] += gf;
+#pragma unroll
+    for (int k = 0; k < 24; ++k) {
+        const double v = lane_sum<L>(o[k]);
+        if (live && k % L == ql) lam_ug[k * N + j] = v;
+    }
+}
+
+// dJ/du_i and the factor gradient of node i from its bonds' shares
+template <int L>
+__global__ void __launch_bounds__(128) k_vjp_nodes(Dev d, const double4* __restrict__ bond, double* __restrict__ lam_u,
+                                                   double* __restrict__ gradf) {
+    const int64_t N = d.n;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
+    const int ql = threadIdx.x % L;
+    const bool live = slot < N;
+    const int64_t i = live ? slot : 0;
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0, gf = 0.0;
+    const int64_t pe = live ? d.arow[i + 1] : 0;
+#pragma unroll 4
+    for (int64_t p = (live ? d.arow[i] : 0) + ql; p < pe; p += L) {
+        const double4 b = bond[p];
+        a0 += b.x;
+        a1 += b.y;
+        a2 += b.z;
+        gf += b.w;
+    }
+    a0 = lane_sum<L>(a0);
+    a1 = lane_sum<L>(a1);
+    a2 = lane_sum<L>(a2);
+    gf = lane_sum<L>(gf);
+    if (!live || ql) return;
+    lam_u[i] = a0;
+    lam_u[N + i] = a1;
+    lam_u[2 * N + i] = a2;
+    if (d.sfac) gradf[i] += gf;
+}
+
 // FP32 versions of the two VJP halves (same traversal, FP32 point terms and
 // FP32 sums per lane, closed in FP64 across the lanes)
 template <int L>
@@ -357,37 +580,58 @@ __global__ void __launch_bounds__(256) k_vjp_partner_f32(Dev d, const double* __
 // transpose of the MLS gather: lam_us[k] += sum over the Gauss points (j,g)
 // of nodes without a boundary condition that k contributes to, of
 // coeff * lam_ug[j,g].  tptr/tj/tpos: for each k, the (node j, position of k
-// in j's contributor list) pairs.
-__global__ void k_gather_T(Dev d, const int64_t* __restrict__ tptr, const int32_t* __restrict__ tj,
+// in j's contributor list) pairs.  A warp per node: the lanes take the pairs
+// side by side (one thread per node walked its hundred-odd pairs as a chain of
+// dependent loads: 320 us for 8,192 nodes,
+// 326 us for 32,768; now 43 and 138 us, bound by the
+// L1 wavefronts of the coefficient rows).
+__global__ void __launch_bounds__(256) k_gather_T(Dev d, const int64_t* __restrict__ tptr, const int32_t* __restrict__ tj,
                            const int32_t* __restrict__ tpos, const double* __restrict__ lam_ug,
                            double* __restrict__ lam_us) {
     const int64_t N = d.n;
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (k >= N) return;
     const int npt = d.npt;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
     if (!d.mls) {  // every Gauss point of a node without a BC takes the node's displacement
         if (d.bc[k] >= 0) return;
-        for (int g = 0; g < npt; ++g) {
+        for (int g = lane; g < npt; g += 32) {
             a0 += lam_ug[(int64_t)(3 * g) * N + k];
             a1 += lam_ug[(int64_t)(3 * g + 1) * N + k];
             a2 += lam_ug[(int64_t)(3 * g + 2) * N + k];
         }
-        lam_us[k] += a0;
-        lam_us[N + k] += a1;
-        lam_us[2 * N + k] += a2;
-        return;
-    }
-    for (int64_t e = tptr[k]; e < tptr[k + 1]; ++e) {
-        const int64_t j = tj[e];
-        const double* cf = d.coeff + (d.cbptr[j] + tpos[e]) * npt;
-        for (int g = 0; g < npt; ++g) {
-            const double c = cf[g];
-            a0 += c * lam_ug[(int64_t)(3 * g) * N + j];
-            a1 += c * lam_ug[(int64_t)(3 * g + 1) * N + j];
-            a2 += c * lam_ug[(int64_t)(3 * g + 2) * N + j];
+    } else {
+        for (int64_t e = tptr[k] + lane; e < tptr[k + 1]; e += 32) {
+            const int64_t j = tj[e];
+            const double* cf = d.coeff + (d.cbptr[j] + tpos[e]) * npt;
+            if (npt == 8) {  // a pair's 64 bytes in four loads
+                const double2* c2 = reinterpret_cast<const double2*>(cf);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const double2 c = __ldg(c2 + h);
+                    const double* l = lam_ug + (int64_t)(6 * h) * N + j;
+                    a0 += c.x * l[0];
+                    a1 += c.x * l[N];
+                    a2 += c.x * l[2 * N];
+                    a0 += c.y * l[3 * N];
+                    a1 += c.y * l[4 * N];
+                    a2 += c.y * l[5 * N];
+                }
+                continue;
+            }
+            for (int g = 0; g < npt; ++g) {
+                const double c = cf[g];
+                a0 += c * lam_ug[(int64_t)(3 * g) * N + j];
+                a1 += c * lam_ug[(int64_t)(3 * g + 1) * N + j];
+                a2 += c * lam_ug[(int64_t)(3 * g + 2) * N + j];
+            }
         }
     }
+    a0 = lane_sum<32>(a0);
+    a1 = lane_sum<32>(a1);
+    a2 = lane_sum<32>(a2);
+    if (lane) return;
     lam_us[k] += a0;
     lam_us[N + k] += a1;
     lam_us[2 * N + k] += a2;
@@ -513,9 +757,26 @@ void launch_vjp_partner(const Dev& d, const double* teU, const double* teus, con
         else k_vjp_partner<1><<<b1, 256, sh, s>>>(d, teU, teus, teug, lamF, lam_ug, gradf);
     }
 }
+void launch_mirror(const Dev& d, int64_t* mirror, int* err, cudaStream_t s) {
+    if (d.n) k_mirror<<<blocks_for(32 * d.n, 256), 256, 0, s>>>(d, mirror, err);
+}
+void launch_vjp_both(const Dev& d, const double* teU, const double* teus, const double* teug, const double* lamF,
+                     double* lam_u, double* lam_ug, double* gradf, const int64_t* mirror, double4* bond, double* rec,
+                     cudaStream_t s) {
+    if (d.n == 0) return;
+    k_vjp_pack<<<blocks_for(d.n, 256), 256, 0, s>>>(d, teU, teus, lamF, rec);
+    // a warp per node while nodes are few, eight lanes above (fewer idle lanes)
+    if (d.n < 12288) {
+        k_vjp_bonds<32><<<blocks_for(32 * d.n, 128), 128, 0, s>>>(d, rec, teug, lam_ug, gradf, mirror, bond);
+        k_vjp_nodes<32><<<blocks_for(32 * d.n, 128), 128, 0, s>>>(d, bond, lam_u, gradf);
+    } else {
+        k_vjp_bonds<8><<<blocks_for(8 * d.n, 128), 128, 0, s>>>(d, rec, teug, lam_ug, gradf, mirror, bond);
+        k_vjp_nodes<8><<<blocks_for(8 * d.n, 128), 128, 0, s>>>(d, bond, lam_u, gradf);
+    }
+}
 void launch_gather_T(const Dev& d, const int64_t* tptr, const int32_t* tj, const int32_t* tpos, const double* lam_ug,
                      double* lam_us, cudaStream_t s) {
-    k_gather_T<<<blocks_for(d.n, 128), 128, 0, s>>>(d, tptr, tj, tpos, lam_ug, lam_us);
+    k_gather_T<<<blocks_for(32 * d.n, 256), 256, 0, s>>>(d, tptr, tj, tpos, lam_ug, lam_us);
 }
 void launch_adj_combine(const Dev& d, double dt, const double* lUp, const double* lVp, const AdjBuf& A,
                         cudaStream_t s) {

@@ -133,6 +133,10 @@ struct pd_ctx {
     int64_t* sell_off = nullptr;  // SELL copy of the FP32 gather's lists
     int32_t* sell_idx = nullptr;
     float* sell_coef = nullptr;
+    int64_t* adj_mirror = nullptr;  // mirror entries of the unbroken family and a bond's share (k_vjp_bonds)
+    double4* adj_bond = nullptr;
+    uint64_t adj_mirror_gen = ~0ull;
+    bool adj_symmetric = false;
     double* adj_pool = nullptr;  // reverse-sweep work buffers and stage tape
     int64_t adj_pool_count = 0;
     bool have_family = false, have_mls = false;
@@ -155,6 +159,7 @@ struct pd_ctx {
     double graph_dt = 0.0;
     int graph_prec = -1, graph_energy = -1;
     uint64_t generation = 0, graph_generation = ~0ull;
+    uint64_t family_gen = 0;  // families installed
 };
 
 namespace {
@@ -483,6 +488,7 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
                     const double effw = std::pow(w1 * w2 * w3, 1.0 / 3.0);
                     G.W = vol8 * w1 * w2 * w3;
                     G.dxe = effw * d.dx / 2.0;
+                    G.ydxe = 1.0 / G.dxe;
                     G.pw3 = std::pow(0.5 * effw, 3);
                     for (int q = 0; q < 3; ++q) G.hgf[q] = (float)G.hg[q];
                     G.Wf = (float)G.W;
@@ -1015,6 +1021,7 @@ static void install_family(pd_ctx* c, int64_t* frow, int32_t* fcol, uint8_t* fbr
     c->Ha = Ha;
     c->have_family = true;
     c->have_ai = false;                            // its regions follow the family
+    c->family_gen++;
     c->d.tile_x = c->d.tile_y = c->d.tile_z = 0;  // its family radius may have changed
     if (c->fst_mask) fsten_release(c);
     c->generation++;
@@ -2631,18 +2638,42 @@ extern "C" int pd_adjoint_forward(pd_ctx* c, double dt, double t0, int nsteps, i
 // the final U and V ([3N] host, V may be NULL); grad_f [N] receives the
 // gradient with respect to the per-node spring factors.  Leaves the state
 // at the start of the forward run.
+// The mirror entries for the one-evaluation VJP, once per family.
+namespace {
+int mirror_prepare(pd_ctx* c) {
+    if (c->adj_mirror_gen == c->family_gen) return PD_OK;
+    dfree(c, c->adj_mirror);
+    dfree(c, c->adj_bond);
+    c->adj_mirror = nullptr;
+    c->adj_bond = nullptr;
+    c->adj_symmetric = false;
+    c->adj_mirror_gen = c->family_gen;
+    if (c->npt != 8 || c->Ha == 0) return PD_OK;
+    PD_TRY(dalloc(c, &c->adj_mirror, c->Ha));
+    if (dalloc(c, &c->adj_bond, c->Ha) != PD_OK) return PD_OK;  // no room: two evaluations
+    PD_CUDA_TRY(cudaMemsetAsync(c->dflag, 0, sizeof(int), c->stream));
+    pd::launch_mirror(c->d, c->adj_mirror, c->dflag, c->stream);
+    int bad = 1;
+    PD_CUDA_TRY(cudaMemcpyAsync(&bad, c->dflag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    c->adj_symmetric = !bad;
+    return PD_OK;
+}
+}  // namespace
+
 extern "C" int pd_adjoint_backward(pd_ctx* c, const double* lam_U, const double* lam_V, double* grad_f) {
     if (!c || !lam_U || !grad_f) return fail(PD_ERR_ARG, "pd_adjoint_backward: null argument");
     if (c->adj_steps < 1) return fail(PD_ERR_ARG, "pd_adjoint_backward: no forward run to reverse");
     if (!c->d.sfac) return fail(PD_ERR_ARG, "pd_adjoint_backward: set the spring factors first");
     if (c->d.mls) PD_TRY(build_transpose(c));
+    PD_TRY(mirror_prepare(c));
     const int64_t N = c->n, n3 = 3 * N, ng = n3 * c->npt;
     cudaStream_t s = c->stream;
     const pd::Dev& d = c->d;
     const double dt = c->adj_dt;
     // work buffers: carved from one pool that the context keeps between calls
     // (an optimiser calls the pair again and again with the same sizes)
-    const int64_t pool_need = 13 * n3 + 3 * ng + N + (int64_t)c->adj_every * 4 * (2 * n3 + ng) + 32 * 19;
+    const int64_t pool_need = 13 * n3 + 3 * ng + 13 * N + (int64_t)c->adj_every * 4 * (2 * n3 + ng) + 32 * 20;
     if (c->adj_pool_count < pool_need) {
         dfree(c, c->adj_pool);
         c->adj_pool = nullptr;
@@ -2667,11 +2698,12 @@ extern "C" int pd_adjoint_backward(pd_ctx* c, const double* lam_U, const double*
     double* lug = get(ng);
     double* lugSn = get(ng);
     double* gradf = get(N);
+    double* rec = get(12 * N);  // the VJP's node records
     const int every = c->adj_every;
     const int64_t per = 2 * n3 + ng;
     double* tape = get((int64_t)every * 4 * per);
     auto release = [&]() {};
-    if (!ok || !lUp || !lVp || !lugSp || !lug || !lugSn || !gradf || !tape) {
+    if (!ok || !lUp || !lVp || !lugSp || !lug || !lugSn || !gradf || !rec || !tape) {
         release();
         return fail(PD_ERR_OOM, "pd_adjoint_backward: device memory for the tape");
     }
@@ -2702,6 +2734,15 @@ extern "C" int pd_adjoint_backward(pd_ctx* c, const double* lam_U, const double*
             auto teU = [&](int st) { return tp + (int64_t)(st - 1) * per; };
             auto teus = [&](int st) { return tp + (int64_t)(st - 1) * per + n3; };
             auto teug = [&](int st) { return tp + (int64_t)(st - 1) * per + 2 * n3; };
+            auto vjp = [&](int st, double* to) {  // dJ/du and dJ/dug of stage st's force
+                if (c->adj_symmetric && !vjp32) {
+                    pd::launch_vjp_both(d, teU(st), teus(st), teug(st), A.lF, A.lueff, to, gradf, c->adj_mirror,
+                                        c->adj_bond, rec, s);
+                    return;
+                }
+                pd::launch_vjp_own(d, teU(st), teus(st), teug(st), A.lF, A.lueff, gradf, s, vjp32);
+                pd::launch_vjp_partner(d, teU(st), teus(st), teug(st), A.lF, to, gradf, s, vjp32);
+            };
             pd::launch_gather_T(d, c->tptr, c->tj, c->tpos, lugSp, lUp, s);
             pd::launch_adj_combine(d, dt, lUp, lVp, A, s);
             double* lk_of[5] = {nullptr, A.lk1, A.lk2, A.lk3, A.lk4};
@@ -2709,15 +2750,13 @@ extern "C" int pd_adjoint_backward(pd_ctx* c, const double* lam_U, const double*
             for (int st = 4; st >= 2; --st) {
                 const double dts = st >= 3 ? dt : 0.5 * dt;
                 pd::launch_adj_stage_pre(d, dts, lk_of[st], A, s);
-                pd::launch_vjp_own(d, teU(st), teus(st), teug(st), A.lF, A.lueff, gradf, s, vjp32);
-                pd::launch_vjp_partner(d, teU(st), teus(st), teug(st), A.lF, lug, gradf, s, vjp32);
+                vjp(st, lug);
                 pd::launch_adj_stage_node(d, A, s);
                 pd::launch_gather_T(d, c->tptr, c->tj, c->tpos, lug, A.lus, s);
                 pd::launch_adj_stage_post(d, alpha[st], lk_of[st - 1], A, s);
             }
             pd::launch_adj_stage_pre(d, 0.5 * dt, A.lk1, A, s);
-            pd::launch_vjp_own(d, teU(1), teus(1), teug(1), A.lF, A.lueff, gradf, s, vjp32);
-            pd::launch_vjp_partner(d, teU(1), teus(1), teug(1), A.lF, lugSn, gradf, s, vjp32);
+            vjp(1, lugSn);
             pd::launch_adj_stage1_end(d, A, s);
             cudaMemcpyAsync(lUp, A.lU, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
             cudaMemcpyAsync(lVp, A.lV, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);

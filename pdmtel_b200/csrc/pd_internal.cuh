@@ -33,7 +33,7 @@ struct BcDev {
 struct GaussConst {
     double hg[3];
     double W;
-    double dxe;
+    double dxe, ydxe;  // ydxe = 1 / dxe
     double pw3;
     float hgf[3];
     float Wf;
@@ -391,6 +391,12 @@ void launch_vjp_own(const Dev& d, const double* teU, const double* teus, const d
                     double* lam_u, double* gradf, cudaStream_t s, bool f32);
 void launch_vjp_partner(const Dev& d, const double* teU, const double* teus, const double* teug, const double* lamF,
                         double* lam_ug, double* gradf, cudaStream_t s, bool f32);
+// both halves in one evaluation (2x2x2 points, FP64): bond [Ha] and rec [12 N]
+// are scratch, mirror [Ha] from launch_mirror (err: set when the family is not symmetric)
+void launch_mirror(const Dev& d, int64_t* mirror, int* err, cudaStream_t s);
+void launch_vjp_both(const Dev& d, const double* teU, const double* teus, const double* teug, const double* lamF,
+                     double* lam_u, double* lam_ug, double* gradf, const int64_t* mirror, double4* bond, double* rec,
+                     cudaStream_t s);
 // FP64 Gauss-point displacements [3 npt][N] from the FP32 form's node blocks
 // (the node's trial displacement hi + lo plus each point's FP32 offset)
 void launch_blocks_to_ug(const Dev& d, double* ug, cudaStream_t s);
