@@ -18,8 +18,8 @@
 //               the count of its points past the critical stretch; with the
 //               energy on, every point's energy term in the bond's slots of a
 //               per-point buffer (0.0 for a failed point);
-//  k_ai_sum     one thread per node (one warp with the energy on,
-//               k_ai_sum_energy): the velocity update bond by bond in family
+//  k_ai_sum     one warp per node (k_ai_sum_energy with the energy on): the
+//               velocity update bond by bond in family
 //               order, and the energy terms added point by point in the
 //               reference's order (a sequential sum, formed exactly).
 //               A failing point breaks the bond object the two
@@ -29,9 +29,11 @@
 //               in this stage.  Breaks are committed here for the next stage.
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 #include "pd_ai_eval.h"
 #include "pd_internal.cuh"
+#include "pd_rn.cuh"
 #include "pd_stage.cuh"
 
 namespace pd {
@@ -60,6 +62,19 @@ __global__ void k_ai_gather(Dev d, const double* __restrict__ us) {
     d.ai_u[3 * e] = a0;
     d.ai_u[3 * e + 1] = a1;
     d.ai_u[3 * e + 2] = a2;
+}
+
+// A point with operands outside the range of pd_rn.cuh, out of line: (force
+// density, energy term).
+__device__ __noinline__ double4 point_general(double r2, double p2, double y0, double y1, double y2, double ecrit,
+                                              double be, double c, int* failed) {
+    const double r = sqrt(r2), pl = sqrt(p2);
+    const double u = pl - r;
+    const double s = u / r;
+    *failed = !(u <= 0.0 || (u > 0.0 && s <= ecrit));
+    if (*failed) return make_double4(0.0, 0.0, 0.0, 0.0);
+    const double t = be * 1.0 * c * s;
+    return make_double4(t * y0 / pl, t * y1 / pl, t * y2 / pl, be * 0.5 * (0.5 * 1.0 * (c / r) * u * u));
 }
 
 // The integrand at one trapezoid point of bond i -> j: the force density into
@@ -109,22 +124,34 @@ struct ForceFn {
                          B->val[3 * a + 2] * (p[2] - 0.0);
         }
         const double x0 = p[0] - 0.0, x1 = p[1] - 0.0, x2 = p[2] - 0.0;
-        const double r = sqrt(x0 * x0 + x1 * x1 + x2 * x2);
         const double y0 = x0 + eta[0], y1 = x1 + eta[1], y2 = x2 + eta[2];
-        const double pl = sqrt(y0 * y0 + y1 * y1 + y2 * y2);
+        const double r2 = x0 * x0 + x1 * x1 + x2 * x2, p2 = y0 * y0 + y1 * y1 + y2 * y2;
+        // straight-line square roots and quotients (pd_rn.cuh); operands
+        // outside their range take the compiler's
+        double r, yr, pl, yp;
+        rn_sqrt_rcp(r2, r, yr);
+        rn_sqrt_rcp(p2, pl, yp);
         const double u = pl - r;
-        const double s = u / r;
-        if (u <= 0.0 || (u > 0.0 && s <= ecrit)) {
-            const double t = be * 1.0 * c * s;
-            f[0] = t * y0 / pl;
-            f[1] = t * y1 / pl;
-            f[2] = t * y2 / pl;
-            *e = be * 0.5 * (0.5 * 1.0 * (c / r) * u * u);
-            return 0;
+        const double s = rn_div(u, r, yr);
+        const double t = be * 1.0 * c * s;
+        const double n0 = t * y0, n1 = t * y1, n2 = t * y2;
+        const unsigned far = max(max(rn_dividend(n0), rn_dividend(n1)), max(rn_dividend(n2), rn_dividend(c)));
+        const bool on = u <= 0.0 || (u > 0.0 && s <= ecrit);
+        f[0] = on ? rn_div_signed(n0, pl, yp) : 0.0;
+        f[1] = on ? rn_div_signed(n1, pl, yp) : 0.0;
+        f[2] = on ? rn_div_signed(n2, pl, yp) : 0.0;
+        *e = on ? be * 0.5 * (0.5 * 1.0 * rn_div_signed(c, r, yr) * u * u) : 0.0;
+        int failed = on ? 0 : 1;
+        if (!(rn_range(r2) && rn_range(p2) && far < rn_span)) {
+            int past = 0;
+            const double4 g = point_general(r2, p2, y0, y1, y2, ecrit, be, c, &past);
+            failed = past;
+            f[0] = g.x;
+            f[1] = g.y;
+            f[2] = g.z;
+            *e = g.w;
         }
-        f[0] = f[1] = f[2] = 0.0;
-        *e = 0.0;
-        return 1;
+        return failed;
     }
 };
 
@@ -145,13 +172,22 @@ constexpr int kAiWarps = 4;  // warps per block of k_ai_bond
 // integrand written to shared memory; the row, middle and outer trapezoid
 // sums follow in the order of pdIntgManager::CalcTrapzdQuad (lane = row,
 // lane = outer point, lane 0), so the integral is the serial one bit for bit.
-template <bool ENERGY>
-__global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
+// NI: the trapezoid index, so that every loop and division by the points per
+// direction is compiled in.
+//
+// 20x10x10 bar, index 3 with energies (59.2M points per launch): 2.97 -> 1.35 ms
+// with the square roots and quotients of pd_rn.cuh, NI compiled in, axis and
+// point chosen by selects instead of indexed arrays and a switch, and four
+// blocks per SM (128 registers).  About 400 instructions per 32 points, half of
+// them the rows' limits and the nested sums; FP64 pipe about 30 % busy.
+template <bool ENERGY, int NI>
+__global__ void __launch_bounds__(128, 4) k_ai_bond(Dev d) {
     using namespace pd_ai;
     constexpr unsigned full = 0xffffffffu;
-    __shared__ double sf[kAiWarps][kMaxRegionPoints][3];
-    __shared__ double sh[kAiWarps][kMaxPerDir * kMaxPerDir][3];
-    __shared__ double sg[kAiWarps][kMaxPerDir][3];
+    constexpr int kDir = NI == 1 ? 2 : (NI == 2 ? 3 : 5);
+    __shared__ double sf[kAiWarps][kDir * kDir * kDir][3];
+    __shared__ double sh[kAiWarps][kDir * kDir][3];
+    __shared__ double sg[kAiWarps][kDir][3];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (w >= d.ai_nent) return;
@@ -184,7 +220,7 @@ __global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
     fn.K = d.ai_mls ? d.ai_tptr[j + 1] - d.ai_tptr[j] : 0;
     const double xj[3] = {d.x[j] - d.x[i], d.x[N + j] - d.x[N + i], d.x[2 * N + j] - d.x[2 * N + i]};
     const double delta = d.delta, dx = d.dx;
-    const int n = d.ai_n, np = points_per_dir(n), nrow = np * np;
+    constexpr int n = NI, np = NI == 1 ? 2 : (NI == 2 ? 3 : 5), nrow = np * np;
     double F[3] = {0.0, 0.0, 0.0};
     int fail = 0;
     int64_t q0 = ENERGY ? d.ai_eptr[p] : 0;
@@ -219,7 +255,8 @@ __global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
             const int base = incl - cnt;
             const int total = __shfl_sync(full, incl, 31);
             // points
-            const int nslot = nrow * np;
+            constexpr int nslot = nrow * np;
+#pragma unroll 1
             for (int s0 = 0; s0 < nslot; s0 += 32) {
                 const int slot = s0 + lane;
                 const int row = slot < nslot ? slot / np : 0;
@@ -229,9 +266,9 @@ __global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
                 if (slot < nslot && rok) {
                     const int m = slot - row * np;
                     double pp[3], f[3], e;
-                    pp[R.axis[0]] = rt;
-                    pp[R.axis[1]] = rs;
-                    pp[R.axis[2]] = point(n, m, rzl, rzh);
+                    const double rz = point(n, m, rzl, rzh);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) pp[a] = R.axis[0] == a ? rt : (R.axis[1] == a ? rs : rz);
                     fail += fn.eval(pp, rbase + m, f, &e);
                     sf[wib][slot][0] = f[0];
                     sf[wib][slot][1] = f[1];
@@ -245,6 +282,7 @@ __global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
                 double h[3] = {0.0, 0.0, 0.0};
                 if (row_ok) {
                     double acc[3];
+#pragma unroll
                     for (int m = 0; m < np; ++m) accumulate(m, np, sf[wib][lane * np + m], acc);
                     const double wgt = scale(n, zl, zh);
                     h[0] = wgt * acc[0];
@@ -264,6 +302,7 @@ __global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
                 double g[3] = {0.0, 0.0, 0.0};
                 if (kok) {
                     double acc[3];
+#pragma unroll
                     for (int l = 0; l < np; ++l) accumulate(l, np, sh[wib][lane * np + l], acc);
                     const double wgt = scale(n, kml, kmh);
                     g[0] = wgt * acc[0];
@@ -277,6 +316,7 @@ __global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
             __syncwarp();
             if (lane == 0) {
                 double acc[3];
+#pragma unroll
                 for (int k = 0; k < np; ++k) accumulate(k, np, sg[wib][k], acc);
                 const double wgt = scale(n, R.a, R.b);
                 out[0] = wgt * acc[0];
@@ -306,53 +346,67 @@ __global__ void __launch_bounds__(128) k_ai_bond(Dev d) {
     }
 }
 
-__global__ void k_ai_sum(Dev d, double dts) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
+// The velocity update, the damage count and the break bookkeeping of one node
+// by its warp: the lanes take the bonds side by side, lanes 0..2 add their
+// increments in family order (a skipped bond's is -0.0, which changes no sum).
+__device__ __forceinline__ void ai_node_sum(const Dev& d, int64_t i, int lane, double dts, double (*inc)[3]) {
     const int64_t N = d.n;
     const MatDev Mi = d.mats[d.mat[i]];
     const double rho = Mi.density;
-    const double b0 = Mi.grav[0] * rho, b1 = Mi.grav[1] * rho, b2 = Mi.grav[2] * rho;
-    double v0 = d.vbuf[i], v1 = d.vbuf[N + i], v2 = d.vbuf[2 * N + i];
-    int dmg = d.ai_dmg[i];
+    const double b[3] = {Mi.grav[0] * rho, Mi.grav[1] * rho, Mi.grav[2] * rho};
+    double v = lane < 3 ? d.vbuf[(int64_t)lane * N + i] : 0.0;
+    int dmg = 0;
     const int64_t pe = d.frow[i + 1];
-    for (int64_t p = d.frow[i]; p < pe; ++p) {
-        if (d.ai_brk[p]) continue;
-        const int64_t j = d.fcol[p];
-        const int64_t q = d.ai_mirror[p];
-        if (j < i && d.ai_fail[q] > 0) {
-            d.ai_brk[p] = 1;  // broken by node j's visit of this bond in this stage
-            continue;
+    for (int64_t base = d.frow[i]; base < pe; base += 32) {
+        const int64_t p = base + lane;
+        double w[3] = {-0.0, -0.0, -0.0};
+        if (p < pe && !d.ai_brk[p]) {
+            const int64_t j = d.fcol[p];
+            const int own = d.ai_fail[p], other = d.ai_fail[d.ai_mirror[p]];
+            if (j < i && other > 0) {
+                d.ai_brk[p] = 1;  // broken by node j's visit of this bond in this stage
+            } else {
+                for (int a = 0; a < 3; ++a) w[a] = (d.ai_F[3 * p + a] + b[a]) * dts / rho;
+                dmg += own;
+                if (own > 0 || (j > i && other > 0)) d.ai_brk[p] = 1;
+            }
         }
-        const double F[3] = {d.ai_F[3 * p], d.ai_F[3 * p + 1], d.ai_F[3 * p + 2]};
-        dmg += d.ai_fail[p];
-        v0 += (F[0] + b0) * dts / rho;
-        v1 += (F[1] + b1) * dts / rho;
-        v2 += (F[2] + b2) * dts / rho;
-        if (d.ai_fail[p] > 0 || (j > i && d.ai_fail[q] > 0)) d.ai_brk[p] = 1;
+        for (int a = 0; a < 3; ++a) inc[lane][a] = w[a];
+        __syncwarp();
+        if (lane < 3) {
+#pragma unroll 8
+            for (int q = 0; q < 32; ++q) v += inc[q][lane];
+        }
+        __syncwarp();
     }
-    d.vbuf[i] = v0;
-    d.vbuf[N + i] = v1;
-    d.vbuf[2 * N + i] = v2;
-    d.ai_dmg[i] = dmg;
+    for (int o = 16; o > 0; o >>= 1) dmg += __shfl_xor_sync(0xffffffffu, dmg, o);
+    if (lane < 3) d.vbuf[(int64_t)lane * N + i] = v;
+    if (lane == 0) d.ai_dmg[i] += dmg;
 }
 
-// With the energy on: one warp per node.  The node's energy terms are
-// contiguous (its entries' slots in family order; k_ai_bond zeroes the slots
-// of bonds broken before the stage, and adding +0.0 to a non-negative sum
-// changes nothing), so the warp streams them 128 at a time through shared
-// memory, the next round's loads in flight while lane 0 adds the current
-// round in point order: the reference's sequential sum, formed exactly.  A
-// node with a bond its lower node broke in this stage (rare) takes the terms
-// bond by bond instead.  Lane 0 then does the velocity update and the break
-// bookkeeping of k_ai_sum.
+__global__ void __launch_bounds__(128) k_ai_sum(Dev d, double dts) {
+    __shared__ double inc[4][32][3];
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (i >= d.n) return;
+    ai_node_sum(d, i, threadIdx.x & 31, dts, inc[threadIdx.x >> 5]);
+}
+
+// With the energy on: the node's energy terms are contiguous (its entries'
+// slots in family order; k_ai_bond zeroes the slots of bonds broken before the
+// stage, and adding +0.0 to a non-negative sum changes nothing), so the warp
+// streams them 128 at a time through shared memory, the next round's loads in
+// flight while lane 0 adds the current round in point order, its next eight
+// terms in registers before it adds the present ones: the reference's
+// sequential sum, formed exactly, and bound by the latency of its additions.
+// A node with a bond its lower node broke in this stage (rare) takes the terms
+// bond by bond instead.
 __global__ void __launch_bounds__(128) k_ai_sum_energy(Dev d, double dts) {
     constexpr int kRound = 128;
     __shared__ double buf[4][2][kRound];
+    __shared__ double inc[4][32][3];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (i >= d.n) return;
-    const int64_t N = d.n;
     const int64_t pb = d.frow[i], pe = d.frow[i + 1];
     // a bond skipped because node j's visit of it failed in this stage?
     int skip = 0;
@@ -367,7 +421,7 @@ __global__ void __launch_bounds__(128) k_ai_sum_energy(Dev d, double dts) {
 #pragma unroll
         for (int u = 0; u < kRound / 32; ++u) {
             const int64_t e = E0 + 32 * u + lane;
-            nxt[u] = e < E1 ? d.ai_e[e] : 0.0;
+            nxt[u] = e < E1 ? d.ai_e[e] : -0.0;  // past the end: changes no sum
         }
         int cur = 0;
         for (int64_t base = E0; base < E1; base += kRound) {
@@ -377,21 +431,24 @@ __global__ void __launch_bounds__(128) k_ai_sum_energy(Dev d, double dts) {
 #pragma unroll
             for (int u = 0; u < kRound / 32; ++u) {
                 const int64_t e = base + kRound + 32 * u + lane;
-                nxt[u] = e < E1 ? d.ai_e[e] : 0.0;
+                nxt[u] = e < E1 ? d.ai_e[e] : -0.0;
             }
             if (lane == 0) {
-                const int m = (E1 - base) < kRound ? (int)(E1 - base) : kRound;
                 const double* b = buf[wib][cur];
-                int k = 0;
-                // eight shared-memory loads in flight ahead of the in-order adds
-                for (; k + 8 <= m; k += 8) {
-                    double v[8];
+                double v[8], w[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) v[u] = b[k + u];
+                for (int u = 0; u < 8; ++u) v[u] = b[u];
+#pragma unroll 1
+                for (int k = 0; k < kRound; k += 16) {
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) w[u] = b[k + 8 + u];
 #pragma unroll
                     for (int u = 0; u < 8; ++u) eacc += v[u];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[u] = b[(k + 16 + u) & (kRound - 1)];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) eacc += w[u];
                 }
-                for (; k < m; ++k) eacc += b[k];
             }
             cur ^= 1;
         }
@@ -407,31 +464,8 @@ __global__ void __launch_bounds__(128) k_ai_sum_energy(Dev d, double dts) {
             stream(d.ai_eptr[p], d.ai_eptr[p + 1]);
         }
     }
-    if (lane != 0) return;
-    const MatDev Mi = d.mats[d.mat[i]];
-    const double rho = Mi.density;
-    const double b0 = Mi.grav[0] * rho, b1 = Mi.grav[1] * rho, b2 = Mi.grav[2] * rho;
-    double v0 = d.vbuf[i], v1 = d.vbuf[N + i], v2 = d.vbuf[2 * N + i];
-    int dmg = d.ai_dmg[i];
-    for (int64_t p = pb; p < pe; ++p) {
-        if (d.ai_brk[p]) continue;
-        const int64_t j = d.fcol[p];
-        const int64_t q = d.ai_mirror[p];
-        if (j < i && d.ai_fail[q] > 0) {
-            d.ai_brk[p] = 1;  // broken by node j's visit of this bond in this stage
-            continue;
-        }
-        dmg += d.ai_fail[p];
-        v0 += (d.ai_F[3 * p] + b0) * dts / rho;
-        v1 += (d.ai_F[3 * p + 1] + b1) * dts / rho;
-        v2 += (d.ai_F[3 * p + 2] + b2) * dts / rho;
-        if (d.ai_fail[p] > 0 || (j > i && d.ai_fail[q] > 0)) d.ai_brk[p] = 1;
-    }
-    d.vbuf[i] = v0;
-    d.vbuf[N + i] = v1;
-    d.vbuf[2 * N + i] = v2;
-    d.ai_dmg[i] = dmg;
-    d.eed[i] = eacc;
+    if (lane == 0) d.eed[i] = eacc;
+    ai_node_sum(d, i, lane, dts, inc[wib]);
 }
 
 inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
@@ -447,11 +481,17 @@ void launch_ai_force(const Dev& d, double dts, cudaStream_t s) {
     if (d.n == 0) return;
     if (d.ai_nent > 0) {
         const unsigned nb = blocks_for(d.ai_nent, kAiWarps);
-        if (d.energy) k_ai_bond<true><<<nb, 32 * kAiWarps, 0, s>>>(d);
-        else k_ai_bond<false><<<nb, 32 * kAiWarps, 0, s>>>(d);
+        auto bond = [&](auto index) {
+            constexpr int n = decltype(index)::value;
+            if (d.energy) k_ai_bond<true, n><<<nb, 32 * kAiWarps, 0, s>>>(d);
+            else k_ai_bond<false, n><<<nb, 32 * kAiWarps, 0, s>>>(d);
+        };
+        if (d.ai_n == 1) bond(std::integral_constant<int, 1>{});
+        else if (d.ai_n == 2) bond(std::integral_constant<int, 2>{});
+        else bond(std::integral_constant<int, 3>{});
     }
     if (d.energy) k_ai_sum_energy<<<blocks_for(32 * d.n, 128), 128, 0, s>>>(d, dts);
-    else k_ai_sum<<<blocks_for(d.n, 128), 128, 0, s>>>(d, dts);
+    else k_ai_sum<<<blocks_for(32 * d.n, 128), 128, 0, s>>>(d, dts);
 }
 
 }  // namespace pd

@@ -23,6 +23,7 @@
 #include "../../include/pdmtel_b200.h"
 
 #ifdef __CUDACC__
+#include "pd_rn.cuh"
 #define PD_AI_HD __host__ __device__ __forceinline__
 #else
 #define PD_AI_HD inline
@@ -52,15 +53,13 @@ PD_AI_HD int points_per_dir(int n) { return n == 1 ? 2 : (n == 2 ? 3 : 5); }
 
 // the k-th trapezoid point of [a, b] (CalcTrapzdQuad cases 1-3)
 PD_AI_HD double point(int n, int k, double a, double b) {
-    if (k == 0) return a;
-    if (n == 1) return b;
-    if (n == 2) return k == 1 ? 0.5 * (a + b) : b;
-    switch (k) {
-        case 1: return 0.25 * (3.0 * a + b);
-        case 2: return 0.5 * (a + b);
-        case 3: return 0.25 * (a + 3.0 * b);
-        default: return b;
-    }
+    if (n == 1) return k == 0 ? a : b;
+    if (n == 2) return k == 0 ? a : (k == 1 ? 0.5 * (a + b) : b);
+    // 0.25 (3 a + b), 0.5 (a + b), 0.25 (a + 3 b) for k = 1, 2, 3 by selects:
+    // the points of a row differ in k and share a warp
+    const double p = k <= 2 ? a : b, q = k <= 2 ? b : a;
+    const double inner = (k == 2 ? 0.5 : 0.25) * ((k == 2 ? 1.0 : 3.0) * p + q);
+    return k == 0 ? a : (k >= 4 ? b : inner);
 }
 
 // width factor of the rule: (b-a), 0.5 (b-a), 0.25 (b-a)
@@ -87,19 +86,32 @@ PD_AI_HD void accumulate(int k, int np, const double f[3], double acc[3]) {
     }
 }
 
+// IEEE square root (on the device without the branches of the compiler's own)
+PD_AI_HD double root(double v) {
+#ifdef __CUDA_ARCH__
+    double r, y;
+    pd::rn_sqrt_rcp(v, r, y);
+    if (pd::rn_range(v)) return r;
+#endif
+    return sqrt(v);
+}
+
+// v[k] by selects (an indexed local array would live in memory on the device)
+PD_AI_HD double pick(const double v[3], int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); }
+
 PD_AI_HD double mid_limit(int code, double t, const double xj[3], double delta, double dx) {
     if (code < 8) {
         const int ax = code >> 1;
-        return (code & 1) ? xj[ax] + 0.5 * dx : xj[ax] - 0.5 * dx;
+        return (code & 1) ? pick(xj, ax) + 0.5 * dx : pick(xj, ax) - 0.5 * dx;
     }
     const int c = code - 8;
     const int sign = c & 1, side = (c >> 1) & 1, ab = c >> 2;
     const int A = ab / 3, B = ab % 3, C = 3 - A - B;
-    const double h = side ? xj[C] + 0.5 * dx : xj[C] - 0.5 * dx;
+    const double h = side ? pick(xj, C) + 0.5 * dx : pick(xj, C) - 0.5 * dx;
     const double rsq = delta * delta - h * h;
     const double tt = t - 0.0;
     const double vsq = rsq - tt * tt;
-    double v = vsq < 0.0 ? -1.0 : sqrt(vsq);  // SolveBinaryQuadric, pdIntgManager2.cpp:812-834
+    double v = vsq < 0.0 ? -1.0 : root(vsq);  // SolveBinaryQuadric, pdIntgManager2.cpp:812-834
     if (v < 0.0) v = 0.0;
     return sign ? v : -v;
 }
@@ -107,10 +119,10 @@ PD_AI_HD double mid_limit(int code, double t, const double xj[3], double delta, 
 PD_AI_HD double in_limit(int code, double t, double s, const double xj[3], double delta, double dx) {
     if (code < 8) {
         const int ax = code >> 1;
-        return (code & 1) ? xj[ax] + 0.5 * dx : xj[ax] - 0.5 * dx;
+        return (code & 1) ? pick(xj, ax) + 0.5 * dx : pick(xj, ax) - 0.5 * dx;
     }
     const double zsq = delta * delta - t * t - s * s;
-    const double v = zsq < 0.0 ? 0.0 : sqrt(zsq);
+    const double v = zsq < 0.0 ? 0.0 : root(zsq);
     return (code & 1) ? v : -v;
 }
 

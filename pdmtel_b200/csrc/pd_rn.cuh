@@ -64,15 +64,16 @@ __device__ __forceinline__ double rsqrt_near(double a) {
     return rn_pow2(fma(h, fma(-g, h, 0.5), h), 1);
 }
 
-// a / b with y = 1/b; a zero or rn_quotient_ok (the quotient of a zero is +0)
+// a / b with y = 1/b, b > 0; a zero or rn_quotient_ok (the quotient of a zero
+// is +0)
 __device__ __forceinline__ double rn_div(double a, double b, double y) {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
-// the same with the sign of a zero kept
+// the same with the sign of a zero kept (any quotient has the sign of a)
 __device__ __forceinline__ double rn_div_signed(double a, double b, double y) {
     const double q = rn_div(a, b, y);
-    return a == 0.0 ? a : q;
+    return __hiloint2double((__double2hiint(q) & 0x7fffffff) | (__double2hiint(a) & 0x80000000), __double2loint(q));
 }
 
 // whether a positive operand of rn_sqrt_rcp is in [2^-400, 2^400)
