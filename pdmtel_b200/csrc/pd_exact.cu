@@ -14,6 +14,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "pd_gather.cuh"
 #include "pd_internal.cuh"
 #include "pd_rn.cuh"
 #include "pd_stage.cuh"
@@ -315,6 +316,23 @@ __global__ void __launch_bounds__(128, 3) k_force_f64(Dev d, double dts) {
 
 // ----------------------------------------------------------------- gather
 
+// The Gauss-point displacement of a node with a boundary condition
+// (UpdateIntgPointStatusWithBC, pdDataManager.cpp:2604-2703): its flagged
+// directions.
+__device__ __forceinline__ void gather_bc(const Dev& d, int64_t i, int g, double t, double* ug) {
+    const int64_t N = d.n;
+    const BcDev& B = d.bcs[d.bc[i]];
+    const double fac = time_factor(B, t);
+    const GaussConst& G = d.gc[g];
+    const double q0 = G.hg[0] + d.x[i], q1 = G.hg[1] + d.x[N + i], q2 = G.hg[2] + d.x[2 * N + i];
+    for (int a = 0; a < 3; ++a) {
+        if (B.dir[a] != 1) continue;
+        if (B.type == PD_BC_DISPL) ug[a * N] = B.val[a] * fac;
+        else if (B.type == PD_BC_DISPLGRAD)
+            ug[a * N] = (B.val[3 * a] * q0 + B.val[3 * a + 1] * q1 + B.val[3 * a + 2] * q2) * fac;
+    }
+}
+
 // One thread per (node, Gauss point): CalcIntgPointDisplRK4 (pdDataManager.cpp:
 // 2402-2495) with UpdateIntgPointStatusWithBC (:2604-2703).  Nodes with a
 // boundary condition keep the displacement of their unflagged directions
@@ -328,18 +346,8 @@ __global__ void k_gather_f64(Dev d, const double* __restrict__ us) {
     const int64_t i = d.order[tid / d.npt];
     const int g = (int)(tid % d.npt);
     double* ug = d.ug + (int64_t)(3 * g) * N + i;
-    const int b = d.bc[i];
-    if (b >= 0) {
-        const BcDev& B = d.bcs[b];
-        const double fac = time_factor(B, t);
-        const GaussConst& G = d.gc[g];
-        const double q0 = G.hg[0] + d.x[i], q1 = G.hg[1] + d.x[N + i], q2 = G.hg[2] + d.x[2 * N + i];
-        for (int a = 0; a < 3; ++a) {
-            if (B.dir[a] != 1) continue;
-            if (B.type == PD_BC_DISPL) ug[a * N] = B.val[a] * fac;
-            else if (B.type == PD_BC_DISPLGRAD)
-                ug[a * N] = (B.val[3 * a] * q0 + B.val[3 * a + 1] * q1 + B.val[3 * a + 2] * q2) * fac;
-        }
+    if (d.bc[i] >= 0) {
+        gather_bc(d, i, g, t, ug);
         return;
     }
     if (d.mls) {
@@ -386,6 +394,43 @@ __global__ void k_gather_f64(Dev d, const double* __restrict__ us) {
         ug[N] = us[N + i];
         ug[2 * N] = us[2 * N + i];
     }
+}
+
+// The same for the 2x2x2 rule (gather_chunks): 20x10x10 bar 21 -> 13 us, plate
+// 200x200x4 272 -> 171 us per launch (844 MB: 4.9 TB/s, 0.75 of the copy rate).
+constexpr int kGatherStages = 4;
+__global__ void __launch_bounds__(128) k_gather_f64_lanes(Dev d, const double* __restrict__ us) {
+    extern __shared__ __align__(16) char gather_sm[];
+    const int64_t N = d.n;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+    const int g = threadIdx.x & 7;
+    const bool live = slot < N;
+    const int64_t i = d.order[live ? slot : 0];
+    const bool free = live && d.bc[i] < 0;
+    const int64_t c0 = d.cbptr[i];
+    const int nc = free ? (int)(d.cbptr[i + 1] - c0) : 0;
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    gather_chunks<double, kGatherStages>(
+        gather_sm + (threadIdx.x >> 5) * gather_warp_bytes<double>(kGatherStages), d.coeff + c0 * 8, d.cbidx + c0, nc,
+        [&](int m, double* v) {
+            v[0] = us[m];
+            v[1] = us[N + m];
+            v[2] = us[2 * N + m];
+        },
+        [&](double c, const double* v) {
+            a0 += v[0] * c;
+            a1 += v[1] * c;
+            a2 += v[2] * c;
+        });
+    if (!live) return;
+    double* ug = d.ug + (int64_t)(3 * g) * N + i;
+    if (!free) {
+        gather_bc(d, i, g, *d.tdev, ug);
+        return;
+    }
+    ug[0] = a0;
+    ug[N] = a1;
+    ug[2 * N] = a2;
 }
 
 // --------------------------------------------------------------- epilogue
@@ -528,6 +573,10 @@ void launch_gather_f64(const Dev& d, const double* us, cudaStream_t s) {
         return;
     }
     if (d.cci || d.n == 0) return;
+    if (d.npt == 8 && d.mls) {
+        k_gather_f64_lanes<<<blocks_for(8 * d.n, 128), 128, 4 * gather_warp_bytes<double>(kGatherStages), s>>>(d, us);
+        return;
+    }
     const int bs = 256;
     k_gather_f64<<<blocks_for(d.n * d.npt, bs), bs, 0, s>>>(d, us);
 }

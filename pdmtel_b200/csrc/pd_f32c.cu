@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <climits>
 
+#include "pd_gather.cuh"
 #include "pd_internal.cuh"
 #include "pd_stage.cuh"
 
@@ -1218,11 +1219,6 @@ __device__ __forceinline__ BlkOut blk_out(const Dev& d, int64_t i) {
 // ill-conditioned moment matrices allow, hence the second term).  Nodes with a
 // boundary condition keep the reference's rules on the FP64 Gauss-point
 // displacement (pdDataManager.cpp:2604-2703) and store its difference.
-// SELL (sliced ELLPACK, 16 nodes per slice in the work order): contributor
-// slot k of the 16 nodes of a slice is stored side by side, so a warp's index
-// load reads 64 contiguous bytes and its coefficient load 512 (the CSR rows:
-// one 32-byte sector in each of 16 rows).  Every thread still walks only its
-// own node's contributors, in order: the same sums bit for bit.
 // The part of a gather thread's work that needs no contributor: the node's
 // trial displacement (u0, u1, u2) and its FP32 hi/lo split (group 0), and the
 // whole job for nodes with a boundary condition or without MLS.  True when
@@ -1278,7 +1274,7 @@ __device__ __forceinline__ bool gather_head(const Dev& d, const double* us, int6
 
 // PAT: contributor ids from the node's pattern (id offsets in an L1/L2-resident
 // table) instead of its list; the index load then no longer waits on memory.
-template <bool PERSIST, bool SELL = false, bool PAT = false>
+template <bool PERSIST, bool PAT = false>
 __device__ __forceinline__ void gather_group(const Dev& d, const double* us, int64_t tid, double t) {
     const int64_t N = d.n;
     const int npt = d.npt, ngrp = (npt + 3) / 4;
@@ -1296,22 +1292,14 @@ __device__ __forceinline__ void gather_group(const Dev& d, const double* us, int
         const int64_t q0 = __ldg(d.gpat_ptr + pid);
         nc = __ldg(d.gpat_ptr + pid + 1) - q0;
         po = d.gpat_off + q0;
-        if (!SELL) c0 = d.cbptr[i];
+        c0 = d.cbptr[i];
     } else {
         c0 = d.cbptr[i];
         nc = d.cbptr[i + 1] - c0;
     }
-    // contributor k: index cb[k * cs], coefficients cf[k * fs + q]
+    // contributor k: index cb[k], coefficients cf[k * npt + q]
     const int32_t* cb = d.cbidx + c0;
     const float* cf = d.coeff32 + c0 * npt + g0;
-    int64_t cs = 1, fs = npt;
-    if (SELL) {
-        const int64_t slot = tid / ngrp, sl = slot / kSell, l = slot % kSell, base = d.sell_off[sl];
-        cb = d.sell_idx + base * kSell + l;
-        cf = d.sell_coef + (base * kSell + l) * 8 + g0;
-        cs = kSell;
-        fs = kSell * 8;
-    }
     const bool vec = (ng == 4) && ((npt & 3) == 0);
     int64_t k = 0;
     if (vec) {
@@ -1322,8 +1310,8 @@ __device__ __forceinline__ void gather_group(const Dev& d, const double* us, int
             float4 cv[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                m[u] = PAT ? (int)i + __ldg(po + k + u) : __ldg(cb + (k + u) * cs);
-                cv[u] = ld4(cf + (k + u) * fs);
+                m[u] = PAT ? (int)i + __ldg(po + k + u) : __ldg(cb + k + u);
+                cv[u] = ld4(cf + (k + u) * npt);
             }
             double dd[4][3];
 #pragma unroll
@@ -1345,15 +1333,15 @@ __device__ __forceinline__ void gather_group(const Dev& d, const double* us, int
         }
     }
     for (; k < nc; ++k) {
-        const int64_t m = PAT ? i + po[k] : cb[k * cs];
+        const int64_t m = PAT ? i + po[k] : cb[k];
         const double d0 = ldm<PERSIST>(us + m) - u0, d1 = ldm<PERSIST>(us + N + m) - u1,
                      d2 = ldm<PERSIST>(us + 2 * N + m) - u2;
         float c[4];
         if (vec) {
-            const float4 v = ld4(cf + k * fs);
+            const float4 v = ld4(cf + k * npt);
             c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
         } else {
-            for (int q = 0; q < 4; ++q) c[q] = q < ng ? cf[k * fs + q] : 0.f;
+            for (int q = 0; q < 4; ++q) c[q] = q < ng ? cf[k * npt + q] : 0.f;
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1370,15 +1358,13 @@ __device__ __forceinline__ void gather_group(const Dev& d, const double* us, int
     }
 }
 
-template <bool SELL, bool PAT>
+template <bool PAT>
 __global__ void __launch_bounds__(256) k_gather_f32c(Dev d, const double* __restrict__ us) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (tid >= d.n * ((d.npt + 3) / 4)) return;
-    gather_group<false, SELL, PAT>(d, us, tid, *d.tdev);
+    gather_group<false, PAT>(d, us, tid, *d.tdev);
 }
 
-// 16-byte copy global -> shared that the thread waits for later (L2 only:
-// the coefficient stream is read once).
 // 16 bytes to shared memory with an L2 eviction policy (the coefficient stream is read once
 // per gather: evict it first, so that the node blocks the force reads next
 // stay in L2)
@@ -1403,7 +1389,9 @@ __device__ __forceinline__ void cp_async_wait() {
 // 16: 1.78; 24: 1.78)
 constexpr int kRingSlots = 16;
 
-// The SELL + pattern gather (2x2x2 points) with the coefficient stream run
+// The SELL (sliced ELLPACK, 16 nodes of the work order per slice: contributor
+// slot k of a slice's nodes side by side) + pattern gather (2x2x2 points) with
+// the coefficient stream run
 // through a shared-memory ring: each thread copies its own 16 bytes of each
 // contributor slot kRing slots ahead of the arithmetic (one commit group per
 // slot), so a warp keeps about 8 KB of the stream in flight without holding
@@ -1513,6 +1501,55 @@ __global__ void __launch_bounds__(256, 2) k_gather_f32c_ring(Dev d, const double
         o[8 + g0 + q] = (float)fma(S, u1, a[q][1]);
         o[16 + g0 + q] = (float)fma(S, u2, a[q][2]);
     }
+}
+
+// The gather of the 2x2x2 rule with a lane per point (gather_chunks): the same
+// FMAs in the same contributor order as gather_group, from the CSR lists: the
+// same result bit for bit.  Per launch: 61x47x9 83 -> 42 us, 13x11x7 41 -> 18,
+// 400x400x4 763 -> 521; shared-memory wavefronts 73 % busy.
+constexpr int kGatherStages = 4;
+__global__ void __launch_bounds__(128) k_gather_f32c_lanes(Dev d, const double* __restrict__ us) {
+    extern __shared__ __align__(16) char gather_sm[];
+    const int64_t N = d.n;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+    const int g = threadIdx.x & 7;
+    const bool live = slot < N;
+    const int64_t i = d.order[live ? slot : 0];
+    const bool free = live && d.bc[i] < 0;
+    const double u0 = us[i], u1 = us[N + i], u2 = us[2 * N + i];
+    const int64_t c0 = d.cbptr[i];
+    const int nc = free ? (int)(d.cbptr[i + 1] - c0) : 0;
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    gather_chunks<float, kGatherStages>(
+        gather_sm + (threadIdx.x >> 5) * gather_warp_bytes<float>(kGatherStages), d.coeff32 + c0 * 8, d.cbidx + c0, nc,
+        [&](int m, double* v) {
+            v[0] = us[m] - u0;
+            v[1] = us[N + m] - u1;
+            v[2] = us[2 * N + m] - u2;
+        },
+        [&](float c, const double* v) {
+            const double cd = (double)c;
+            a0 = fma(cd, v[0], a0);
+            a1 = fma(cd, v[1], a1);
+            a2 = fma(cd, v[2], a2);
+        });
+    if (!live) return;
+    const BlkOut o = blk_out(d, i);
+    if (!free) {  // nodes with a boundary condition, four points per call
+        double x0, x1, x2;
+        if (!(g & 3)) gather_head<false>(d, us, i, g >> 2, *d.tdev, o, x0, x1, x2);
+        return;
+    }
+    if (g < 3) {  // the node's own displacement, FP32 hi and lo
+        const double u = g == 0 ? u0 : (g == 1 ? u1 : u2);
+        const float h = (float)u;
+        o[24 + g] = h;
+        o[27 + g] = (float)(u - (double)h);
+    }
+    const double S = (double)d.csum[i * 8 + g];
+    o[g] = (float)fma(S, u0, a0);
+    o[8 + g] = (float)fma(S, u1, a1);
+    o[16 + g] = (float)fma(S, u2, a2);
 }
 
 // FP64 Gauss-point displacements from the node blocks the FP32 gather wrote:
@@ -1949,7 +1986,15 @@ void launch_gather_f32c(const Dev& d, const double* us, cudaStream_t s) {
     const int ngrp = (d.npt + 3) / 4;
     const unsigned nb = blocks_for(d.n * ngrp, 256);
     const bool sell = d.sell_on && d.sell_idx && d.mls && d.npt == 8, pat = d.gpat_id && d.mls;
-    if (sell && pat && d.npt == 8) {
+    // the ring wins once its stream of coefficients fills the memory system
+    // (640,000 nodes 433 us against 521, a batch of 97,000 121 against 125;
+    // 5,500 nodes 37 against 21)
+    const bool ring = sell && pat && d.n >= kStencilFrom;
+    if (d.npt == 8 && d.mls && !ring) {
+        k_gather_f32c_lanes<<<blocks_for(8 * d.n, 128), 128, 4 * gather_warp_bytes<float>(kGatherStages), s>>>(d, us);
+        return;
+    }
+    if (ring) {
         static bool attr = false;  // once per process: the ring needs more than the 48 KB default
         const size_t sh = (size_t)8 * kRingSlots * 32 * sizeof(float4);
         if (!attr) {
@@ -1957,12 +2002,10 @@ void launch_gather_f32c(const Dev& d, const double* us, cudaStream_t s) {
             attr = true;
         }
         k_gather_f32c_ring<kRingSlots><<<nb, 256, sh, s>>>(d, us);
-    } else if (sell) {
-        if (pat) k_gather_f32c<true, true><<<nb, 256, 0, s>>>(d, us);
-        else k_gather_f32c<true, false><<<nb, 256, 0, s>>>(d, us);
+    } else if (pat) {
+        k_gather_f32c<true><<<nb, 256, 0, s>>>(d, us);
     } else {
-        if (pat) k_gather_f32c<false, true><<<nb, 256, 0, s>>>(d, us);
-        else k_gather_f32c<false, false><<<nb, 256, 0, s>>>(d, us);
+        k_gather_f32c<false><<<nb, 256, 0, s>>>(d, us);
     }
 }
 
