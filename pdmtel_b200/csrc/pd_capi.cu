@@ -154,11 +154,23 @@ struct pd_ctx {
     double* hstage = nullptr;  // pinned host staging, 3N doubles x 2
     double* hscalar = nullptr; // pinned host scalars
     int* dflag = nullptr;      // device flags (pd_rk4_steps_host: the uploaded U differs)
-    // CUDA graph of one RK4 step
-    cudaGraphExec_t step_graph = nullptr;
-    double graph_dt = 0.0;
-    int graph_prec = -1, graph_energy = -1;
-    uint64_t generation = 0, graph_generation = ~0ull;
+    // what a step's launches depend on, and CUDA graphs of one RK4 step: [0] at
+    // a given time, [1] advancing it
+    struct StepKey {
+        double dt = 0.0;
+        int prec = -1, energy = -1;
+        uint64_t generation = ~0ull;
+        bool operator==(const StepKey& o) const {
+            return dt == o.dt && prec == o.prec && energy == o.energy && generation == o.generation;
+        }
+    };
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        StepKey key;
+    } graphs[2];
+    StepKey last_single;  // the last pd_rk4_step
+    double* ue = nullptr;    // [2][3N] one-point scheme: the displacements its bonds use, by stage
+    uint64_t generation = 0;
     uint64_t family_gen = 0;  // families installed
 };
 
@@ -217,9 +229,8 @@ int download_vec3(pd_ctx* c, double* dst_aos, const double* src_soa) {
 }
 
 int set_time(pd_ctx* c, double t) {
-    *c->hscalar = t;
-    PD_CUDA_TRY(cudaMemcpyAsync(c->d.tdev, c->hscalar, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    pd::launch_set_time(c->d.tdev, t, c->stream);
+    PD_CUDA_TRY(cudaGetLastError());
     return PD_OK;
 }
 
@@ -299,40 +310,68 @@ bool ready_dynamic(pd_ctx* c) {
     return true;
 }
 
-// the four stages of pdDataManager::RK4 and the closing gather
-void enqueue_step_body(pd_ctx* c, double dt, bool closing_gather = true) {
+// one stage's forces and epilogue (one launch where the force kernel takes the
+// epilogue along)
+void enqueue_stage(pd_ctx* c, bool f32, int stage, double dts, double dt) {
+    pd::Dev d = c->d;
+    if (c->ue && !f32) {
+        d.ue = c->ue + (stage & 1 ? 0 : 3 * c->n);
+        d.ue_next = c->ue + (stage & 1 ? 3 * c->n : 0);
+    }
+    const bool whole = f32 ? pd::launch_force_f32c(d, dts, c->stream, stage, dt)
+                           : pd::launch_force_f64(d, dts, c->stream, stage, dt);
+    if (!whole) pd::launch_epilogue(c->d, stage, dts, dt, c->stream);
+}
+
+// the four stages of pdDataManager::RK4 and the closing gather, after t += dt
+// when advance
+void enqueue_step_body(pd_ctx* c, double dt, bool advance, bool closing_gather = true) {
     cudaStream_t s = c->stream;
     const pd::Dev& d = c->d;
-    const int64_t n3 = 3 * c->n;
     const bool f32 = c->precision == PD_PREC_FP32C;
-    auto force = [&](double dts) {
-        if (f32) pd::launch_force_f32c(d, dts, s);
-        else pd::launch_force_f64(d, dts, s);
-    };
     auto gather = [&](const double* us) {
         if (f32) pd::launch_gather_f32c(d, us, s);
         else pd::launch_gather_f64(d, us, s);
     };
     const double dtHalf = 0.5 * dt;
-    // InitDynamicSolve: vbuf = V, energy density 0; u1 = us = U
-    cudaMemcpyAsync(d.vbuf, d.V, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.u1, d.U, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.us, d.U, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    if (d.energy) cudaMemsetAsync(d.eed, 0, sizeof(double) * c->n, s);
-    if (d.ai) cudaMemsetAsync(d.ai_dmg, 0, sizeof(int32_t) * c->n, s);
-    force(dtHalf);
-    pd::launch_epilogue(d, 1, dtHalf, dt, s);
+    pd::launch_step_begin(d, dt, advance, f32 ? nullptr : c->ue, s);
+    enqueue_stage(c, f32, 1, dtHalf, dt);
     gather(d.us);
-    force(dtHalf);
-    pd::launch_epilogue(d, 2, dtHalf, dt, s);
+    enqueue_stage(c, f32, 2, dtHalf, dt);
     gather(d.us);
-    force(dt);
-    pd::launch_epilogue(d, 3, dt, dt, s);
+    enqueue_stage(c, f32, 3, dt, dt);
     gather(d.us);
-    force(dt);
-    pd::launch_epilogue(d, 4, dt, dt, s);
+    enqueue_stage(c, f32, 4, dt, dt);
     if (d.energy) pd::launch_energy_reduce(d, s);
     if (closing_gather) gather(d.U);
+}
+
+// The graph of one step (with or without the time's advance), captured again
+// when what it holds has changed.
+int step_graph(pd_ctx* c, double dt, bool advance, cudaGraphExec_t* out) {
+    pd_ctx::StepGraph& G = c->graphs[advance];
+    const pd_ctx::StepKey key{dt, c->precision, c->d.energy, c->generation};
+    if (!G.exec || !(G.key == key)) {
+        if (G.exec) {
+            PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
+            cudaGraphExecDestroy(G.exec);
+            G.exec = nullptr;
+        }
+        cudaGraph_t g = nullptr;
+        PD_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        enqueue_step_body(c, dt, advance);
+        cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+        if (e != cudaSuccess) return pd::fail_cuda(e, "capture", __FILE__, __LINE__);
+        e = cudaGraphInstantiate(&G.exec, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) {
+            G.exec = nullptr;
+            return pd::fail_cuda(e, "instantiate", __FILE__, __LINE__);
+        }
+        G.key = key;
+    }
+    *out = G.exec;
+    return PD_OK;
 }
 
 // the closing gather of a step alone (CalcIntgPointDisplRK4 at the new U)
@@ -448,6 +487,7 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
         (rc = dalloc(c, &red, 2 * N + 4 + 2 * 160)) || (rc = dalloc(c, &tdev, 1)) ||
         (rc = dalloc(c, &c->dotpart, 2 * (N + 4096))) || (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
         return bail(rc);
+    if (d.cci && (rc = dalloc(c, &c->ue, 2 * n3)) != PD_OK) return bail(rc);
     if (c->nslit) {
         double* sl = nullptr;
         if ((rc = dalloc(c, &sl, 6 * c->nslit)) != PD_OK) return bail(rc);
@@ -608,7 +648,8 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
 int pd_ctx_destroy(pd_ctx* c) {
     if (!c) return PD_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
+    for (pd_ctx::StepGraph& G : c->graphs)
+        if (G.exec) cudaGraphExecDestroy(G.exec);
     if (c->persist_graph) cudaGraphExecDestroy(c->persist_graph);
     for (void* p : c->owned)
         if (p) cudaFree(p);
@@ -1810,7 +1851,16 @@ int pd_rk4_step(pd_ctx* c, double dt, double time, double* ke, double* ee) {
     if (!c) return fail(PD_ERR_ARG, "pd_rk4_step: null context");
     if (!ready_dynamic(c)) return fail(PD_ERR_ARG, "pd_rk4_step: family/MLS data not set");
     PD_TRY(set_time(c, time));
-    enqueue_step_body(c, dt);
+    // a step like the last one runs as a graph (a lone step is not worth the capture)
+    const pd_ctx::StepKey key{dt, c->precision, c->d.energy, c->generation};
+    if (c->last_single == key) {
+        cudaGraphExec_t g = nullptr;
+        PD_TRY(step_graph(c, dt, false, &g));
+        PD_CUDA_TRY(cudaGraphLaunch(g, c->stream));
+    } else {
+        enqueue_step_body(c, dt, false);
+        c->last_single = key;
+    }
     PD_CUDA_TRY(cudaGetLastError());
     if (c->d.energy && (ke || ee)) {
         PD_CUDA_TRY(cudaMemcpyAsync(c->hscalar, c->d.red + 2 * c->n, 2 * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1827,27 +1877,9 @@ int pd_rk4_steps(pd_ctx* c, double dt, double t0, int nsteps) {
     if (!ready_dynamic(c)) return fail(PD_ERR_ARG, "pd_rk4_steps: family/MLS data not set");
     if (nsteps == 0) return PD_OK;
     PD_TRY(set_time(c, t0));
-    if (!c->step_graph || c->graph_dt != dt || c->graph_prec != c->precision || c->graph_energy != c->d.energy ||
-        c->graph_generation != c->generation) {
-        if (c->step_graph) {
-            cudaGraphExecDestroy(c->step_graph);
-            c->step_graph = nullptr;
-        }
-        cudaGraph_t g = nullptr;
-        PD_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        pd::launch_advance_time(c->d.tdev, dt, c->stream);
-        enqueue_step_body(c, dt);
-        cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-        if (e != cudaSuccess) return pd::fail_cuda(e, "capture", __FILE__, __LINE__);
-        e = cudaGraphInstantiate(&c->step_graph, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return pd::fail_cuda(e, "instantiate", __FILE__, __LINE__);
-        c->graph_dt = dt;
-        c->graph_prec = c->precision;
-        c->graph_energy = c->d.energy;
-        c->graph_generation = c->generation;
-    }
-    for (int k = 0; k < nsteps; ++k) PD_CUDA_TRY(cudaGraphLaunch(c->step_graph, c->stream));
+    cudaGraphExec_t g = nullptr;
+    PD_TRY(step_graph(c, dt, true, &g));
+    for (int k = 0; k < nsteps; ++k) PD_CUDA_TRY(cudaGraphLaunch(g, c->stream));
     PD_CUDA_TRY(cudaGetLastError());
     return PD_OK;
 }
@@ -1892,8 +1924,7 @@ int pd_rk4_steps_host(pd_ctx* c, double dt, double t0, int nsteps, const double*
             PD_CUDA_TRY(cudaEventCreateWithFlags(&c->ev_final, cudaEventDisableTiming));
             PD_CUDA_TRY(cudaEventCreateWithFlags(&c->ev_copied, cudaEventDisableTiming));
         }
-        pd::launch_advance_time(c->d.tdev, dt, c->stream);
-        enqueue_step_body(c, dt, false);
+        enqueue_step_body(c, dt, true, false);
         PD_CUDA_TRY(cudaEventRecord(c->ev_final, c->stream));
         PD_CUDA_TRY(cudaStreamWaitEvent(c->copy_stream, c->ev_final, 0));
         enqueue_closing_gather(c);
@@ -1949,7 +1980,6 @@ int pd_profile_step(pd_ctx* c, double dt, double time, double* ms) {
     cudaStream_t s = c->stream;
     const pd::Dev& d = c->d;
     const bool f32 = c->precision == PD_PREC_FP32C;
-    const int64_t n3 = 3 * c->n;
     std::vector<cudaEvent_t> ev;
     std::vector<int> cls;
     auto mark = [&](int k) {
@@ -1978,10 +2008,7 @@ int pd_profile_step(pd_ctx* c, double dt, double time, double* ms) {
     };
     const double h = 0.5 * dt;
     mark(-1);
-    cudaMemcpyAsync(d.vbuf, d.V, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.u1, d.U, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.us, d.U, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    if (d.energy) cudaMemsetAsync(d.eed, 0, sizeof(double) * c->n, s);
+    pd::launch_step_begin(d, dt, false, nullptr, s);
     mark(3);
     force(h); epi(1, h);
     gather(d.us); force(h); epi(2, h);
@@ -2499,34 +2526,23 @@ void enqueue_step_tape(pd_ctx* c, double dt, double* tape, bool f32) {
         if (f32) pd::launch_blocks_to_ug(d, t + 2 * n3, s);
         else cudaMemcpyAsync(t + 2 * n3, d.ug, sizeof(double) * ng, cudaMemcpyDeviceToDevice, s);
     };
-    auto force = [&](double dts) {
-        if (f32) pd::launch_force_f32c(d, dts, s);
-        else pd::launch_force_f64(d, dts, s);
-    };
     auto gather = [&](const double* us) {
         if (f32) pd::launch_gather_f32c(d, us, s);
         else pd::launch_gather_f64(d, us, s);
     };
     const double h = 0.5 * dt;
-    pd::launch_advance_time(d.tdev, dt, s);
-    cudaMemcpyAsync(d.vbuf, d.V, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.u1, d.U, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.us, d.U, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s);
+    pd::launch_step_begin(d, dt, true, f32 ? nullptr : c->ue, s);
     copy(1);
-    force(h);
-    pd::launch_epilogue(d, 1, h, dt, s);
+    enqueue_stage(c, f32, 1, h, dt);
     gather(d.us);
     copy(2);
-    force(h);
-    pd::launch_epilogue(d, 2, h, dt, s);
+    enqueue_stage(c, f32, 2, h, dt);
     gather(d.us);
     copy(3);
-    force(dt);
-    pd::launch_epilogue(d, 3, dt, dt, s);
+    enqueue_stage(c, f32, 3, dt, dt);
     gather(d.us);
     copy(4);
-    force(dt);
-    pd::launch_epilogue(d, 4, dt, dt, s);
+    enqueue_stage(c, f32, 4, dt, dt);
     gather(d.U);
 }
 

@@ -143,19 +143,23 @@ __device__ __forceinline__ bool point_rn(const BetaIn& B, double bE, double c, d
 // then add the round's L bonds in family order, so every sum has the
 // reference's terms in the reference's order, bit for bit.  Lanes past the
 // family's end store -0.0, which changes no sum.  UNI: the 2x2x2 rule with
-// equal weights, four points unrolled (their offsets are two per axis, so they
-// share squares), twice; else any rule, point by point.
+// equal weights, its points in four pairs (their offsets are two per axis, so
+// they share squares); else any rule, point by point.  stage 1..4: the stage's
+// epilogue follows on the same lanes (stage_axis), which saves a launch and a
+// round trip of vbuf per stage; the one-point scheme, whose bonds read their
+// far nodes' displacements, then reads ue and leaves the next stage's in
+// ue_next.
 //
 // Bound by the FP64 pipe and the latency of its chains: 146 instructions per
-// evaluation, about 71 of them FP64 (pipe 53 % busy at 168 registers and three
-// blocks per SM; four blocks at 128 registers measured 1.54-1.57 ms, two at
-// 196 1.82, all eight points unrolled 1.67-1.91).  200x200x4 cracked plate, per
-// launch: 3.86 -> 1.50 ms against one thread per node with the compiler's
-// square roots and divisions (474 instructions); 20x10x10 bar with energies
-// 560 -> 62 us, 10x10x10 CCI cube 568 -> 17 us, where one thread (or eight
-// lanes) per node left a serial chain of 250 bonds on a few SMs.
+// evaluation, about 71 of them FP64 (pipe 53 % busy), and no faster with more
+// warps (five blocks per SM 1.51 ms, six 1.48, against 1.45 with four; four
+// points side by side at three blocks 1.50, all eight 1.67-1.91).  200x200x4
+// cracked plate, per launch: 3.86 -> 1.45 ms against one thread per node with
+// the compiler's square roots and divisions (474 instructions); 20x10x10 bar
+// with energies 560 -> 62 us, 10x10x10 CCI cube 568 -> 17 us, where one thread
+// (or eight lanes) per node left a serial chain of 250 bonds on a few SMs.
 template <bool CCI, bool ENERGY, bool SFAC, bool ACC, bool UNI, int L>
-__global__ void __launch_bounds__(128, 3) k_force_f64(Dev d, double dts) {
+__global__ void __launch_bounds__(128, 4) k_force_f64(Dev d, double dts, int stage, double dt) {
     constexpr int GS = 3 * L + 4;  // shared doubles per group: 4 more than its bonds, so that groups differ in bank
     constexpr int G = 32 / L;
     extern __shared__ double sh64[];
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(128, 3) k_force_f64(Dev d, double dts) {
     const double rho = Mi.density, yrho = 1.0 / rho;
     const bool rho_ok = rn_range(rho);
     const double b0 = Mi.grav[0] * rho, b1 = Mi.grav[1] * rho, b2 = Mi.grav[2] * rho;
-    const double* src = (d.bc[i] >= 0) ? d.U : d.us;
+    const double* src = CCI && d.ue ? d.ue : ((d.bc[i] >= 0) ? d.U : d.us);
     const double ui0 = src[i], ui1 = src[N + i], ui2 = src[2 * N + i];
     const double xi0 = d.x[i], xi1 = d.x[N + i], xi2 = d.x[2 * N + i];
     const double bEi = d.bdry[i];
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(128, 3) k_force_f64(Dev d, double dts) {
             const bool c_ok = !ENERGY || rn_quotient_ok(c);
             double F0 = 0.0, F1 = 0.0, F2 = 0.0;
             if (CCI) {
-                const double* sj = (d.bc[j] >= 0) ? d.U : d.us;
+                const double* sj = d.ue ? d.ue : ((d.bc[j] >= 0) ? d.U : d.us);
                 const double x0 = xj0 - xi0, x1 = xj1 - xi1, x2 = xj2 - xi2;
                 const double e0 = sj[j] - ui0, e1 = sj[N + j] - ui1, e2 = sj[2 * N + j] - ui2;
                 double el = 0.0;
@@ -231,17 +235,18 @@ __global__ void __launch_bounds__(128, 3) k_force_f64(Dev d, double dts) {
                 const double xc[2] = {(hlo + xj2) - xi2, (hhi + xj2) - xi2};
                 bool ok = c_ok;
 #pragma unroll 1
-                for (int a = 0; a < 2; ++a) {
-                    const double x0 = a ? xa[1] : xa[0];
+                for (int a = 0; a < 4; ++a) {
+                    const double x0 = a & 2 ? xa[1] : xa[0], x1 = a & 1 ? xb[1] : xb[0];
+                    const double x01 = x0 * x0 + x1 * x1;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int g = 4 * a + q;
-                        const double x1 = xb[q >> 1], x2 = xc[q & 1];
+                    for (int q = 0; q < 2; ++q) {
+                        const int g = 2 * a + q;
+                        const double x2 = xc[q];
                         const double* ugp = d.ug + (int64_t)(3 * g) * N + j;
                         double f0, f1, f2, el;
-                        ok &= point_rn<false, ENERGY, ACC>(B, bE, c, ecp, 0.0, pw3, x0, x1, x2,
-                                                           x0 * x0 + x1 * x1 + x2 * x2, ugp[0] - ui0, ugp[N] - ui1,
-                                                           ugp[2 * N] - ui2, f0, f1, f2, el);
+                        ok &= point_rn<false, ENERGY, ACC>(B, bE, c, ecp, 0.0, pw3, x0, x1, x2, x01 + x2 * x2,
+                                                           ugp[0] - ui0, ugp[N] - ui1, ugp[2 * N] - ui2, f0, f1, f2,
+                                                           el);
                         F0 += W * f0;
                         F1 += W * f1;
                         F2 += W * f2;
@@ -310,8 +315,23 @@ __global__ void __launch_bounds__(128, 3) k_force_f64(Dev d, double dts) {
         }
         __syncwarp();
     }
-    if (live && ql < 3) d.vbuf[(int64_t)ql * N + i] = acc;
     if (ENERGY && live && ql == 3) d.eed[i] = acc;
+    if (stage < 0) {
+        if (live && ql < 3) d.vbuf[(int64_t)ql * N + i] = acc;
+        return;
+    }
+    double v = acc;
+    if (live && ql < 3) {
+        double eff;
+        v = stage_axis<false>(d, i, ql, stage, dts, dt, *d.tdev, rho, acc, eff);
+        if (CCI) d.ue_next[(int64_t)ql * N + i] = eff;
+    }
+    if (ENERGY && stage == 4) {  // the lanes of a group hold v0, v1, v2 and the energy density
+        const int first = lane - ql;
+        const double v0 = __shfl_sync(0xffffffffu, v, first), v1 = __shfl_sync(0xffffffffu, v, first + 1),
+                     v2 = __shfl_sync(0xffffffffu, v, first + 2), e = __shfl_sync(0xffffffffu, v, first + 3);
+        if (live && ql == 0) stage_energy(d, i, rho, v0, v1, v2, e);
+    }
 }
 
 // ----------------------------------------------------------------- gather
@@ -440,12 +460,21 @@ __global__ void __launch_bounds__(128) k_gather_f64_lanes(Dev d, const double* _
 // k = vbuf*dt_s (:1977-1990) and the RK4 bookkeeping of pdDataManager::RK4
 // (:2027-2092): next trial displacement, k3 += k2, and at stage 4 the
 // combination, the damping and the new velocity.
-__global__ void k_epilogue(Dev d, int stage, double dts, double dt) {
+// Bound by memory: a thread per component (per node where the energies need
+// all three).  640,000 nodes: 27 us with a thread per node and U and vbuf
+// always rewritten, 20 us now.
+template <int STAGE>
+__global__ void k_epilogue(Dev d, double dts, double dt) {
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k >= 3 * d.n) return;
+    const int a = k >= 2 * d.n ? 2 : (k >= d.n ? 1 : 0);
+    const int64_t i = k - a * d.n;
+    double eff;
+    stage_axis<true>(d, i, a, STAGE, dts, dt, *d.tdev, d.mats[d.mat[i]].density, __ldcg(d.vbuf + k), eff);
+}
+__global__ void k_epilogue_energy(Dev d, int stage, double dts, double dt) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
-    const double t = *d.tdev;
-    if (d.energy) stage_epilogue<true>(d, i, stage, dts, dt, t);
-    else stage_epilogue<false>(d, i, stage, dts, dt, t);
+    if (i < d.n) stage_epilogue<true>(d, i, stage, dts, dt, *d.tdev);
 }
 
 // Deterministic two-level sum of red[0..N) and red[N..2N) into red[2N], red[2N+1].
@@ -472,16 +501,17 @@ __global__ void k_energy_partial(const double* __restrict__ red, int64_t N, doub
     }
 }
 
-__global__ void k_energy_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double a = 0.0, c = 0.0;
-        for (int k = 0; k < nb; ++k) {
-            a += part[2 * k];
-            c += part[2 * k + 1];
-        }
-        out[0] = a;
-        out[1] = c;
-    }
+// The sums of the blocks' partial sums in block order: all loads first, then
+// one thread per sum.
+__global__ void __launch_bounds__(256) k_energy_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
+    __shared__ double sp[2 * 256];
+    for (int k = threadIdx.x; k < 2 * nb; k += blockDim.x) sp[k] = part[k];
+    __syncthreads();
+    if (threadIdx.x >= 2) return;
+    double a = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < nb; ++k) a += sp[2 * k + threadIdx.x];
+    out[threadIdx.x] = a;
 }
 
 __global__ void k_to_soa(const double* __restrict__ aos, double* __restrict__ soa, int64_t n, int comps) {
@@ -522,12 +552,13 @@ inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) /
 
 }  // namespace
 
-void launch_force_f64(const Dev& d, double dts, cudaStream_t s) {
-    if (d.n == 0) return;
+bool launch_force_f64(const Dev& d, double dts, cudaStream_t s, int stage, double dt) {
+    if (d.n == 0) return true;
     if (d.ai) {
         launch_ai_force(d, dts, s);
-        return;
+        return false;
     }
+    if (d.cci && !d.ue) stage = -1;
     // The 2x2x2 rule with equal weights takes the unrolled form.  A small
     // problem gives a node a whole warp, so that the SMs fill; a larger one
     // eight lanes, which waste fewer on a family's last round and add its bonds
@@ -546,7 +577,7 @@ void launch_force_f64(const Dev& d, double dts, cudaStream_t s) {
     const bool sf = d.sfac != nullptr;
     auto go = [&](auto kernel) {
         if (sh > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-        kernel<<<nb, 32 * warps, sh, s>>>(d, dts);
+        kernel<<<nb, 32 * warps, sh, s>>>(d, dts, stage, dt);
     };
     auto lanes_of = [&](auto C, auto E, auto S, auto A, auto Un) {
         constexpr bool c = decltype(C)::value, e = decltype(E)::value, f = decltype(S)::value;
@@ -565,6 +596,7 @@ void launch_force_f64(const Dev& d, double dts, cudaStream_t s) {
     };
     if (d.energy) { if (sf) form(std::true_type{}, std::true_type{}); else form(std::true_type{}, std::false_type{}); }
     else { if (sf) form(std::false_type{}, std::true_type{}); else form(std::false_type{}, std::false_type{}); }
+    return stage > 0;
 }
 
 void launch_gather_f64(const Dev& d, const double* us, cudaStream_t s) {
@@ -584,7 +616,13 @@ void launch_gather_f64(const Dev& d, const double* us, cudaStream_t s) {
 void launch_epilogue(const Dev& d, int stage, double dts, double dt, cudaStream_t s) {
     if (d.n == 0) return;
     const int bs = 256;
-    k_epilogue<<<blocks_for(d.n, bs), bs, 0, s>>>(d, stage, dts, dt);
+    const unsigned nb = blocks_for(3 * d.n, bs);
+    if (d.energy) k_epilogue_energy<<<blocks_for(d.n, bs), bs, 0, s>>>(d, stage, dts, dt);
+    else if (stage == 0) k_epilogue<0><<<nb, bs, 0, s>>>(d, dts, dt);
+    else if (stage == 1) k_epilogue<1><<<nb, bs, 0, s>>>(d, dts, dt);
+    else if (stage == 2) k_epilogue<2><<<nb, bs, 0, s>>>(d, dts, dt);
+    else if (stage == 3) k_epilogue<3><<<nb, bs, 0, s>>>(d, dts, dt);
+    else k_epilogue<4><<<nb, bs, 0, s>>>(d, dts, dt);
 }
 
 // t += dt on the device, as pdSolve.cpp:61 advances currentTime
@@ -594,11 +632,33 @@ __global__ void k_advance_time(double* t, double dt) {
 
 void launch_advance_time(double* t, double dt, cudaStream_t s) { k_advance_time<<<1, 32, 0, s>>>(t, dt); }
 
+__global__ void k_set_time(double* t, double v) { *t = v; }
+void launch_set_time(double* t, double v, cudaStream_t s) { k_set_time<<<1, 1, 0, s>>>(t, v); }
+
+// One launch for what were three copies, one or two fills and the time's
+// advance: at a few thousand nodes each cost a launch of about 2 us.
+__global__ void k_step_begin(Dev d, double dt, int advance, double* ue) {
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k == 0 && advance) *d.tdev = *d.tdev + dt;
+    if (k >= 3 * d.n) return;
+    const double U = d.U[k];
+    d.vbuf[k] = d.V[k];
+    d.u1[k] = U;
+    d.us[k] = U;
+    if (ue) ue[k] = U;
+    if (k >= d.n) return;
+    if (d.energy) d.eed[k] = 0.0;
+    if (d.ai) d.ai_dmg[k] = 0;
+}
+void launch_step_begin(const Dev& d, double dt, bool advance, double* ue, cudaStream_t s) {
+    k_step_begin<<<std::max(1u, blocks_for(3 * d.n, 256)), 256, 0, s>>>(d, dt, advance, ue);
+}
+
 void launch_energy_reduce(const Dev& d, cudaStream_t s) {
     const int nb = 148;
     double* part = d.red + 2 * d.n + 2;
     k_energy_partial<<<nb, 256, 0, s>>>(d.red, d.n, part);
-    k_energy_final<<<1, 32, 0, s>>>(part, nb, d.red + 2 * d.n);
+    k_energy_final<<<1, 256, 0, s>>>(part, nb, d.red + 2 * d.n);
 }
 
 // ============================================================ MLS setup

@@ -496,14 +496,19 @@ __host__ __device__ constexpr int lane_group_words(int L) { return L == 4 ? 20 :
 // bit.  A round's 32 neighbour blocks (128 bytes each) are copied to shared
 // memory a round ahead, eight lanes to a block, so that a load touches four
 // lines where a lane reading its own neighbour would touch 32.
+// stage 1..4: the stage's epilogue follows on the lanes that hold the sums
+// (the 26,000-node case 2.43 -> 2.34 ms per 4 steps).  The stencil kernel does
+// without: the epilogue costs its loop registers (24-36 bytes spilt, 16 before;
+// 640,000 nodes 24.9 -> 25.4 ms, a batch of 97,000 8.23 -> 8.40).
 template <bool HASFAIL, bool LAT, bool BDRY, bool SFAC, bool MULTIMAT, int L, bool CM>
-__global__ void __launch_bounds__(128, 4) k_force_f32c_lanes(Dev d, const __grid_constant__ PointPack<8> G, double dts) {
+__global__ void __launch_bounds__(128, 4) k_force_f32c_lanes(Dev d, const __grid_constant__ PointPack<8> G,
+                                                             double dts, int stage, double dt) {
     constexpr int GS = lane_group_words(L);
     constexpr int kRow = kTileStride;
     extern __shared__ float4 lane_sm[];
     const int lane = threadIdx.x & 31, ql = lane % L, grp = lane / L;
-    float* stage = reinterpret_cast<float*>(lane_sm) + (threadIdx.x >> 5) * (2 * 32 * kRow + 32 / L * GS);
-    float* prod = stage + 2 * 32 * kRow + grp * GS;
+    float* ring = reinterpret_cast<float*>(lane_sm) + (threadIdx.x >> 5) * (2 * 32 * kRow + 32 / L * GS);
+    float* prod = ring + 2 * 32 * kRow + grp * GS;
     const int64_t N = d.n;
     const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
     const bool live = slot < N;
@@ -517,7 +522,7 @@ __global__ void __launch_bounds__(128, 4) k_force_f32c_lanes(Dev d, const __grid
     float sum = 0.f, comp = 0.f;  // Kahan sum of component ql of the family force (ql < 3)
     auto neighbour = [&](int base) { return base + ql < cnt ? d.acol[row + base + ql] : (int)i; };
     auto fetch = [&](int j, int buf) {  // the blocks of the warp's 32 neighbours
-        float* to = stage + buf * 32 * kRow + (CM ? lane * kRow : (lane >> 3) * kRow + 4 * (lane & 7));
+        float* to = ring + buf * 32 * kRow + (CM ? lane * kRow : (lane >> 3) * kRow + 4 * (lane & 7));
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             if (CM) {
@@ -563,7 +568,7 @@ __global__ void __launch_bounds__(128, 4) k_force_f32c_lanes(Dev d, const __grid
         const float epsc = HASFAIL ? eps_crit(ecrit) : 0.f;
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
-        const float* bj = stage + buf * 32 * kRow + lane * kRow;
+        const float* bj = ring + buf * 32 * kRow + lane * kRow;
         const float4 us0 = *reinterpret_cast<const float4*>(bj + 24), us1 = *reinterpret_cast<const float4*>(bj + 28);
         const float du[3] = {split_diff(us0.x, us0.w, O.uh[0], O.ul[0]), split_diff(us0.y, us1.x, O.uh[1], O.ul[1]),
                              split_diff(us0.z, us1.y, O.uh[2], O.ul[2])};
@@ -612,7 +617,10 @@ __global__ void __launch_bounds__(128, 4) k_force_f32c_lanes(Dev d, const __grid
         const MatDev& M = d.mats[O.mat];
         const double rho = M.density;
         const double v0 = d.vbuf[ql * N + i];
-        d.vbuf[ql * N + i] = v0 + ((double)sum - (double)comp + (double)cnt * (M.grav[ql] * rho)) * dts / rho;
+        const double v = v0 + ((double)sum - (double)comp + (double)cnt * (M.grav[ql] * rho)) * dts / rho;
+        double eff;
+        if (stage > 0) stage_axis<false>(d, i, ql, stage, dts, dt, *d.tdev, rho, v, eff);
+        else d.vbuf[ql * N + i] = v;
     }
 }
 
@@ -1825,14 +1833,15 @@ inline int force_lanes(const Dev& d) { return d.n < 12288 ? 32 : (d.n < 131072 ?
 // against 298, a batch of 97,000 375 against 432).
 constexpr int64_t kStencilFrom = 65536;
 
-void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
-    if (d.n == 0) return;
+bool launch_force_f32c(const Dev& d, double dts, cudaStream_t s, int stage, double dt) {
+    if (d.n == 0) return true;
+    if (d.energy) stage = -1;  // the energies are the epilogue kernel's
     const unsigned nb = blocks_for(d.n, 128);
     if (d.cci) {
         k_pack_cci<<<blocks_for(d.n, 256), 256, 0, s>>>(d);
         if (d.sfac) k_force_f32c_cci<true><<<nb, 128, 0, s>>>(d, dts);
         else k_force_f32c_cci<false><<<nb, 128, 0, s>>>(d, dts);
-        return;
+        return false;
     }
     const int lanes = force_lanes(d);
     const unsigned nbl = blocks_for(lanes * d.n, 128);
@@ -1842,8 +1851,8 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
         const PointPack<8> P = pack_points<8>(d, d.gc_host);
 #define PD_STEN_L(HF, BD, SF)                                                                                  \
     do {                                                                                                       \
-        if (lanes == 32) k_force_f32c_lanes<HF, true, BD, SF, false, 32, true><<<nbl, 128, shl, s>>>(d, P, dts); \
-        else k_force_f32c_lanes<HF, true, BD, SF, false, 8, true><<<nbl, 128, shl, s>>>(d, P, dts);             \
+        if (lanes == 32) k_force_f32c_lanes<HF, true, BD, SF, false, 32, true><<<nbl, 128, shl, s>>>(d, P, dts, stage, dt); \
+        else k_force_f32c_lanes<HF, true, BD, SF, false, 8, true><<<nbl, 128, shl, s>>>(d, P, dts, stage, dt);             \
     } while (0)
         if (d.hasfail) {
             if (bd) { if (sf) PD_STEN_L(true, true, true); else PD_STEN_L(true, true, false); }
@@ -1853,7 +1862,7 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
             else { if (sf) PD_STEN_L(false, false, true); else PD_STEN_L(false, false, false); }
         }
 #undef PD_STEN_L
-        return;
+        return stage > 0;
     }
     if (d.blk_cm && d.sten_mask && d.npt == 8 && d.gc_host) {
         // the gather stores chunk-major blocks
@@ -1873,7 +1882,7 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
             else { if (sf) PD_STEN(false, false, true); else PD_STEN(false, false, false); }
         }
 #undef PD_STEN
-        return;
+        return false;
     }
     if (d.npt == 8 && d.gc_host && d.tile_x > 0 && d.lat && d.pos2id) {
         const PointPack<8> P = pack_points<8>(d, d.gc_host);
@@ -1890,7 +1899,7 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
             if (sf) k_force_f32c_tiled<false, false, true, false><<<nt, bs, sh, s>>>(d, P, dts);
             else k_force_f32c_tiled<false, false, false, false><<<nt, bs, sh, s>>>(d, P, dts);
         }
-        return;
+        return false;
     }
     if (d.npt == 8 && d.gc_host && d.force_quad && d.lat && !d.hasfail && !d.multimat) {
         const PointPack<8> P = pack_points<8>(d, d.gc_host);
@@ -1903,16 +1912,16 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
             if (sf) k_force_f32c_quad<false, true><<<nq, 128, 0, s>>>(d, P, dts);
             else k_force_f32c_quad<false, false><<<nq, 128, 0, s>>>(d, P, dts);
         }
-        return;
+        return false;
     }
     if (d.npt == 8 && d.gc_host) {
         const PointPack<8> P = pack_points<8>(d, d.gc_host);
         const bool lat = d.lat != nullptr, bd = d.bdry_on != 0, sf = d.sfac != nullptr;
 #define PD_F32(HF, LT, BD, SF, MM)                                                         \
     do {                                                                                   \
-        if (lanes == 32) k_force_f32c_lanes<HF, LT, BD, SF, MM, 32, false><<<nbl, 128, shl, s>>>(d, P, dts); \
-        else if (lanes == 8) k_force_f32c_lanes<HF, LT, BD, SF, MM, 8, false><<<nbl, 128, shl, s>>>(d, P, dts); \
-        else k_force_f32c_lanes<HF, LT, BD, SF, MM, 4, false><<<nbl, 128, shl, s>>>(d, P, dts); \
+        if (lanes == 32) k_force_f32c_lanes<HF, LT, BD, SF, MM, 32, false><<<nbl, 128, shl, s>>>(d, P, dts, stage, dt); \
+        else if (lanes == 8) k_force_f32c_lanes<HF, LT, BD, SF, MM, 8, false><<<nbl, 128, shl, s>>>(d, P, dts, stage, dt); \
+        else k_force_f32c_lanes<HF, LT, BD, SF, MM, 4, false><<<nbl, 128, shl, s>>>(d, P, dts, stage, dt); \
     } while (0)
         if (d.hasfail || d.multimat) {
             PD_F32(true, false, true, true, true);
@@ -1924,10 +1933,11 @@ void launch_force_f32c(const Dev& d, double dts, cudaStream_t s) {
             else { if (sf) PD_F32(false, false, false, true, false); else PD_F32(false, false, false, false, false); }
         }
 #undef PD_F32
-        return;
+        return stage > 0;
     }
     if (d.sfac) k_force_f32c_any<true><<<nb, 128, 0, s>>>(d, dts);
     else k_force_f32c_any<false><<<nb, 128, 0, s>>>(d, dts);
+    return false;
 }
 
 // The persistent kernel's variant for the problem, and how many of its

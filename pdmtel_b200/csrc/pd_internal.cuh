@@ -76,6 +76,10 @@ struct Dev {
     double* vbuf;
     double* u1;
     double* us;
+    // one-point scheme with fused epilogues: the displacement every node's bonds
+    // use in this stage and in the next ([3][N] each; null: U or us per node)
+    const double* ue;
+    double* ue_next;
     double* k1;
     double* k2;
     double* k32;
@@ -173,9 +177,15 @@ struct Dev {
 };
 
 // kernel launchers (pd_exact.cu: compiled without FMA contraction)
-void launch_force_f64(const Dev& d, double dts, cudaStream_t s);
+// The forces of a stage.  stage 1..4 asks for the stage's epilogue in the same
+// kernel (with ue / ue_next set for the one-point scheme); true when it ran.
+bool launch_force_f64(const Dev& d, double dts, cudaStream_t s, int stage = -1, double dt = 0.0);
 void launch_gather_f64(const Dev& d, const double* us, cudaStream_t s);
 void launch_epilogue(const Dev& d, int stage, double dts, double dt, cudaStream_t s);
+// the start of a step (InitDynamicSolve: vbuf = V, u1 = us = U, energy density and
+// AI damage counts zero; ue, if set, = U), after t += dt when advance
+void launch_step_begin(const Dev& d, double dt, bool advance, double* ue, cudaStream_t s);
+void launch_set_time(double* t, double v, cudaStream_t s);
 void launch_advance_time(double* t, double dt, cudaStream_t s);
 void launch_energy_reduce(const Dev& d, cudaStream_t s);
 // InitIntegrationPoint on the device (k_mls_contrib, k_mls_coeff): contributor
@@ -215,7 +225,7 @@ void launch_ai_gather(const Dev& d, const double* us, cudaStream_t s);
 void launch_ai_force(const Dev& d, double dts, cudaStream_t s);
 
 // FP32 compensated form (pd_f32c.cu)
-void launch_force_f32c(const Dev& d, double dts, cudaStream_t s);
+bool launch_force_f32c(const Dev& d, double dts, cudaStream_t s, int stage = -1, double dt = 0.0);
 void launch_gather_f32c(const Dev& d, const double* us, cudaStream_t s);
 void launch_pack_cci_f32c(const Dev& d, cudaStream_t s);
 size_t tiled_smem_bytes(const Dev& d);

@@ -21,78 +21,95 @@ __device__ __forceinline__ double bc_time_factor(const BcDev& b, double t) {
 }
 
 // After the bond forces of stage `stage` (1..4; 0 for a lone stage whose k
-// goes to k1) have been added to vbuf at time t: the traction load (project
-// rule: value*factor/dx added to vbuf once per stage), UpdateNodeStatusWithBC
-// (pdDataManager.cpp:2497-2602), k = vbuf*dt_s (:1977-1990) and the RK4
-// bookkeeping of pdDataManager::RK4 (:2027-2092).  With ENERGY, stage 4
-// leaves the node's kinetic and elastic energy in red[i], red[N+i].
-template <bool ENERGY>
-__device__ __forceinline__ void stage_epilogue(const Dev& d, int64_t i, int stage, double dts, double dt, double t) {
-    const int64_t N = d.n;
-    const double rho = d.mats[d.mat[i]].density;
-    double v[3] = {__ldcg(d.vbuf + i), __ldcg(d.vbuf + N + i), __ldcg(d.vbuf + 2 * N + i)};
-    double U[3] = {__ldcg(d.U + i), __ldcg(d.U + N + i), __ldcg(d.U + 2 * N + i)};
+// goes to k1) have been added to vbuf at time t, component a of node i: the
+// traction load (project rule: value*factor/dx added to vbuf once per stage),
+// UpdateNodeStatusWithBC (pdDataManager.cpp:2497-2602), k = vbuf*dt_s
+// (:1977-1990) and the RK4 bookkeeping of pdDataManager::RK4 (:2027-2092).  v:
+// the component of vbuf with the stage's forces (HELD: vbuf itself holds it);
+// returns its final value.  eff: the displacement a one-point force of the next
+// stage uses for the node.  U and a held vbuf are touched only where a
+// condition or the last stage may change them: two passes over each less in
+// three stages of four.
+template <bool HELD>
+__device__ __forceinline__ double stage_axis(const Dev& d, int64_t i, int a, int stage, double dts, double dt, double t,
+                                             double rho, double v, double& eff) {
+    const int64_t N = d.n, r = a * N + i;
     const int b = d.bc[i];
+    const bool changes = b >= 0 || stage == 4;
+    double U = changes ? __ldcg(d.U + r) : 0.0;
     if (b >= 0) {
         const BcDev& B = d.bcs[b];
-        const double fac = bc_time_factor(B, t);
-        const double X[3] = {d.x[i], d.x[N + i], d.x[2 * N + i]};
-        for (int a = 0; a < 3; ++a) {
-            if (B.dir[a] != 1) continue;
+        if (B.dir[a] == 1) {
+            const double fac = bc_time_factor(B, t);
             if (B.type == PD_BC_TRACTION) {
                 const double tb = __ddiv_rn(__dmul_rn(B.val[a], fac), d.dx);
-                v[a] = __dadd_rn(v[a], __ddiv_rn(__dmul_rn(tb, dts), rho));
+                v = __dadd_rn(v, __ddiv_rn(__dmul_rn(tb, dts), rho));
             } else if (B.type == PD_BC_DISPL) {
-                U[a] = __dmul_rn(B.val[a], fac);
-                v[a] = 0.0;
+                U = __dmul_rn(B.val[a], fac);
+                v = 0.0;
             } else if (B.type == PD_BC_VELOC) {
-                v[a] = __dmul_rn(B.val[a], fac);
+                v = __dmul_rn(B.val[a], fac);
             } else if (B.type == PD_BC_DISPLGRAD) {
-                const double e = __dadd_rn(__dadd_rn(__dmul_rn(B.val[3 * a], X[0]), __dmul_rn(B.val[3 * a + 1], X[1])),
-                                           __dmul_rn(B.val[3 * a + 2], X[2]));
-                U[a] = __dmul_rn(e, fac);
-                v[a] = 0.0;
+                const double e = __dadd_rn(__dadd_rn(__dmul_rn(B.val[3 * a], d.x[i]),
+                                                     __dmul_rn(B.val[3 * a + 1], d.x[N + i])),
+                                           __dmul_rn(B.val[3 * a + 2], d.x[2 * N + i]));
+                U = __dmul_rn(e, fac);
+                v = 0.0;
             }
         }
     }
     const double dt6 = 1.0 / 6.0;
-    for (int a = 0; a < 3; ++a) {
-        const int64_t r = a * N + i;
-        const double k = __dmul_rn(v[a], dts);
-        if (stage == 0) {
-            d.k1[r] = k;
-        } else if (stage == 1) {
-            d.k1[r] = k;
-            d.us[r] = __dadd_rn(__ldcg(d.u1 + r), __dmul_rn(0.5, k));
-        } else if (stage == 2) {
-            d.k2[r] = k;
-            d.us[r] = __dadd_rn(__ldcg(d.u1 + r), __dmul_rn(0.5, k));
-        } else if (stage == 3) {
-            d.us[r] = __dadd_rn(__ldcg(d.u1 + r), k);
-            d.k32[r] = __dadd_rn(k, __ldcg(d.k2 + r));
+    const double k = __dmul_rn(v, dts);
+    double us = 0.0;
+    if (stage == 0) {
+        d.k1[r] = k;
+    } else if (stage == 1) {
+        d.k1[r] = k;
+        d.us[r] = us = __dadd_rn(__ldcg(d.u1 + r), __dmul_rn(0.5, k));
+    } else if (stage == 2) {
+        d.k2[r] = k;
+        d.us[r] = us = __dadd_rn(__ldcg(d.u1 + r), __dmul_rn(0.5, k));
+    } else if (stage == 3) {
+        d.us[r] = us = __dadd_rn(__ldcg(d.u1 + r), k);
+        d.k32[r] = __dadd_rn(k, __ldcg(d.k2 + r));
+    } else {
+        const double Vold = __ldcg(d.V + r);
+        const double inc = __dmul_rn(dt6, __dadd_rn(__dadd_rn(__ldcg(d.k1 + r), k), __dmul_rn(2.0, __ldcg(d.k32 + r))));
+        if (b >= 0) {
+            U = __dadd_rn(U, inc);
         } else {
-            const double Vold = __ldcg(d.V + r);
-            const double inc =
-                __dmul_rn(dt6, __dadd_rn(__dadd_rn(__ldcg(d.k1 + r), k), __dmul_rn(2.0, __ldcg(d.k32 + r))));
-            if (b >= 0) {
-                U[a] = __dadd_rn(U[a], inc);
-            } else {
-                const double damp = __ddiv_rn(__dmul_rn(__dmul_rn(__dmul_rn(dt, d.damping), Vold), dt), rho);
-                U[a] = __dsub_rn(__dadd_rn(U[a], inc), damp);
-            }
-            v[a] = __dadd_rn(v[a], __ddiv_rn(__dmul_rn(__dmul_rn(-d.damping, Vold), dt), rho));
-            d.V[r] = v[a];
-            d.u1[r] = U[a];
-            d.us[r] = U[a];
+            const double damp = __ddiv_rn(__dmul_rn(__dmul_rn(__dmul_rn(dt, d.damping), Vold), dt), rho);
+            U = __dsub_rn(__dadd_rn(U, inc), damp);
         }
-        d.vbuf[r] = v[a];
-        d.U[r] = U[a];
+        v = __dadd_rn(v, __ddiv_rn(__dmul_rn(__dmul_rn(-d.damping, Vold), dt), rho));
+        d.V[r] = v;
+        d.u1[r] = U;
+        d.us[r] = us = U;
     }
-    if (ENERGY && stage == 4) {
-        const double velsq = __dadd_rn(__dadd_rn(__dmul_rn(v[0], v[0]), __dmul_rn(v[1], v[1])), __dmul_rn(v[2], v[2]));
-        d.red[i] = __dmul_rn(__dmul_rn(__dmul_rn(0.5, rho), velsq), d.vol);
-        d.red[N + i] = __dmul_rn(d.vol, __ldcg(d.eed + i));
-    }
+    if (!HELD || changes) d.vbuf[r] = v;
+    if (changes) d.U[r] = U;
+    eff = b >= 0 ? U : us;
+    return v;
+}
+
+// The node's kinetic and elastic energy of a step, from its final velocity and
+// energy density, into red[i], red[N+i].
+__device__ __forceinline__ void stage_energy(const Dev& d, int64_t i, double rho, double v0, double v1, double v2,
+                                             double eed) {
+    const double velsq = __dadd_rn(__dadd_rn(__dmul_rn(v0, v0), __dmul_rn(v1, v1)), __dmul_rn(v2, v2));
+    d.red[i] = __dmul_rn(__dmul_rn(__dmul_rn(0.5, rho), velsq), d.vol);
+    d.red[d.n + i] = __dmul_rn(d.vol, eed);
+}
+
+// All of node i at the end of a stage; with ENERGY, stage 4 leaves its energies.
+template <bool ENERGY>
+__device__ __forceinline__ void stage_epilogue(const Dev& d, int64_t i, int stage, double dts, double dt, double t) {
+    const int64_t N = d.n;
+    const double rho = d.mats[d.mat[i]].density;
+    double v[3], eff;
+    for (int a = 0; a < 3; ++a)
+        v[a] = stage_axis<true>(d, i, a, stage, dts, dt, t, rho, __ldcg(d.vbuf + a * N + i), eff);
+    if (ENERGY && stage == 4) stage_energy(d, i, rho, v[0], v[1], v[2], __ldcg(d.eed + i));
 }
 
 }  // namespace pd
