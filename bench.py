@@ -954,9 +954,9 @@ def run_ours(args):
     # the kernels the tuner kept
     sten = bool(tune.get("force_stencil"))
     force_kernel = ("k_force_f32c_sten" if sten else "k_force_f32c_quad" if tune.get("force_quad")
-                    else "k_force_f32c_tiled" if tune.get("force_tile") else "k_force_f32c_pair")
+                    else "k_force_f32c_tiled" if tune.get("force_tile") else "k_force_f32c_lanes")
     pat, sell = bool(tune.get("gather_stencil")), bool(tune.get("gather_sell"))
-    gather_kernel = "k_gather_f32c_ring" if (pat and sell) else "k_gather_f32c"
+    gather_kernel = "k_gather_f32c_ring" if (pat and sell) else "k_gather_f32c_lanes"
     # coefficients, contributor ids (pattern ids instead with patterns), trial
     # displacement, output blocks, partition-of-unity sums, row pointers
     gather_bytes = (ncb * npt * 4 + (n * 4 if pat else ncb * 4 + (n + 1) * 8) + n * 8 * 4 + n * npt * 12

@@ -186,6 +186,15 @@ int dalloc(pd_ctx* c, T** p, size_t count) {
     return PD_OK;
 }
 
+// for a buffer that can be done without: null when there is no room
+template <typename T>
+bool try_dalloc(pd_ctx* c, T** p, size_t count) {
+    if (dalloc(c, p, count) == PD_OK) return true;
+    *p = nullptr;
+    cudaGetLastError();  // answered here
+    return false;
+}
+
 void dfree(pd_ctx* c, void* p) {
     if (!p) return;
     auto it = std::find(c->owned.begin(), c->owned.end(), p);
@@ -487,7 +496,7 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
         (rc = dalloc(c, &red, 2 * N + 4 + 2 * 160)) || (rc = dalloc(c, &tdev, 1)) ||
         (rc = dalloc(c, &c->dotpart, 2 * (N + 4096))) || (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
         return bail(rc);
-    if (d.cci && (rc = dalloc(c, &c->ue, 2 * n3)) != PD_OK) return bail(rc);
+    if (d.cci) try_dalloc(c, &c->ue, 2 * n3);  // without it the epilogues run apart
     if (c->nslit) {
         double* sl = nullptr;
         if ((rc = dalloc(c, &sl, 6 * c->nslit)) != PD_OK) return bail(rc);
@@ -2650,23 +2659,26 @@ extern "C" int pd_adjoint_forward(pd_ctx* c, double dt, double t0, int nsteps, i
     return rc;
 }
 
-// Reverse sweep of the last pd_adjoint_forward.  lam_U, lam_V: adjoints of
-// the final U and V ([3N] host, V may be NULL); grad_f [N] receives the
-// gradient with respect to the per-node spring factors.  Leaves the state
-// at the start of the forward run.
-// The mirror entries for the one-evaluation VJP, once per family.
+// The mirror entries for the one-evaluation VJP, once per family; where there
+// is no room for them the points are evaluated twice.
 namespace {
-int mirror_prepare(pd_ctx* c) {
-    if (c->adj_mirror_gen == c->family_gen) return PD_OK;
+void mirror_free(pd_ctx* c) {
     dfree(c, c->adj_mirror);
     dfree(c, c->adj_bond);
     c->adj_mirror = nullptr;
     c->adj_bond = nullptr;
     c->adj_symmetric = false;
+}
+
+int mirror_prepare(pd_ctx* c) {
+    if (c->adj_mirror_gen == c->family_gen) return PD_OK;
+    mirror_free(c);
     c->adj_mirror_gen = c->family_gen;
     if (c->npt != 8 || c->Ha == 0) return PD_OK;
-    PD_TRY(dalloc(c, &c->adj_mirror, c->Ha));
-    if (dalloc(c, &c->adj_bond, c->Ha) != PD_OK) return PD_OK;  // no room: two evaluations
+    if (!try_dalloc(c, &c->adj_mirror, c->Ha) || !try_dalloc(c, &c->adj_bond, c->Ha)) {
+        mirror_free(c);
+        return PD_OK;
+    }
     PD_CUDA_TRY(cudaMemsetAsync(c->dflag, 0, sizeof(int), c->stream));
     pd::launch_mirror(c->d, c->adj_mirror, c->dflag, c->stream);
     int bad = 1;
@@ -2677,6 +2689,10 @@ int mirror_prepare(pd_ctx* c) {
 }
 }  // namespace
 
+// Reverse sweep of the last pd_adjoint_forward.  lam_U, lam_V: adjoints of
+// the final U and V ([3N] host, V may be NULL); grad_f [N] receives the
+// gradient with respect to the per-node spring factors.  Leaves the state
+// at the start of the forward run.
 extern "C" int pd_adjoint_backward(pd_ctx* c, const double* lam_U, const double* lam_V, double* grad_f) {
     if (!c || !lam_U || !grad_f) return fail(PD_ERR_ARG, "pd_adjoint_backward: null argument");
     if (c->adj_steps < 1) return fail(PD_ERR_ARG, "pd_adjoint_backward: no forward run to reverse");
@@ -2694,8 +2710,11 @@ extern "C" int pd_adjoint_backward(pd_ctx* c, const double* lam_U, const double*
         dfree(c, c->adj_pool);
         c->adj_pool = nullptr;
         c->adj_pool_count = 0;
-        if (dalloc(c, &c->adj_pool, pool_need) != PD_OK)
-            return fail(PD_ERR_OOM, "pd_adjoint_backward: device memory for the tape");
+        if (!try_dalloc(c, &c->adj_pool, pool_need)) {
+            mirror_free(c);
+            if (!try_dalloc(c, &c->adj_pool, pool_need))
+                return fail(PD_ERR_OOM, "pd_adjoint_backward: device memory for the tape");
+        }
         c->adj_pool_count = pool_need;
     }
     int64_t carved = 0;
