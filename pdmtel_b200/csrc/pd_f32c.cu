@@ -1073,104 +1073,36 @@ __global__ void k_family_radius(Dev d, int* out) {
     atomicMax(out, r);
 }
 
-// The same for any number of Gauss points (constants from shared memory).
-template <bool SFAC>
-__global__ void __launch_bounds__(128) k_force_f32c_any(Dev d, double dts) {
-    __shared__ PointF sp[kMaxPoints];
-    for (int g = threadIdx.x; g < d.npt; g += blockDim.x) {
-        const GaussConst& Q = d.gc[g];
-        sp[g] = PointF{Q.hgf[0], Q.hgf[1], Q.hgf[2], Q.Wf, Q.A, Q.B};
-    }
-    __syncthreads();
-    const int64_t N = d.n;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (tid >= N) return;
-    const int64_t i = d.order[tid];
-    const int npt = d.npt, bs = d.bs;
-    const double* src = d.bc[i] >= 0 ? d.U : d.us;
-    const double u0 = src[i], u1 = src[N + i], u2 = src[2 * N + i];
-    const float uh0 = (float)u0, uh1 = (float)u1, uh2 = (float)u2;
-    const float ul0 = (float)(u0 - (double)uh0), ul1 = (float)(u1 - (double)uh1), ul2 = (float)(u2 - (double)uh2);
-    const float* si = d.sblk + 8 * i;
-    const int mi = d.mat[i];
-    const MatDev& Mi = d.mats[mi];
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, k0 = 0.f, k1 = 0.f, k2 = 0.f;
-    const int64_t pb = d.arow[i], pe = d.arow[i + 1];
-    for (int64_t p = pb; p < pe; ++p) {
-        const int64_t j = d.acol[p];
-        const float* bj = d.nblk + j * bs;
-        const float* sj = d.sblk + 8 * j;
-        const float dx0 = (sj[0] - si[0]) + (sj[3] - si[3]);
-        const float dx1 = (sj[1] - si[1]) + (sj[4] - si[4]);
-        const float dx2 = (sj[2] - si[2]) + (sj[5] - si[5]);
-        const float* uj = bj + 3 * npt;
-        const float du0 = (uj[0] - uh0) + (uj[3] - ul0);
-        const float du1 = (uj[1] - uh1) + (uj[4] - ul1);
-        const float du2 = (uj[2] - uh2) + (uj[5] - ul2);
-        const MatDev& Mj = d.mats[d.mat[j]];
-        const float ecrit = (float)fmin(Mi.ecrit, Mj.ecrit);
-        float coef = 0.5f * (si[6] + sj[6]) * (float)fmin(Mi.spring, Mj.spring);
-        if (SFAC) coef *= 0.5f * (si[7] + sj[7]);
-        float F0 = 0.f, F1 = 0.f, F2 = 0.f;
-        for (int g = 0; g < npt; ++g) {
-            const PointF& P = sp[g];
-            const float x0 = dx0 + P.hx, x1 = dx1 + P.hy, x2 = dx2 + P.hz;
-            const float e0 = du0 + bj[g], e1 = du1 + bj[npt + g], e2 = du2 + bj[2 * npt + g];
-            const float y0 = x0 + e0, y1 = x1 + e1, y2 = x2 + e2;
-            const float r2 = fmaf(x0, x0, fmaf(x1, x1, x2 * x2));
-            const float dd = fmaf(e0, x0 + y0, fmaf(e1, x1 + y1, e2 * (x2 + y2)));
-            const float p2 = r2 + dd;
-            const float rinv = rsqrtf(r2), pinv = rsqrtf(p2);
-            const float r = r2 * rinv;
-            const float s = dd * rinv * __fdividef(1.0f, fmaf(p2, pinv, r));
-            const float beta = __saturatef((P.A - r) * P.B);
-            float fm = P.W * beta * s * pinv;
-            if (dd > 0.f && s > ecrit) fm = 0.f;
-            F0 = fmaf(fm, y0, F0);
-            F1 = fmaf(fm, y1, F1);
-            F2 = fmaf(fm, y2, F2);
-        }
-        F0 *= coef; F1 *= coef; F2 *= coef;
-        float y = F0 - k0, t = s0 + y; k0 = (t - s0) - y; s0 = t;
-        y = F1 - k1; t = s1 + y; k1 = (t - s1) - y; s1 = t;
-        y = F2 - k2; t = s2 + y; k2 = (t - s2) - y; s2 = t;
-    }
-    const double rho = Mi.density, nb = (double)(pe - pb);
-    d.vbuf[i] += ((double)s0 - (double)k0 + nb * (Mi.grav[0] * rho)) * dts / rho;
-    d.vbuf[N + i] += ((double)s1 - (double)k1 + nb * (Mi.grav[1] * rho)) * dts / rho;
-    d.vbuf[2 * N + i] += ((double)s2 - (double)k2 + nb * (Mi.grav[2] * rho)) * dts / rho;
-}
+// Any number of Gauss points (constants in shared memory), and the one-point
+// scheme (pdDataManager.cpp:1818-1866), whose nodes' effective displacements (U
+// for nodes with a boundary condition, us otherwise) k_pack_cci leaves as hi/lo.
+// The node's side of a bond.
+struct OwnAny {
+    float x[6], u[6], bE, sf;
+    const MatDev* M;
+};
 
-// CCI in FP32 form: one point at node j, pdDataManager.cpp:1818-1866.  The
-// effective displacement of every node (U for nodes with a boundary
-// condition, us otherwise) is packed as hi/lo by k_pack_cci.
-template <bool SFAC>
-__global__ void __launch_bounds__(128) k_force_f32c_cci(Dev d, double dts) {
-    const int64_t N = d.n;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (tid >= N) return;
-    const int64_t i = d.order[tid];
-    const float* si = d.sblk + 8 * i;
-    const float* ui = d.nblk + i * d.bs;
-    const MatDev& Mi = d.mats[d.mat[i]];
-    const float dl = (float)d.delta, h = (float)d.dx;
-    const float outer = d.cci_mdf ? dl + 0.5f * h : dl;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, k0 = 0.f, k1 = 0.f, k2 = 0.f;
-    const int64_t pb = d.arow[i], pe = d.arow[i + 1];
-    for (int64_t p = pb; p < pe; ++p) {
-        const int64_t j = d.acol[p];
-        const float* sj = d.sblk + 8 * j;
-        const float* uj = d.nblk + j * d.bs;
-        const float x0 = (sj[0] - si[0]) + (sj[3] - si[3]);
-        const float x1 = (sj[1] - si[1]) + (sj[4] - si[4]);
-        const float x2 = (sj[2] - si[2]) + (sj[5] - si[5]);
-        const float e0 = (uj[0] - ui[0]) + (uj[3] - ui[3]);
-        const float e1 = (uj[1] - ui[1]) + (uj[4] - ui[4]);
-        const float e2 = (uj[2] - ui[2]) + (uj[5] - ui[5]);
-        const MatDev& Mj = d.mats[d.mat[j]];
-        const float ecrit = (float)fmin(Mi.ecrit, Mj.ecrit);
-        float coef = 0.5f * (si[6] + sj[6]) * (float)fmin(Mi.spring, Mj.spring) * (float)d.vol_cci;
-        if (SFAC) coef *= 0.5f * (si[7] + sj[7]);
+// Bond (i, j): its force is m f.
+template <bool SFAC, bool CCI>
+__device__ __forceinline__ void bond_any(const Dev& d, const PointF* sp, const OwnAny& O, float outer, int64_t j,
+                                         float (&f)[3], float& m) {
+    const int npt = d.npt;
+    const float4 sa = __ldg(reinterpret_cast<const float4*>(d.sblk + 8 * j));
+    const float4 sb = __ldg(reinterpret_cast<const float4*>(d.sblk + 8 * j) + 1);
+    const float* bj = d.nblk + j * d.bs;
+    const float dx0 = (sa.x - O.x[0]) + (sa.w - O.x[3]);
+    const float dx1 = (sa.y - O.x[1]) + (sb.x - O.x[4]);
+    const float dx2 = (sa.z - O.x[2]) + (sb.y - O.x[5]);
+    const float* uj = CCI ? bj : bj + 3 * npt;
+    const float du0 = (uj[0] - O.u[0]) + (uj[3] - O.u[3]);
+    const float du1 = (uj[1] - O.u[1]) + (uj[4] - O.u[4]);
+    const float du2 = (uj[2] - O.u[2]) + (uj[5] - O.u[5]);
+    const MatDev& Mj = d.mats[d.mat[j]];
+    const float ecrit = (float)fmin(O.M->ecrit, Mj.ecrit);
+    float coef = 0.5f * (O.bE + sb.z) * (float)fmin(O.M->spring, Mj.spring);
+    if (CCI) coef *= (float)d.vol_cci;
+    if (SFAC) coef *= 0.5f * (O.sf + sb.w);
+    auto point = [&](float x0, float x1, float x2, float e0, float e1, float e2, auto&& term) {
         const float y0 = x0 + e0, y1 = x1 + e1, y2 = x2 + e2;
         const float r2 = fmaf(x0, x0, fmaf(x1, x1, x2 * x2));
         const float dd = fmaf(e0, x0 + y0, fmaf(e1, x1 + y1, e2 * (x2 + y2)));
@@ -1178,18 +1110,102 @@ __global__ void __launch_bounds__(128) k_force_f32c_cci(Dev d, double dts) {
         const float rinv = rsqrtf(r2), pinv = rsqrtf(p2);
         const float r = r2 * rinv;
         const float s = dd * rinv * __fdividef(1.0f, fmaf(p2, pinv, r));
-        const float beta = (r > outer) ? 0.f : __saturatef((dl + 0.5f * h - r) / h);
-        float fm = coef * beta * s * pinv;
-        if (dd > 0.f && s > ecrit) fm = 0.f;
-        const float F0 = fm * y0, F1 = fm * y1, F2 = fm * y2;
-        float y = F0 - k0, t = s0 + y; k0 = (t - s0) - y; s0 = t;
-        y = F1 - k1; t = s1 + y; k1 = (t - s1) - y; s1 = t;
-        y = F2 - k2; t = s2 + y; k2 = (t - s2) - y; s2 = t;
+        term(y0, y1, y2, r, s, pinv, dd > 0.f && s > ecrit);
+    };
+    if (CCI) {
+        const float dl = (float)d.delta, h = (float)d.dx;
+        point(dx0, dx1, dx2, du0, du1, du2, [&](float y0, float y1, float y2, float r, float s, float pinv, bool cut) {
+            const float beta = (r > outer) ? 0.f : __saturatef((dl + 0.5f * h - r) / h);
+            m = cut ? 0.f : coef * beta * s * pinv;
+            f[0] = y0, f[1] = y1, f[2] = y2;
+        });
+    } else {
+        f[0] = f[1] = f[2] = 0.f;
+        for (int g = 0; g < npt; ++g) {
+            const PointF& P = sp[g];
+            point(dx0 + P.hx, dx1 + P.hy, dx2 + P.hz, du0 + bj[g], du1 + bj[npt + g], du2 + bj[2 * npt + g],
+                  [&](float y0, float y1, float y2, float r, float s, float pinv, bool cut) {
+                      const float beta = __saturatef((P.A - r) * P.B);
+                      const float fm = cut ? 0.f : P.W * beta * s * pinv;
+                      f[0] = fmaf(fm, y0, f[0]);
+                      f[1] = fmaf(fm, y1, f[1]);
+                      f[2] = fmaf(fm, y2, f[2]);
+                  });
+        }
+        m = coef;
     }
-    const double rho = Mi.density, nb = (double)(pe - pb);
-    d.vbuf[i] += ((double)s0 - (double)k0 + nb * (Mi.grav[0] * rho)) * dts / rho;
-    d.vbuf[N + i] += ((double)s1 - (double)k1 + nb * (Mi.grav[1] * rho)) * dts / rho;
-    d.vbuf[2 * N + i] += ((double)s2 - (double)k2 + nb * (Mi.grav[2] * rho)) * dts / rho;
+}
+
+// L lanes per node, a bond each; lanes 0..2 add the round's bonds to the
+// compensated family sums in ascending order (m f fused into the first
+// subtraction) and take the stage's epilogue along (stage 1..4).
+// Bound by issue at size and by the latency of a node's rounds below.  Per
+// launch against one thread per node walking its family: one point 1,000 nodes
+// 143 -> 22 us, 26,000 190 -> 71, 100,000 370 -> 220, 400,000 1368 -> 695;
+// 27 points 1,000 nodes 1125 -> 54 us, 40,000 1211 -> 556.
+template <bool SFAC, bool CCI, int L>
+__global__ void __launch_bounds__(128) k_force_f32c_any(Dev d, double dts, int stage, double dt) {
+    __shared__ PointF sp[CCI ? 1 : kMaxPoints];
+    __shared__ float4 terms[128 / L][L + 1];  // the groups' terms read together lie in different banks
+    if (!CCI) {
+        for (int g = threadIdx.x; g < d.npt; g += blockDim.x) {
+            const GaussConst& Q = d.gc[g];
+            sp[g] = PointF{Q.hgf[0], Q.hgf[1], Q.hgf[2], Q.Wf, Q.A, Q.B};
+        }
+        __syncthreads();
+    }
+    const int64_t N = d.n;
+    const int ql = threadIdx.x % L;
+    const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
+    const bool live = slot < N;
+    const int64_t i = d.order[live ? slot : 0];
+    OwnAny O;
+    O.M = d.mats + d.mat[i];
+    for (int k = 0; k < 6; ++k) O.x[k] = d.sblk[8 * i + k];
+    O.bE = d.sblk[8 * i + 6];
+    O.sf = d.sblk[8 * i + 7];
+    if (CCI) {
+        for (int k = 0; k < 6; ++k) O.u[k] = d.nblk[i * d.bs + k];
+    } else {
+        const double* src = d.bc[i] >= 0 ? d.U : d.us;
+        for (int a = 0; a < 3; ++a) {
+            const double u = src[a * N + i];
+            O.u[a] = (float)u;
+            O.u[3 + a] = (float)(u - (double)O.u[a]);
+        }
+    }
+    const float dl = (float)d.delta, outer = d.cci_mdf ? dl + 0.5f * (float)d.dx : dl;
+    const int64_t pb = d.arow[i];
+    const int cnt = live ? (int)(d.arow[i + 1] - pb) : 0;
+    float4* own = terms[threadIdx.x / L];
+    float sum = 0.f, comp = 0.f;
+    for (int base = 0; __any_sync(0xffffffffu, base < cnt); base += L) {
+        if (base + ql < cnt) {
+            float f[3], m;
+            bond_any<SFAC, CCI>(d, sp, O, outer, d.acol[pb + base + ql], f, m);
+            own[ql] = make_float4(f[0], f[1], f[2], m);
+        }
+        __syncwarp();
+        if (ql < 3) {
+            const float* t4 = reinterpret_cast<const float*>(own);
+#pragma unroll 8
+            for (int q = 0; q < L; ++q) {
+                if (base + q >= cnt) continue;
+                const float y = fmaf(t4[4 * q + ql], t4[4 * q + 3], -comp), t = sum + y;
+                comp = (t - sum) - y;
+                sum = t;
+            }
+        }
+        __syncwarp();
+    }
+    if (live && ql < 3) {
+        const double rho = O.M->density;
+        const double v0 = d.vbuf[ql * N + i];
+        const double v = v0 + ((double)sum - (double)comp + (double)cnt * (O.M->grav[ql] * rho)) * dts / rho;
+        double eff;
+        if (stage > 0) stage_axis<false>(d, i, ql, stage, dts, dt, *d.tdev, rho, v, eff);
+        else d.vbuf[ql * N + i] = v;
+    }
 }
 
 __global__ void k_pack_cci(Dev d) {
@@ -1833,15 +1849,28 @@ inline int force_lanes(const Dev& d) { return d.n < 12288 ? 32 : (d.n < 131072 ?
 // against 298, a batch of 97,000 375 against 432).
 constexpr int64_t kStencilFrom = 65536;
 
+template <bool CCI>
+void launch_any(const Dev& d, double dts, cudaStream_t s, int stage, double dt) {
+    const int lanes = force_lanes(d);
+    const unsigned nb = blocks_for(lanes * d.n, 128);
+    auto go = [&](auto sf) {
+        constexpr bool SF = decltype(sf)::value;
+        if (lanes == 32) k_force_f32c_any<SF, CCI, 32><<<nb, 128, 0, s>>>(d, dts, stage, dt);
+        else if (lanes == 8) k_force_f32c_any<SF, CCI, 8><<<nb, 128, 0, s>>>(d, dts, stage, dt);
+        else k_force_f32c_any<SF, CCI, 4><<<nb, 128, 0, s>>>(d, dts, stage, dt);
+    };
+    if (d.sfac) go(std::true_type{});
+    else go(std::false_type{});
+}
+
 bool launch_force_f32c(const Dev& d, double dts, cudaStream_t s, int stage, double dt) {
     if (d.n == 0) return true;
     if (d.energy) stage = -1;  // the energies are the epilogue kernel's
     const unsigned nb = blocks_for(d.n, 128);
     if (d.cci) {
         k_pack_cci<<<blocks_for(d.n, 256), 256, 0, s>>>(d);
-        if (d.sfac) k_force_f32c_cci<true><<<nb, 128, 0, s>>>(d, dts);
-        else k_force_f32c_cci<false><<<nb, 128, 0, s>>>(d, dts);
-        return false;
+        launch_any<true>(d, dts, s, stage, dt);
+        return stage > 0;
     }
     const int lanes = force_lanes(d);
     const unsigned nbl = blocks_for(lanes * d.n, 128);
@@ -1935,9 +1964,8 @@ bool launch_force_f32c(const Dev& d, double dts, cudaStream_t s, int stage, doub
 #undef PD_F32
         return stage > 0;
     }
-    if (d.sfac) k_force_f32c_any<true><<<nb, 128, 0, s>>>(d, dts);
-    else k_force_f32c_any<false><<<nb, 128, 0, s>>>(d, dts);
-    return false;
+    launch_any<false>(d, dts, s, stage, dt);
+    return stage > 0;
 }
 
 // The persistent kernel's variant for the problem, and how many of its
