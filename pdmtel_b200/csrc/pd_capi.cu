@@ -3072,6 +3072,14 @@ extern "C" int pd_autotune(pd_ctx* c, double dt, int steps, pd_tune_result* out)
         }
         if ((rc = pd_set_option(c, PD_OPT_FORCE_STENCIL, best.ms < before ? keep : f0)) != PD_OK) return done(rc);
         out->force_stencil = c->fst_shape;
+        // the tiles were timed with another force; the stencil force has its own
+        // order, so the gather's is left to choose (the 640,000-node plate: 0.474
+        // ms per gather in the tiles best for k_force_f32c_lanes, 0.434 so)
+        if (c->fst_shape)
+            for (int64_t tl : tiles)
+                if (tl != best.tile &&
+                    (rc = trial({tl, 0, c->persist_per_sm, c->force_chunk, c->gather_chunk, 0.0})) != PD_OK)
+                    return done(rc);
     }
     if (c->precision == PD_PREC_FP32C && !c->d.cci && c->npt == 8 && c->d.lat && !c->d.hasfail &&
         !c->d.multimat && !c->fst_shape) {
