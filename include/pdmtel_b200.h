@@ -357,8 +357,10 @@ int pd_static_rhs(pd_ctx* ctx, double time, double* b);
  * PD_PREC_FP32C: the iterations' matvec in FP32 (FP64 vectors, dot products
  * and node sums), refined in FP64 by replacing the residual with the true
  * b - K x whenever it has fallen 100-fold and at convergence ("reliable
- * updates"); convergence is judged on the FP64 true residual.  x [3N] is the
- * initial guess in and the solution out.  iters/relres may be NULL. */
+ * updates"); convergence is judged on the FP64 true residual.  On a cracked
+ * lattice stencil (PD_OPT_STATIC_STENCIL) the FP32C iterations' matvec is the
+ * FP64 one.  x [3N] is the initial guess in and the solution out.
+ * iters/relres may be NULL. */
 int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int maxit, double* x, int* iters,
                     double* relres);
 
@@ -377,8 +379,8 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  *   the queue at a time (multiples of 128; defaults 128 and 256).
  * PD_OPT_STATIC_STENCIL: 1 (default) lets the static operator run as a
  *   lattice stencil when the problem is a complete box with one material and
- *   stencil-shaped families (checked; broken bonds are subtracted from a list
- *   of their own); 0 keeps the family-list kernel.
+ *   stencil-shaped families (checked; the rows of nodes with broken bonds are
+ *   formed from lists of their unbroken ones); 0 keeps the family-list kernel.
  * PD_OPT_GATHER_PER_POINT: 1 runs the FP32-form MLS gather with one thread
  *   per (node, Gauss point), 0 (default) with one per four points.
  * PD_OPT_FORCE_TILE: the FP32-form force (2x2x2 points, nodes on one

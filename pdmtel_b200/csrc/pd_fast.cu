@@ -299,9 +299,10 @@ __global__ void k_box_slots(const int4* __restrict__ list, int nlist, int* __res
 __global__ void k_broken_counts(Dev d, int64_t* __restrict__ flag, int64_t* __restrict__ cnt) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= d.n) return;
-    const int64_t c = (d.frow[i + 1] - d.frow[i]) - (d.arow[i + 1] - d.arow[i]);
-    cnt[i] = c;
-    flag[i] = c > 0;
+    const int64_t whole = d.arow[i + 1] - d.arow[i];
+    const bool broken = d.frow[i + 1] - d.frow[i] > whole;
+    cnt[i] = broken ? whole : 0;
+    flag[i] = broken;
 }
 
 __global__ void k_broken_fill(Dev d, const int* __restrict__ map, const int64_t* __restrict__ flag,
@@ -319,21 +320,26 @@ __global__ void k_broken_fill(Dev d, const int* __restrict__ map, const int64_t*
     bnode[k] = (int32_t)i;
     int64_t o = cpos[i];
     bptr[k] = o;
-    for (int64_t p = d.frow[i]; p < d.frow[i + 1]; ++p)
-        if (d.fbroken[p]) bent[o++] = make_int2(d.fcol[p], map[box_key(d.lat[i], d.lat[d.fcol[p]])]);
+    for (int64_t p = d.arow[i]; p < d.arow[i + 1]; ++p)
+        bent[o++] = make_int2(d.acol[p], map[box_key(d.lat[i], d.lat[d.acol[p]])]);
 }
 
-// What the broken bonds of a node would add to the stencil operator, a warp
-// per node that has some; the operator kernels subtract it.  A cracked box then
-// runs on the stencil, with a list only of what the crack cut: 60x40x12 with a
-// slit, 62 us per matvec on the family lists, 7 us here and about 15 in
-// k_static_nd.
-template <typename T, bool SFAC>
-__global__ void __launch_bounds__(128) k_static_broken(Dev d, StencilDev S, const T* __restrict__ xm) {
+// The rows of the nodes with broken bonds from their unbroken entries, a warp
+// per node; the operator kernels store them in place of their own.  A cracked
+// box then runs on the stencil, with lists only where the crack cut: 60x40x12
+// with a slit, 62 us per matvec on the family lists, 7 us here and about 15 in
+// k_static_nd; the solve 4.43 -> 4.31 ms, 96x96x96 90 -> 95 ms, against
+// subtracting the broken entries from the whole stencil.  (That difference is
+// rounding noise where a node, or one direction of it, has no stiffness left;
+// the preconditioner weights the noise by 17 orders of magnitude and the solve
+// does not converge.)  Entries in a list: read from acol through the lattice
+// positions and an offset table the same solve took 4.54 ms.
+template <bool SFAC>
+__global__ void __launch_bounds__(128) k_static_rows(Dev d, StencilDev S, const double* __restrict__ xm) {
     const int k = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (k >= S.nbrk) return;
     const int64_t N = d.n, i = S.bnode[k];
-    const T x0 = xm[i], x1 = xm[N + i], x2 = xm[2 * N + i];
+    const double x0 = xm[i], x1 = xm[N + i], x2 = xm[2 * N + i];
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
     for (int64_t p = S.bptr[k] + lane; p < S.bptr[k + 1]; p += 32) {
         const int2 e = S.bent[p];
@@ -341,26 +347,25 @@ __global__ void __launch_bounds__(128) k_static_broken(Dev d, StencilDev S, cons
         const double4 g = S.geo[e.y];
         double w = g.w;
         if (SFAC) w = w * (0.5 * (d.sfac[i] + d.sfac[j]));
-        const T f0 = (T)g.x, f1 = (T)g.y, f2 = (T)g.z;
-        const T pr = (T)w * (f0 * (x0 - xm[j]) + f1 * (x1 - xm[N + j]) + f2 * (x2 - xm[2 * N + j]));
-        a0 += (double)(pr * f0);
-        a1 += (double)(pr * f1);
-        a2 += (double)(pr * f2);
+        const double pr = w * (g.x * (x0 - xm[j]) + g.y * (x1 - xm[N + j]) + g.z * (x2 - xm[2 * N + j]));
+        a0 += pr * g.x;
+        a1 += pr * g.y;
+        a2 += pr * g.z;
     }
     for (int o = 16; o > 0; o >>= 1) {
         a0 += __shfl_xor_sync(0xffffffffu, a0, o);
         a1 += __shfl_xor_sync(0xffffffffu, a1, o);
         a2 += __shfl_xor_sync(0xffffffffu, a2, o);
     }
-    if (lane < 3) S.bfix[3 * (int64_t)k + lane] = lane == 0 ? a0 : (lane == 1 ? a1 : a2);
+    if (lane < 3) S.brow[3 * (int64_t)k + lane] = lane == 0 ? a0 : (lane == 1 ? a1 : a2);
 }
-__device__ __forceinline__ void less_broken(const StencilDev& S, int64_t i, double& a0, double& a1, double& a2) {
+__device__ __forceinline__ void listed_row(const StencilDev& S, int64_t i, double& a0, double& a1, double& a2) {
     if (S.nbrk == 0) return;
     const int k = S.bidx[i];
     if (k < 0) return;
-    a0 -= S.bfix[3 * (int64_t)k];
-    a1 -= S.bfix[3 * (int64_t)k + 1];
-    a2 -= S.bfix[3 * (int64_t)k + 2];
+    a0 = S.brow[3 * (int64_t)k];
+    a1 = S.brow[3 * (int64_t)k + 1];
+    a2 = S.brow[3 * (int64_t)k + 2];
 }
 
 // FP64: bond terms and sums in FP64.  FP32: bond terms in FP32 from an FP32
@@ -449,7 +454,7 @@ __global__ void __launch_bounds__(256) k_static_stencil(Dev d, StencilDev S, con
     const bool inner = ix >= R && ix < S.nx - R && iy >= R && iy < S.ny - R && iz >= R && iz < S.nz - R;
     if (inner) stencil_sum<T, SFAC, false>(d, S, sgeo, sgeof, soff, i, ix, iy, iz, xm, sfi, a0, a1, a2);
     else stencil_sum<T, SFAC, true>(d, S, sgeo, sgeof, soff, i, ix, iy, iz, xm, sfi, a0, a1, a2);
-    less_broken(S, i, a0, a1, a2);
+    listed_row(S, i, a0, a1, a2);
     y[i] = (mi & 1) ? x[i] : a0;
     y[N + i] = (mi & 2) ? x[N + i] : a1;
     y[2 * N + i] = (mi & 4) ? x[2 * N + i] : a2;
@@ -599,7 +604,7 @@ __global__ void __launch_bounds__(128) k_static_zcol(Dev d, StencilDev S, const 
     for (int m = 0; m < R; ++m) {
         if (!in_xy || iz0 + m >= S.nz) continue;
         const int64_t i = i0 + m * nxy;
-        less_broken(S, i, acc[m][0], acc[m][1], acc[m][2]);
+        listed_row(S, i, acc[m][0], acc[m][1], acc[m][2]);
         const unsigned mi = S.pmask[i];
         y[i] = (mi & 1) ? x[i] : acc[m][0];
         y[N + i] = (mi & 2) ? x[N + i] : acc[m][1];
@@ -792,7 +797,7 @@ __global__ void __launch_bounds__(256) k_static_nd(Dev d, StencilDev S, const __
             double v[3] = {fma(B[0], u0, fma(B[3], u1, fma(B[4], u2, acc[m][0]))),
                            fma(B[3], u0, fma(B[1], u1, fma(B[5], u2, acc[m][1]))),
                            fma(B[4], u0, fma(B[5], u1, fma(B[2], u2, acc[m][2])))};
-            less_broken(S, i, v[0], v[1], v[2]);
+            listed_row(S, i, v[0], v[1], v[2]);
             const unsigned mi = S.pmask[i];
             if (mi) {  // prescribed rows: y = x
                 for (int a = 0; a < 3; ++a) {
@@ -1042,11 +1047,6 @@ bool launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const do
     const bool zcol = S.ncol > 0 && S.rz >= 1 && S.rz <= 4;
     if (f32) {
         float* xm = reinterpret_cast<float*>(S.xm);
-        if (S.nbrk) {
-            const unsigned bb = blocks_for(32 * (int64_t)S.nbrk, 128);
-            if (d.sfac) k_static_broken<float, true><<<bb, 128, 0, s>>>(d, S, xm);
-            else k_static_broken<float, false><<<bb, 128, 0, s>>>(d, S, xm);
-        }
         if (zcol) {
             if (d.sfac) launch_zcol<float, true, 8>(d, S, x, xm, y, s);
             else launch_zcol<float, false, 8>(d, S, x, xm, y, s);
@@ -1059,8 +1059,8 @@ bool launch_static_stencil(const Dev& d, const StencilDev& S, bool f32, const do
         double* xm = S.xm;
         if (S.nbrk) {
             const unsigned bb = blocks_for(32 * (int64_t)S.nbrk, 128);
-            if (d.sfac) k_static_broken<double, true><<<bb, 128, 0, s>>>(d, S, xm);
-            else k_static_broken<double, false><<<bb, 128, 0, s>>>(d, S, xm);
+            if (d.sfac) k_static_rows<true><<<bb, 128, 0, s>>>(d, S, xm);
+            else k_static_rows<false><<<bb, 128, 0, s>>>(d, S, xm);
         }
         if (S.ndcol > 0 && S.ndhost && !d.sfac && (S.ndr == 2 || S.ndr == 4 || S.ndr == 8) && nd_halo(S) > 0 &&
             nd_smem(S, S.ndr) <= 226 * 1024) {

@@ -345,16 +345,16 @@ struct StencilDev {
     const double2* ndtap;
     const double* ndiag;
     const struct NdTab* ndhost;  // host copy of the tables, passed as a kernel parameter
-    // broken bonds (a slit): the operator of the whole stencil less bfix, the
-    // broken bonds' share (k_static_broken).  bnode [nbrk] the nodes that have
-    // some, bptr / bent their entries (neighbour, slot of off / geo), bidx [N]
-    // a node's place in bnode or -1, bfix [nbrk][3]
+    // nodes with broken bonds (a slit): their rows, brow [nbrk][3], come from
+    // their unbroken entries (k_static_rows).  bnode [nbrk] these nodes, bptr /
+    // bent their unbroken entries (neighbour, slot of off / geo), bidx [N] a
+    // node's place in bnode or -1
     int nbrk;
     const int32_t* bnode;
     const int64_t* bptr;
     const int2* bent;
     const int32_t* bidx;
-    double* bfix;
+    double* brow;
 };
 // The split form's tables as one kernel parameter (constant bank: warp-uniform
 // reads through the constant cache, no shared-memory traffic).
@@ -372,8 +372,9 @@ void launch_static_pmask(const Dev& d, uint8_t* pm, cudaStream_t s);
 // + nx (y + ny z), an offset is outside or a size differs
 void launch_box_offsets(const Dev& d, int* map, int* err, int4* list, cudaStream_t s);
 void launch_box_check(const Dev& d, const int4* list, int nlist, int* map, int* err, cudaStream_t s);
-// nodes with broken entries: flags and counts per node, and (from their scans)
-// the list that StencilDev::bnode .. bidx describe, map giving the slots
+// nodes with broken entries: flags and unbroken entries per such node, and (from
+// their scans) the list that StencilDev::bnode .. bidx describe, map giving the
+// slots
 void launch_broken_counts(const Dev& d, int64_t* flag, int64_t* cnt, cudaStream_t s);
 void launch_broken_fill(const Dev& d, const int* map, const int64_t* flag, const int64_t* fpos, const int64_t* cpos,
                         int32_t* bnode, int64_t* bptr, int2* bent, int32_t* bidx, cudaStream_t s);
