@@ -120,8 +120,8 @@ __global__ void k_family_prescribed(Dev d, double t, double4* __restrict__ xm) {
 // One thread per node walked its family as a chain of dependent loads, six of
 // them 8-byte gathers, with an IEEE root and division per bond: 198 us for
 // 28,800 nodes (225 blocks, SMs mostly waiting).  A group of lanes takes the
-// bonds side by side, gathers two 32-byte records each, and forms 1/r by the
-// unrounded iteration of pd_rn.cuh: 62 us.
+// bonds side by side, gathers two 32-byte records each, and takes the root and
+// the quotient of pd_rn.cuh: 65 us.
 template <bool SFAC, bool F32, int L>
 __device__ __forceinline__ void family_sum(const Dev& d, const FamilyDev& F, int64_t i, int ql, double4 gi,
                                            double4 xi, double& a0, double& a1, double& a2) {
@@ -145,8 +145,13 @@ __device__ __forceinline__ void family_sum(const Dev& d, const FamilyDev& F, int
             a2 += (double)(pr * f2);
         } else {
             const double r2 = e0 * e0 + e1 * e1 + e2 * e2;
-            const double ri = rn_range(r2) ? rsqrt_near(r2) : 1.0 / sqrt(r2);
-            const double pr = (c * d.vol) * (ri * ri * ri) * (e0 * d0 + e1 * d1 + e2 * d2);
+            const double cv = c * d.vol;
+            double r, y;
+            rn_sqrt_rcp(r2, r, y);
+            const double r3 = r2 * r;
+            double w = rn_div(cv, r3, rn_rcp(r3, y * y * y));
+            if (!(rn_range_cubed(r2) && rn_quotient_ok(cv))) w = cv / (r2 * sqrt(r2));
+            const double pr = w * (e0 * d0 + e1 * d1 + e2 * d2);
             a0 += pr * e0;
             a1 += pr * e1;
             a2 += pr * e2;
@@ -327,7 +332,7 @@ __global__ void k_broken_fill(Dev d, const int* __restrict__ map, const int64_t*
 // The rows of the nodes with broken bonds from their unbroken entries, a warp
 // per node; the operator kernels store them in place of their own.  A cracked
 // box then runs on the stencil, with lists only where the crack cut: 60x40x12
-// with a slit, 62 us per matvec on the family lists, 7 us here and about 15 in
+// with a slit, 65 us per matvec on the family lists, 7 us here and about 15 in
 // k_static_nd; the solve 4.43 -> 4.31 ms, 96x96x96 90 -> 95 ms, against
 // subtracting the broken entries from the whole stencil.  (That difference is
 // rounding noise where a node, or one direction of it, has no stiffness left;

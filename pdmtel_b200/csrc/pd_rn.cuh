@@ -52,6 +52,13 @@ __device__ __forceinline__ void rn_sqrt_rcp(double a, double& s, double& y) {
     y = fma(fma(-s, y, 1.0), y, y);
 }
 
+// y = 1/b rounded to nearest as in rn_sqrt_rcp from an estimate y0 with a
+// relative error below 2^-50; b and 1/b normal
+__device__ __forceinline__ double rn_rcp(double b, double y0) {
+    const double y = __hiloint2double(__double2hiint(y0), __double2loint(y0) | 1);
+    return fma(fma(-b, y, 1.0), y, y);
+}
+
 // 1 / sqrt(a) to about 2^-51 (the iteration above without its last rounding);
 // a in rn_range
 __device__ __forceinline__ double rsqrt_near(double a) {
@@ -79,6 +86,10 @@ __device__ __forceinline__ double rn_div_signed(double a, double b, double y) {
 // whether a positive operand of rn_sqrt_rcp is in [2^-400, 2^400)
 __device__ __forceinline__ bool rn_range(double a) {
     return (unsigned)__double2hiint(a) - (623u << 20) < (800u << 20);
+}
+// the same for [2^-200, 2^200), whose third powers are in range too
+__device__ __forceinline__ bool rn_range_cubed(double a) {
+    return (unsigned)__double2hiint(a) - (823u << 20) < (400u << 20);
 }
 // distance of |a| from the range [2^-500, 2^500) of dividends, as an unsigned
 // number: below rn_span inside; zeros count as inside
