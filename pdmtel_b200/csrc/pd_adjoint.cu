@@ -245,14 +245,6 @@ __global__ void __launch_bounds__(256) k_vjp_partner(Dev d, const double* __rest
     if (live && lane == 0 && d.sfac) gradf[j] += gf;
 }
 
-// 1 / v for v in rn_range, to about 2^-52
-__device__ __forceinline__ double rcp_near(double v) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-    y = fma(fma(-v, y, 1.0), y, y);
-    return fma(fma(-v, y, 1.0), y, y);
-}
-
 // The place of every unbroken family entry's mirror: entry p of node j's row
 // is (j, i), mirror[p] the entry (i, j) of node i's row.  err: set where there
 // is none.
@@ -390,10 +382,10 @@ __global__ void __launch_bounds__(128, 2) k_vjp_bonds(Dev d, const double* __res
             const double r = r2 * rinv, pl = p2 * ip, sum = pl + r;
             // p - r = eta.(2 xi + eta) / (p + r)
             const double q2 = e0 * (x0 + y0) + e1 * (x1 + y1) + e2 * (x2 + y2);
-            const double ext = q2 * rcp_near(sum);
+            const double ext = rn_quotient(q2, sum);
             const double st = ext * rinv;
             const double beta = r <= d.delta - 0.5 * G.dxe ? 1.0
-                                : r <= d.delta + 0.5 * G.dxe ? (d.delta + 0.5 * G.dxe - r) * G.ydxe
+                                : r <= d.delta + 0.5 * G.dxe ? rn_div(d.delta + 0.5 * G.dxe - r, G.dxe, G.ydxe)
                                                              : 0.0;
             const double bw = ext > 0.0 && st > ecrit ? 0.0 : bE * beta * G.W;
             const double a = st * ip;  // 1/r - 1/p

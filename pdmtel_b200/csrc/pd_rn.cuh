@@ -59,16 +59,18 @@ __device__ __forceinline__ double rn_rcp(double b, double y0) {
     return fma(fma(-b, y, 1.0), y, y);
 }
 
-// 1 / sqrt(a) to about 2^-51 (the iteration above without its last rounding);
-// a in rn_range
+// 1 / sqrt(a) within half a unit in the last place and 2^-49 of one, a in
+// rn_range: with e = 1 - a y^2, the root's reciprocal is y (1 + e/2 + 3 e^2/8 +
+// ...); one step of third order from the 20-bit seed, then one of first order
+// whose e has the rounding of a y taken out.
 __device__ __forceinline__ double rsqrt_near(double a) {
-    double y0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
-    double g = a * y0, h = rn_pow2(y0, -1);
-    const double e = fma(-g, h, 0.5);
-    g = fma(g, e, g);
-    h = fma(h, e, h);
-    return rn_pow2(fma(h, fma(-g, h, 0.5), h), 1);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    double e = fma(-(a * y), y, 1.0);
+    y = fma(y * e, fma(0.375, e, 0.5), y);
+    const double g = a * y;
+    e = fma(-fma(a, y, -g), y, fma(-g, y, 1.0));
+    return fma(rn_pow2(y, -1), e, y);
 }
 
 // a / b with y = 1/b, b > 0; a zero or rn_quotient_ok (the quotient of a zero
@@ -77,7 +79,15 @@ __device__ __forceinline__ double rn_div(double a, double b, double y) {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
-// the same with the sign of a zero kept (any quotient has the sign of a)
+// a / b without a reciprocal at hand, b > 0 in rn_range; an a outside
+// rn_quotient_ok may end one unit off
+__device__ __forceinline__ double rn_quotient(double a, double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    return rn_div(a, b, rn_rcp(b, fma(y, fma(e, e, e), y)));
+}
+// the same as rn_div with the sign of a zero kept (any quotient has the sign of a)
 __device__ __forceinline__ double rn_div_signed(double a, double b, double y) {
     const double q = rn_div(a, b, y);
     return __hiloint2double((__double2hiint(q) & 0x7fffffff) | (__double2hiint(a) & 0x80000000), __double2loint(q));
