@@ -752,6 +752,7 @@ __global__ void __launch_bounds__(256) k_mls_contrib(Dev d, const double* __rest
                 c += __popc(m);
             }
             if (c >= 10) break;
+            __syncwarp();  // the wider pass stores over these entries, from other lanes
         }
         if (lane == 0) cbidx[o] = (int32_t)i;
         return;
