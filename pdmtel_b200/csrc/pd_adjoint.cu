@@ -16,9 +16,9 @@
 // With 2x2x2 points every evaluation (i, j, g) serves both: k_vjp_bonds runs
 // over node j's family, sums dJ/dug of j's Gauss points in registers and leaves
 // each bond's share of dJ/du_i and dJ/dc in i's own entry of the bond, which
-// k_vjp_nodes then sums.  Other rules (and families that are not symmetric)
-// evaluate twice: k_vjp_own over node i's family for dJ/du_i, k_vjp_partner
-// over node j's for dJ/dug.
+// k_vjp_nodes then sums.  Other rules (and families that are not symmetric, or
+// list a bond twice) evaluate twice: k_vjp_own over node i's family for
+// dJ/du_i, k_vjp_partner over node j's for dJ/dug.
 #include "pd_internal.cuh"
 #include "pd_rn.cuh"
 
@@ -247,7 +247,8 @@ __global__ void __launch_bounds__(256) k_vjp_partner(Dev d, const double* __rest
 
 // The place of every unbroken family entry's mirror: entry p of node j's row
 // is (j, i), mirror[p] the entry (i, j) of node i's row.  err: set where there
-// is none.
+// is none, and where a row does not ascend (a bond listed twice would share
+// one place).
 __global__ void __launch_bounds__(256) k_mirror(Dev d, int64_t* __restrict__ mirror, int* __restrict__ err) {
     const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (j >= d.n) return;
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(256) k_mirror(Dev d, int64_t* __restrict__ mir
         }
         const bool found = lo <= hi && d.acol[lo] == (int32_t)j;
         mirror[p] = found ? lo : p;
-        if (!found) atomicOr(err, 1);
+        if (!found || (p > d.arow[j] && d.acol[p - 1] >= i)) atomicOr(err, 1);
     }
 }
 

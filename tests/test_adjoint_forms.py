@@ -3,7 +3,7 @@ below 12,288 nodes, eight lanes above) against the one that evaluates it from
 both ends, which a family without some mirror entries takes: two nodes far from
 the specimen carry a bond listed at one end only, which changes nothing on the
 specimen.  Boundary factors, two materials with a critical stretch, lengths
-outside the range of the branch-free roots."""
+outside the range of the branch-free roots, a bond listed twice."""
 import numpy as np
 import pytest
 
@@ -63,13 +63,25 @@ def gradient(s, mirrored, precision, h, dt):
     return out[0][:3 * n], out[1][:3 * n], g[:n]
 
 
+def twice(rp, col, i, k):
+    """Entry k of node i's row, and its mirror, listed once more."""
+    j = col[rp[i] + k]
+    for a, b in ((i, j), (j, i)):
+        at = rp[a] + np.searchsorted(col[rp[a]:rp[a + 1]], b)
+        col = np.insert(col, at, b)
+        rp = rp + (np.arange(len(rp)) > a)
+    return rp, col
+
+
 @pytest.mark.parametrize("kw", [{}, dict(factors=True), dict(materials=2), dict(precision=P.PREC_FP64A),
-                                dict(precision=P.PREC_FP32C), dict(tiny=True)],
+                                dict(precision=P.PREC_FP32C), dict(tiny=True), dict(twice=True)],
                          ids=lambda kw: "-".join(kw) or "plain")
 @pytest.mark.parametrize("dims", [(9, 7, 5), (29, 23, 19)])  # 317 and 12,675 nodes
 def test_one_evaluation_equals_two(dims, kw):
     h = 1e-70 if kw.get("tiny") else 1e-3
     s = specimen(dims, h, kw.get("materials", 1), kw.get("factors", False))
+    if kw.get("twice"):
+        s["rp"], s["col"] = twice(s["rp"], s["col"], 100, 3)
     dt = 1.0 if kw.get("tiny") else 5e-8
     prec = kw.get("precision", P.PREC_FP64)
     want, got = (gradient(s, mirrored, prec, h, dt) for mirrored in (False, True))
