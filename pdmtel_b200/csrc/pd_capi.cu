@@ -1862,14 +1862,14 @@ int pd_rk4_step(pd_ctx* c, double dt, double time, double* ke, double* ee) {
     PD_TRY(set_time(c, time));
     // a step like the last one runs as a graph (a lone step is not worth the capture)
     const pd_ctx::StepKey key{dt, c->precision, c->d.energy, c->generation};
-    if (c->last_single == key) {
-        cudaGraphExec_t g = nullptr;
-        PD_TRY(step_graph(c, dt, false, &g));
-        PD_CUDA_TRY(cudaGraphLaunch(g, c->stream));
-    } else {
-        enqueue_step_body(c, dt, false);
-        c->last_single = key;
+    cudaGraphExec_t g = nullptr;
+    if (c->last_single == key && step_graph(c, dt, false, &g) != PD_OK) {
+        g = nullptr;
+        cudaGetLastError();  // a stream that takes no capture (the legacy default one): launches
     }
+    c->last_single = key;
+    if (g) PD_CUDA_TRY(cudaGraphLaunch(g, c->stream));
+    else enqueue_step_body(c, dt, false);
     PD_CUDA_TRY(cudaGetLastError());
     if (c->d.energy && (ke || ee)) {
         PD_CUDA_TRY(cudaMemcpyAsync(c->hscalar, c->d.red + 2 * c->n, 2 * sizeof(double), cudaMemcpyDeviceToHost,
