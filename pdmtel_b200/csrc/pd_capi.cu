@@ -167,8 +167,12 @@ struct pd_ctx {
     struct StepGraph {
         cudaGraphExec_t exec = nullptr;
         StepKey key;
+        bool holds(const StepKey& k) const { return exec && key == k; }
     } graphs[2];
-    StepKey last_single;  // the last pd_rk4_step
+    // pd_rk4_step: the last call, how many calls like it in a row, how many of
+    // them a new graph waits for, and the uses of the present one
+    StepKey last_single;
+    int single_run = 0, single_wait = 2, single_uses = 0;
     double* ue = nullptr;    // [2][3N] one-point scheme: the displacements its bonds use, by stage
     uint64_t generation = 0;
     uint64_t family_gen = 0;  // families installed
@@ -360,7 +364,7 @@ void enqueue_step_body(pd_ctx* c, double dt, bool advance, bool closing_gather =
 int step_graph(pd_ctx* c, double dt, bool advance, cudaGraphExec_t* out) {
     pd_ctx::StepGraph& G = c->graphs[advance];
     const pd_ctx::StepKey key{dt, c->precision, c->d.energy, c->generation};
-    if (!G.exec || !(G.key == key)) {
+    if (!G.holds(key)) {
         if (G.exec) {
             PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
             cudaGraphExecDestroy(G.exec);
@@ -1860,14 +1864,27 @@ int pd_rk4_step(pd_ctx* c, double dt, double time, double* ke, double* ee) {
     if (!c) return fail(PD_ERR_ARG, "pd_rk4_step: null context");
     if (!ready_dynamic(c)) return fail(PD_ERR_ARG, "pd_rk4_step: family/MLS data not set");
     PD_TRY(set_time(c, time));
-    // a step like the last one runs as a graph (a lone step is not worth the capture)
+    // A run of equal steps becomes a graph with its second.  A capture costs
+    // about 130 us and a graph saves 13 to 20 us a step (120 nodes), so one that
+    // gave way before 16 uses doubles the run that the next waits for: two sizes
+    // in turn, two steps each, took 113 us a step, with every second one captured,
+    // where launches took 53.
     const pd_ctx::StepKey key{dt, c->precision, c->d.energy, c->generation};
-    cudaGraphExec_t g = nullptr;
-    if (c->last_single == key && step_graph(c, dt, false, &g) != PD_OK) {
-        g = nullptr;
-        cudaGetLastError();  // a stream that takes no capture (the legacy default one): launches
-    }
+    constexpr int kPaid = 16, kMostWait = 64;
+    c->single_run = c->last_single == key ? std::min(c->single_run + 1, kMostWait) : 1;
     c->last_single = key;
+    cudaGraphExec_t g = nullptr;
+    const bool held = c->graphs[0].holds(key);
+    if (held || c->single_run >= c->single_wait) {
+        if (!held && c->graphs[0].exec)
+            c->single_wait = c->single_uses < kPaid ? std::min(2 * c->single_wait, kMostWait) : 2;
+        if (step_graph(c, dt, false, &g) == PD_OK) {
+            c->single_uses = held ? std::min(c->single_uses + 1, kPaid) : 1;
+        } else {
+            g = nullptr;
+            cudaGetLastError();  // a stream that takes no capture (the legacy default one): launches
+        }
+    }
     if (g) PD_CUDA_TRY(cudaGraphLaunch(g, c->stream));
     else enqueue_step_body(c, dt, false);
     PD_CUDA_TRY(cudaGetLastError());

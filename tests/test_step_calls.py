@@ -1,4 +1,7 @@
-"""pd_rk4_step on a stream that takes no capture."""
+"""pd_rk4_step call by call: on a stream that takes no capture, and with step
+sizes that change every few calls, which a graph per change would slow down."""
+import time
+
 import numpy as np
 import pytest
 
@@ -29,3 +32,40 @@ def test_legacy_default_stream():
         ctx.close()
     (ea, a), (eb, b) = out
     assert ea == eb and np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("run", [2, 3, 5])
+def test_changing_step_sizes_cost_no_more_than_launches(run):
+    """Steps whose size changes with every call never make a graph; sizes that
+    change every few calls may not cost more than those (a quarter is for noise:
+    a capture per change more than doubles two-call runs, and adds a fifth to a
+    half to the longer ones, which save a launch time in the rest)."""
+    def mean(sizes):
+        ctx = context()
+        took, t = [], 0.0
+        for k in range(400):
+            dt = sizes[k % len(sizes)]
+            t += dt
+            start = time.perf_counter()
+            ctx.rk4_step(dt, t)
+            took.append(time.perf_counter() - start)
+        ctx.close()
+        return np.mean(np.sort(took[40:])[:-36])
+
+    launches = min(mean([1e-9, 2e-9]) for _ in range(3))
+    assert min(mean([1e-9] * run + [2e-9] * run) for _ in range(3)) <= 1.25 * launches
+
+
+def test_changing_step_sizes_change_no_result():
+    sizes = [1e-9] * 3 + [2e-9] * 2 + [1e-9, 3e-9] * 2 + [3e-9] * 20 + [1e-9] * 9
+    out = []
+    for way in ("calls", "apart"):
+        ctx = context()
+        t = 0.0
+        for dt in sizes:
+            t += dt
+            ctx.rk4_step(dt, t) if way == "calls" else ctx.rk4_steps(dt, t - dt, 1)
+        ctx.sync()
+        out.append(ctx.get_state())
+        ctx.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
