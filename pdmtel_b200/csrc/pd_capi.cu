@@ -58,6 +58,7 @@ struct pd_ctx {
     std::vector<int32_t> bc_host;               // per-node bc index
     std::vector<int64_t> cbptr_host;            // MLS contributor CSR (host copy)
     std::vector<int32_t> cbidx_host;
+    int spares_used = 0;                        // InUse
     // adjoint: checkpoints (U, V, Gauss-point u, time) of the last forward
     struct Checkpoint {
         double *U = nullptr, *V = nullptr, *ug = nullptr;
@@ -180,11 +181,18 @@ struct pd_ctx {
 
 namespace {
 
+bool spares_release(pd_ctx* c);
+
 template <typename T>
 int dalloc(pd_ctx* c, T** p, size_t count) {
     void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-    if (e != cudaSuccess) return pd::fail_cuda(e, "cudaMalloc", __FILE__, __LINE__);
+    const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+    cudaError_t e = cudaMalloc(&q, bytes);
+    if (e == cudaErrorMemoryAllocation && spares_release(c)) e = cudaMalloc(&q, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here
+        return pd::fail_cuda(e, "cudaMalloc", __FILE__, __LINE__);
+    }
     c->owned.push_back(q);
     *p = (T*)q;
     return PD_OK;
@@ -195,7 +203,6 @@ template <typename T>
 bool try_dalloc(pd_ctx* c, T** p, size_t count) {
     if (dalloc(c, p, count) == PD_OK) return true;
     *p = nullptr;
-    cudaGetLastError();  // answered here
     return false;
 }
 
@@ -204,6 +211,53 @@ void dfree(pd_ctx* c, void* p) {
     auto it = std::find(c->owned.begin(), c->owned.end(), p);
     if (it != c->owned.end()) c->owned.erase(it);
     cudaFree(p);
+}
+
+// Buffers the context keeps for a later call to use again, by the calls that
+// use them.  An allocation that finds no room gives back those that the running
+// call does not use (InUse) and tries once more.
+enum { kSpareStatic = 1, kSpareAdjoint = 2 };
+struct InUse {
+    pd_ctx* c;
+    int before;
+    InUse(pd_ctx* ctx, int spares) : c(ctx), before(ctx->spares_used) { c->spares_used |= spares; }
+    ~InUse() { c->spares_used = before; }
+};
+
+template <typename T>
+bool give_back(pd_ctx* c, T** p) {
+    if (!*p) return false;
+    dfree(c, *p);
+    *p = nullptr;
+    return true;
+}
+
+void mirror_free(pd_ctx* c) {
+    give_back(c, &c->adj_mirror);
+    give_back(c, &c->adj_bond);
+    c->adj_mirror_gen = ~0ull;
+    c->adj_symmetric = false;
+}
+
+// whether anything was given back
+bool spares_release(pd_ctx* c) {
+    cudaGetLastError();
+    bool any = false;
+    if (!(c->spares_used & kSpareStatic)) {
+        any |= give_back(c, &c->cg_work);
+        any |= give_back(c, &c->dotpart);
+        any |= give_back(c, &c->bj_minv);
+        any |= give_back(c, &c->fam_geo);
+        any |= give_back(c, &c->fam_xm);
+        c->fam_gen = ~0ull;
+    }
+    if (!(c->spares_used & kSpareAdjoint)) {
+        any |= c->adj_mirror || c->adj_bond;
+        mirror_free(c);
+        any |= give_back(c, &c->adj_pool);
+        c->adj_pool_count = 0;
+    }
+    return any;
 }
 
 #define PD_TRY(expr)                       \
@@ -498,7 +552,7 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
         (rc = dalloc(c, &nblk, (size_t)N * d.bs)) || (rc = dalloc(c, &sblk, (size_t)N * 8)) ||
         (rc = dalloc(c, &order, N)) || (rc = dalloc(c, &eed, N)) ||
         (rc = dalloc(c, &red, 2 * N + 4 + 2 * 160)) || (rc = dalloc(c, &tdev, 1)) ||
-        (rc = dalloc(c, &c->dotpart, 2 * (N + 4096))) || (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
+        (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
         return bail(rc);
     if (d.cci) try_dalloc(c, &c->ue, 2 * n3);  // without it the epilogues run apart
     if (c->nslit) {
@@ -1158,8 +1212,12 @@ int pd_bond_search(pd_ctx* c, int64_t* num_halves, int64_t* num_broken, double* 
     double mb = 0.0;
     double reach = 0.0;
     for (int a = 0; a < 3; ++a) reach = std::max(reach, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
-    const int rc = pd::bond_search(c->d, g, ncell, reach, c->nslit, sl, &frow, &fcol, &fbr, &arow, &acol, &nh, &nb,
-                                   &mb, c->stream);
+    auto search = [&]() {
+        return pd::bond_search(c->d, g, ncell, reach, c->nslit, sl, &frow, &fcol, &fbr, &arow, &acol, &nh, &nb, &mb,
+                               c->stream);
+    };
+    int rc = search();
+    if (rc == PD_ERR_OOM && spares_release(c)) rc = search();
     if (rc != PD_OK) return rc;
     install_family(c, frow, fcol, fbr, arow, acol, nh, nh - nb);
     if (num_halves) *num_halves = nh;
@@ -2306,22 +2364,24 @@ int stencil_prepare(pd_ctx* c) {
     PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->sten = pd::StencilDev{(int)nx, (int)ny, (int)nz, ns, radius, c->sten_off, c->sten_geo, c->sten_pmask,
                              c->sten_xm, (int)cols.size(), rz, c->sten_col, c->sten_colgeo};
-    if (const int rc = broken_prepare(c, map)) {
-        if (rc == PD_ERR_OOM) cudaGetLastError();  // the entries do not fit: family lists
-        return done(rc == PD_ERR_OOM ? PD_OK : rc);
-    }
+    if (const int rc = broken_prepare(c, map)) return done(rc == PD_ERR_OOM ? PD_OK : rc);  // no room: family lists
     PD_TRY(split_prepare(c, cols, colgeo));
     c->sten_ok = true;
     return done(PD_OK);
 }
 
-// The node records of the family-list operator (its matvec, and every
-// problem's right-hand side).
-int family_prepare(pd_ctx* c) {
+// What the summing kernels leave per block, and their counter.
+int sums_prepare(pd_ctx* c) {
+    if (!c->dotpart) PD_TRY(dalloc(c, &c->dotpart, 2 * (c->n + 4096)));
     if (!c->dot_done) {
         PD_TRY(dalloc(c, &c->dot_done, 1));
         PD_CUDA_TRY(cudaMemsetAsync(c->dot_done, 0, sizeof(unsigned), c->stream));
     }
+    return PD_OK;
+}
+
+// The node records of the family-list operator (its matvec, and pd_static_rhs).
+int family_prepare(pd_ctx* c) {
     if (c->fam_gen == c->generation || c->n == 0) return PD_OK;
     if (!c->fam_geo) PD_TRY(dalloc(c, &c->fam_geo, c->n));
     if (!c->fam_xm) PD_TRY(dalloc(c, &c->fam_xm, c->n));
@@ -2334,8 +2394,9 @@ int family_prepare(pd_ctx* c) {
 }
 
 int static_prepare(pd_ctx* c) {
+    PD_TRY(sums_prepare(c));
     PD_TRY(stencil_prepare(c));
-    return family_prepare(c);
+    return c->sten_ok ? PD_OK : family_prepare(c);
 }
 
 pd::FamilyDev family_dev(const pd_ctx* c) { return pd::FamilyDev{c->fam_geo, c->fam_xm, c->sten_pmask}; }
@@ -2373,6 +2434,7 @@ extern "C" {
 int pd_static_prepare(pd_ctx* c, int* stencil) {
     if (!c) return fail(PD_ERR_ARG, "pd_static_prepare: null context");
     if (!c->have_family) return fail(PD_ERR_ARG, "pd_static_prepare: no family");
+    InUse use(c, kSpareStatic);
     PD_TRY(static_prepare(c));
     if (stencil) *stencil = c->sten_ok ? 1 : 0;
     return PD_OK;
@@ -2381,6 +2443,7 @@ int pd_static_prepare(pd_ctx* c, int* stencil) {
 int pd_static_matvec(pd_ctx* c, double time, const double* x, double* y) {
     if (!c || !x || !y) return fail(PD_ERR_ARG, "pd_static_matvec: null argument");
     if (!c->have_family) return fail(PD_ERR_ARG, "pd_static_matvec: no family");
+    InUse use(c, kSpareStatic);
     PD_TRY(static_prepare(c));
     PD_TRY(upload_vec3(c, c->d.us, x));
     static_apply(c, false, c->d.us, c->d.k1);
@@ -2391,6 +2454,7 @@ int pd_static_matvec(pd_ctx* c, double time, const double* x, double* y) {
 int pd_static_rhs(pd_ctx* c, double time, double* b) {
     if (!c || !b) return fail(PD_ERR_ARG, "pd_static_rhs: null argument");
     if (!c->have_family) return fail(PD_ERR_ARG, "pd_static_rhs: no family");
+    InUse use(c, kSpareStatic);
     PD_TRY(family_prepare(c));
     pd::launch_static_rhs(c->d, family_dev(c), time, c->d.k1, c->stream);
     PD_CUDA_TRY(cudaGetLastError());
@@ -2494,11 +2558,18 @@ extern "C" int pd_static_solve(pd_ctx* c, double time, int precision, double rto
     if (!c->have_family) return fail(PD_ERR_ARG, "pd_static_solve: no family");
     if (precision != PD_PREC_FP64 && precision != PD_PREC_FP64A && precision != PD_PREC_FP32C)
         return fail(PD_ERR_ARG, "pd_static_solve: precision");
+    InUse use(c, kSpareStatic);
     PD_TRY(static_prepare(c));
     const int64_t n3 = 3 * c->n;
-    // the solve's vectors stay with the context for its next solve
+    // the solve's vectors stay with the context for its next solve (InUse)
     if (!c->cg_work) PD_TRY(dalloc(c, &c->cg_work, 6 * n3));
     double *b = c->cg_work, *xd = b + n3, *r = xd + n3, *p = r + n3, *q = p + n3, *z = q + n3;
+    pd::FamilyDev F = family_dev(c);
+    if (c->sten_ok) {  // only the right-hand side reads the node records: in the vectors that come after it
+        double4* rec = reinterpret_cast<double4*>((reinterpret_cast<uintptr_t>(r) + 31) & ~(uintptr_t)31);
+        F = pd::FamilyDev{rec, rec + c->n, c->sten_pmask};
+        pd::launch_family_geo(c->d, rec, c->stream);
+    }
     int rc = upload_vec3(c, xd, x);
     if (rc != PD_OK) return rc;
     if (c->static_precond && (!c->bj_minv || c->bj_gen != c->generation)) {
@@ -2506,7 +2577,7 @@ extern "C" int pd_static_solve(pd_ctx* c, double time, int precision, double rto
         pd::launch_static_bjacobi(c->d, c->bj_minv, c->stream);
         c->bj_gen = c->generation;
     }
-    pd::launch_static_rhs(c->d, family_dev(c), time, b, c->stream);
+    pd::launch_static_rhs(c->d, F, time, b, c->stream);
     int it = 0, nrep = 0;
     double rel = 0.0;
     // A cracked box iterates with the FP64 stencil throughout: the FP32 one
@@ -2686,21 +2757,12 @@ extern "C" int pd_adjoint_forward(pd_ctx* c, double dt, double t0, int nsteps, i
 // The mirror entries for the one-evaluation VJP, once per family; where there
 // is no room for them the points are evaluated twice.
 namespace {
-void mirror_free(pd_ctx* c) {
-    dfree(c, c->adj_mirror);
-    dfree(c, c->adj_bond);
-    c->adj_mirror = nullptr;
-    c->adj_bond = nullptr;
-    c->adj_symmetric = false;
-}
-
 int mirror_prepare(pd_ctx* c) {
     if (c->adj_mirror_gen == c->family_gen) return PD_OK;
     mirror_free(c);
-    c->adj_mirror_gen = c->family_gen;
     if (c->npt != 8 || c->Ha == 0) return PD_OK;
     if (!try_dalloc(c, &c->adj_mirror, c->Ha) || !try_dalloc(c, &c->adj_bond, c->Ha)) {
-        mirror_free(c);
+        mirror_free(c);  // the next sweep tries again
         return PD_OK;
     }
     PD_CUDA_TRY(cudaMemsetAsync(c->dflag, 0, sizeof(int), c->stream));
@@ -2709,6 +2771,7 @@ int mirror_prepare(pd_ctx* c) {
     PD_CUDA_TRY(cudaMemcpyAsync(&bad, c->dflag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->adj_symmetric = !bad;
+    c->adj_mirror_gen = c->family_gen;
     return PD_OK;
 }
 }  // namespace
@@ -2721,6 +2784,7 @@ extern "C" int pd_adjoint_backward(pd_ctx* c, const double* lam_U, const double*
     if (!c || !lam_U || !grad_f) return fail(PD_ERR_ARG, "pd_adjoint_backward: null argument");
     if (c->adj_steps < 1) return fail(PD_ERR_ARG, "pd_adjoint_backward: no forward run to reverse");
     if (!c->d.sfac) return fail(PD_ERR_ARG, "pd_adjoint_backward: set the spring factors first");
+    InUse use(c, kSpareAdjoint);
     if (c->d.mls) PD_TRY(build_transpose(c));
     PD_TRY(mirror_prepare(c));
     const int64_t N = c->n, n3 = 3 * N, ng = n3 * c->npt;
