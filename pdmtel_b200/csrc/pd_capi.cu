@@ -30,6 +30,7 @@ int fail_cuda(cudaError_t e, const char* what, const char* file, int line) {
     char buf[512];
     std::snprintf(buf, sizeof buf, "%s:%d %s: %s", file, line, what, cudaGetErrorString(e));
     g_last_error = buf;
+    cudaGetLastError();  // reported here: not to the next call that looks
     return e == cudaErrorMemoryAllocation ? PD_ERR_OOM : PD_ERR_CUDA;
 }
 
@@ -189,10 +190,7 @@ int dalloc(pd_ctx* c, T** p, size_t count) {
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
     cudaError_t e = cudaMalloc(&q, bytes);
     if (e == cudaErrorMemoryAllocation && spares_release(c)) e = cudaMalloc(&q, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();  // reported here
-        return pd::fail_cuda(e, "cudaMalloc", __FILE__, __LINE__);
-    }
+    if (e != cudaSuccess) return pd::fail_cuda(e, "cudaMalloc", __FILE__, __LINE__);
     c->owned.push_back(q);
     *p = (T*)q;
     return PD_OK;

@@ -91,3 +91,15 @@ def test_after_a_static_solve(stencil):
     b = ctx.static_rhs(1.0)
     assert np.any(b) and np.array_equal(b, ctx.static_rhs(1.0))
     ctx.close()
+
+
+def test_an_error_is_reported_once():
+    ctx, halves = context((64, 64, 64))
+    other, few = context((9, 8, 7))
+    with Taken(16 * MB), pytest.raises(P.PdError):
+        ctx.set_gauss_displ(np.zeros(24 * ctx.n))
+    assert other.bond_search()[0] == few
+    other.mls_setup(3.0 * H)
+    other.rk4_step(1e-9, 1e-9)
+    ctx.close()
+    other.close()
