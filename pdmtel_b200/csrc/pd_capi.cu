@@ -230,6 +230,13 @@ bool give_back(pd_ctx* c, T** p) {
     return true;
 }
 
+// an allocation of one call, freed at its end
+struct Scratch {
+    pd_ctx* c;
+    void* p;
+    ~Scratch() { dfree(c, p); }
+};
+
 void mirror_free(pd_ctx* c) {
     give_back(c, &c->adj_mirror);
     give_back(c, &c->adj_bond);
@@ -2169,10 +2176,8 @@ int split_prepare(pd_ctx* c, const std::vector<int4>& cols, const std::vector<do
             tap[(size_t)k * 9 + 4 + (q - rz)] = make_double2(g.w, g.w * g.z);
         }
     }
-    if (!c->nd_col) {
-        PD_TRY(dalloc(c, &c->nd_col, pd::kMaxStencil));
-        PD_TRY(dalloc(c, &c->nd_tap, (size_t)pd::kMaxStencil * 9));
-    }
+    if (!c->nd_col) PD_TRY(dalloc(c, &c->nd_col, pd::kMaxStencil));
+    if (!c->nd_tap) PD_TRY(dalloc(c, &c->nd_tap, (size_t)pd::kMaxStencil * 9));
     if (!c->nd_diag) PD_TRY(dalloc(c, &c->nd_diag, (size_t)6 * c->n));
     PD_TRY(upload(c, c->nd_col, nd.data(), sizeof(int4) * nc));
     PD_TRY(upload(c, c->nd_tap, tap.data(), sizeof(double2) * tap.size()));
@@ -2222,36 +2227,33 @@ int broken_prepare(pd_ctx* c, const int* lut) {
     int64_t* w = nullptr;  // [4][N + 1]: flags, counts and their scans
     PD_TRY(dalloc(c, &w, 4 * (N + 1)));
     int64_t *flag = w, *cnt = w + (N + 1), *fpos = w + 2 * (N + 1), *cpos = w + 3 * (N + 1);
-    auto done = [&](int rc) {
-        dfree(c, w);
-        return rc;
-    };
+    Scratch freed{c, w};
     pd::launch_broken_counts(c->d, flag, cnt, c->stream);
     if (pd::exclusive_scan_i64(flag, fpos, N, c->stream) != PD_OK ||
         pd::exclusive_scan_i64(cnt, cpos, N, c->stream) != PD_OK)
-        return done(fail(PD_ERR_CUDA, "static operator: scan"));
+        return fail(PD_ERR_CUDA, "static operator: scan");
     int64_t nodes = 0, total = 0;
     if (cudaMemcpy(&nodes, fpos + N, sizeof(int64_t), cudaMemcpyDeviceToHost) != cudaSuccess ||
         cudaMemcpy(&total, cpos + N, sizeof(int64_t), cudaMemcpyDeviceToHost) != cudaSuccess)
-        return done(fail(PD_ERR_CUDA, "static operator: broken bonds"));
+        return fail(PD_ERR_CUDA, "static operator: broken bonds");
     int rc = PD_OK;
     if ((rc = dalloc(c, &c->sten_bnode, nodes)) || (rc = dalloc(c, &c->sten_bptr, nodes + 1)) ||
         (rc = dalloc(c, &c->sten_bent, total)) || (rc = dalloc(c, &c->sten_bidx, N)) ||
         (rc = dalloc(c, &c->sten_brow, 3 * nodes)))
-        return done(rc);
+        return rc;
     pd::launch_broken_fill(c->d, lut, flag, fpos, cpos, c->sten_bnode, c->sten_bptr, c->sten_bent, c->sten_bidx,
                            c->stream);
     if (cudaMemcpyAsync(c->sten_bptr + nodes, &total, sizeof(int64_t), cudaMemcpyHostToDevice, c->stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
-        return done(fail(PD_ERR_CUDA, "static operator: broken bonds"));
+        return fail(PD_ERR_CUDA, "static operator: broken bonds");
     c->sten.bnode = c->sten_bnode;
     c->sten.bptr = c->sten_bptr;
     c->sten.bent = c->sten_bent;
     c->sten.bidx = c->sten_bidx;
     c->sten.brow = c->sten_brow;
     c->sten.nbrk = (int)nodes;
-    return done(PD_OK);
+    return PD_OK;
 }
 
 int stencil_prepare(pd_ctx* c) {
@@ -2271,24 +2273,21 @@ int stencil_prepare(pd_ctx* c) {
     PD_TRY(dalloc(c, &map, kSpan + 4 + 4 * pd::kMaxStencil));
     int* err = map + kSpan;
     int4* dlist = reinterpret_cast<int4*>(map + kSpan + 4);
-    auto done = [&](int rc) {
-        dfree(c, map);
-        return rc;
-    };
+    Scratch freed{c, map};
     int found[2];
     std::vector<int4> list(pd::kMaxStencil);
     std::vector<std::array<int, 3>> offs;
     if (cudaMemsetAsync(map, 0, sizeof(int) * (kSpan + 4), c->stream) != cudaSuccess)
-        return done(fail(PD_ERR_CUDA, "static operator: offsets"));
+        return fail(PD_ERR_CUDA, "static operator: offsets");
     pd::launch_box_offsets(c->d, map, err, dlist, c->stream);
     if (cudaMemcpyAsync(found, err, sizeof(found), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
         cudaMemcpyAsync(list.data(), dlist, sizeof(int4) * list.size(), cudaMemcpyDeviceToHost, c->stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
-        return done(fail(PD_ERR_CUDA, "static operator: offsets"));
-    if (found[0] || found[1] > pd::kMaxStencil) return done(PD_OK);
+        return fail(PD_ERR_CUDA, "static operator: offsets");
+    if (found[0] || found[1] > pd::kMaxStencil) return PD_OK;
     for (int k = 0; k < found[1]; ++k) offs.push_back({list[k].x, list[k].y, list[k].z});
-    if (offs.empty() || offs.size() > (size_t)pd::kMaxStencil) return done(PD_OK);
+    if (offs.empty() || offs.size() > (size_t)pd::kMaxStencil) return PD_OK;
     std::sort(offs.begin(), offs.end(), [&](const std::array<int, 3>& a, const std::array<int, 3>& b) {
         return a[0] + nx * (a[1] + ny * a[2]) < b[0] + nx * (b[1] + ny * b[2]);
     });
@@ -2297,13 +2296,13 @@ int stencil_prepare(pd_ctx* c) {
         for (const auto& o : offs) list.push_back(make_int4(o[0], o[1], o[2], 0));
         if (cudaMemcpyAsync(dlist, list.data(), sizeof(int4) * list.size(), cudaMemcpyHostToDevice, c->stream) !=
             cudaSuccess)
-            return done(fail(PD_ERR_CUDA, "static operator: offsets"));
+            return fail(PD_ERR_CUDA, "static operator: offsets");
         pd::launch_box_check(c->d, dlist, (int)list.size(), map, err, c->stream);
         int bad = 0;
         if (cudaMemcpyAsync(&bad, err, sizeof(int), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
             cudaStreamSynchronize(c->stream) != cudaSuccess)
-            return done(fail(PD_ERR_CUDA, "static operator: families"));
-        if (bad) return done(PD_OK);
+            return fail(PD_ERR_CUDA, "static operator: families");
+        if (bad) return PD_OK;
     }
     const int ns = (int)offs.size();
     std::vector<int4> off(ns);
@@ -2342,14 +2341,12 @@ int stencil_prepare(pd_ctx* c) {
             colgeo[(size_t)cidx * W + offs[k][2] + rz] = geo[k];
         }
     }
-    if (!c->sten_off) {
-        PD_TRY(dalloc(c, &c->sten_off, pd::kMaxStencil));
-        PD_TRY(dalloc(c, &c->sten_geo, pd::kMaxStencil));
-        if (!c->sten_pmask) PD_TRY(dalloc(c, &c->sten_pmask, N));
-        PD_TRY(dalloc(c, &c->sten_xm, 3 * N));
-        PD_TRY(dalloc(c, &c->sten_col, pd::kMaxStencil));
-        PD_TRY(dalloc(c, &c->sten_colgeo, (size_t)pd::kMaxStencil * 9));
-    }
+    if (!c->sten_off) PD_TRY(dalloc(c, &c->sten_off, pd::kMaxStencil));
+    if (!c->sten_geo) PD_TRY(dalloc(c, &c->sten_geo, pd::kMaxStencil));
+    if (!c->sten_pmask) PD_TRY(dalloc(c, &c->sten_pmask, N));
+    if (!c->sten_xm) PD_TRY(dalloc(c, &c->sten_xm, 3 * N));
+    if (!c->sten_col) PD_TRY(dalloc(c, &c->sten_col, pd::kMaxStencil));
+    if (!c->sten_colgeo) PD_TRY(dalloc(c, &c->sten_colgeo, (size_t)pd::kMaxStencil * 9));
     PD_TRY(upload(c, c->sten_off, off.data(), sizeof(int4) * ns));
     PD_TRY(upload(c, c->sten_geo, geo.data(), sizeof(double4) * ns));
     if (!cols.empty() && cols.size() <= (size_t)pd::kMaxStencil && colgeo.size() <= (size_t)pd::kMaxStencil * 9) {
@@ -2362,10 +2359,10 @@ int stencil_prepare(pd_ctx* c) {
     PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->sten = pd::StencilDev{(int)nx, (int)ny, (int)nz, ns, radius, c->sten_off, c->sten_geo, c->sten_pmask,
                              c->sten_xm, (int)cols.size(), rz, c->sten_col, c->sten_colgeo};
-    if (const int rc = broken_prepare(c, map)) return done(rc == PD_ERR_OOM ? PD_OK : rc);  // no room: family lists
+    if (const int rc = broken_prepare(c, map)) return rc == PD_ERR_OOM ? PD_OK : rc;  // no room: family lists
     PD_TRY(split_prepare(c, cols, colgeo));
     c->sten_ok = true;
-    return done(PD_OK);
+    return PD_OK;
 }
 
 // What the summing kernels leave per block, and their counter.

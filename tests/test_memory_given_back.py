@@ -1,7 +1,8 @@
 """Buffers that a context keeps for its next static solve or reverse sweep are
 given back when another call finds no room, and made again when they are
 needed: with the rest of the device's memory taken, calls succeed that fit
-beside the problem but not beside those buffers."""
+beside the problem but not beside those buffers.  A static preparation that
+fails keeps none of its scratch memory."""
 import numpy as np
 import pytest
 
@@ -103,3 +104,21 @@ def test_an_error_is_reported_once():
     other.rk4_step(1e-9, 1e-9)
     ctx.close()
     other.close()
+
+
+def test_a_failed_preparation_leaves_no_scratch():
+    import torch
+
+    used = []
+    for failures in (0, 4):
+        before = torch.cuda.mem_get_info()[0]
+        ctx, _ = context((64, 64, 64))
+        for _ in range(failures):
+            # the 8 MB offset table fits, the operator's 19 MB do not
+            with Taken(16 * MB), pytest.raises(P.PdError):
+                ctx.static_prepare()
+            ctx.set_option(P.OPT_STATIC_STENCIL, 1)
+        assert ctx.static_prepare()
+        used.append(before - torch.cuda.mem_get_info()[0])
+        ctx.close()
+    assert used[1] - used[0] < 8 * MB
