@@ -951,12 +951,16 @@ def run_ours(args):
     gather_ms = prof[1] / 4.0
     npt = I.num_gauss
     ncb = I.num_contrib
-    # the kernels the tuner kept
-    sten = bool(tune.get("force_stencil"))
-    force_kernel = ("k_force_f32c_sten" if sten else "k_force_f32c_quad" if tune.get("force_quad")
+    # the kernels the tuner kept (below 65,536 nodes the lane kernels run in
+    # place of the stencil force and the ring gather)
+    large = n >= 65536
+    sten = bool(tune.get("force_stencil")) and large
+    force_kernel = ("k_force_f32c_sten" if sten else "k_force_f32c_lanes" if tune.get("force_stencil")
+                    else "k_force_f32c_quad" if tune.get("force_quad")
                     else "k_force_f32c_tiled" if tune.get("force_tile") else "k_force_f32c_lanes")
-    pat, sell = bool(tune.get("gather_stencil")), bool(tune.get("gather_sell"))
-    gather_kernel = "k_gather_f32c_ring" if (pat and sell) else "k_gather_f32c_lanes"
+    pat = bool(tune.get("gather_stencil")) and bool(tune.get("gather_sell")) and large
+    gather_kernel = ("k_gather_f32c_ring" if pat else "k_gather_f32c_pt" if tune.get("gather_per_point")
+                     else "k_gather_f32c_lanes")
     # coefficients, contributor ids (pattern ids instead with patterns), trial
     # displacement, output blocks, partition-of-unity sums, row pointers
     gather_bytes = (ncb * npt * 4 + (n * 4 if pat else ncb * 4 + (n + 1) * 8) + n * 8 * 4 + n * npt * 12
@@ -985,7 +989,9 @@ def run_ours(args):
                 "h2d_bytes_per_step": 2 * 3 * n * 8, "d2h_bytes_per_step": 2 * 3 * n * 8},
         # per step: 4 stages x (gather, force, epilogue) + the time advance;
         # the stencil force is two launches (series pass, exact pass)
-        "gpu_launches": (13 + (4 if sten else 0)) * args.steps,
+        # begin, four forces (the stencil's two passes), four gathers, and four
+        # epilogues where the force does not take them along
+        "gpu_launches": (9 + (8 if sten else 0 if force_kernel == "k_force_f32c_lanes" else 4)) * args.steps,
         "roofline": {"bound": "fp32", "kernel": force_kernel, "achieved": force_flops / (force_ms / 1e3) / 1e12,
                      "peak": peak32 / 1e12, "unit": "TFLOP/s",
                      "frac": force_flops / (force_ms / 1e3) / peak32, "traffic": traffic,

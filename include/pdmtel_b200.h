@@ -382,7 +382,9 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  *   stencil-shaped families (checked; the rows of nodes with broken bonds are
  *   formed from lists of their unbroken ones); 0 keeps the family-list kernel.
  * PD_OPT_GATHER_PER_POINT: 1 runs the FP32-form MLS gather with one thread
- *   per (node, Gauss point), 0 (default) with one per four points.
+ *   per (node, Gauss point) that reads its contributors itself, 0 (default)
+ *   with eight lanes per node that share them (2x2x2 points) or one thread per
+ *   four points (other rules).
  * PD_OPT_FORCE_TILE: the FP32-form force (2x2x2 points, nodes on one
  *   lattice) stages lattice tiles of tx x ty x tz positions and their halo
  *   in shared memory, value = tx | ty << 8 | tz << 16 (tx even, 32 to 256
@@ -392,9 +394,11 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  *   (nodes on one lattice, one material, no critical stretch within reach;
  *   otherwise ignored); 0 (default) with two.
  * PD_OPT_GATHER_SELL: 1 keeps a sliced-ELLPACK copy of the FP32 gather's
- *   contributor lists and coefficients (16 nodes of the work order side by
- *   side per contributor slot: coalesced loads; 2x2x2 points), 0 (default)
- *   reads the CSR lists.  Costs a second FP32 copy of the coefficients.
+ *   coefficients (16 nodes of the work order side by side per contributor
+ *   slot: coalesced loads; 2x2x2 points), which the gather reads when
+ *   PD_OPT_GATHER_STENCIL is on too; 0 (default) reads the CSR lists.  Costs a
+ *   second FP32 copy of the coefficients.  Problems of fewer than 65,536 nodes
+ *   read the lists, and make no copy, whatever the option says.
  * PD_OPT_PERSIST_WAIT_US: how long a grid barrier of the persistent launch
  *   waits before it gives up (default 4 s; 1 ms to 60 s).
  * PD_OPT_PERSIST_TEST_STALL: 1 makes block 0 of the persistent launch skip
@@ -406,7 +410,9 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  *   block covers 16 x-adjacent node pairs by (8x1, 4x2, 2x4, 1x8) rows x
  *   layers for the values 1..4.  Needs 2x2x2 points, one material and a
  *   complete box lattice whose node ids are x + nx (y + ny z) (checked on
- *   the device: PD_ERR_ARG otherwise).  Takes precedence over the other
+ *   the device: PD_ERR_ARG otherwise).  Problems of fewer than 65,536 nodes
+ *   run a lane per bond on the same node blocks, the faster kernel there, for
+ *   each of the four values.  Takes precedence over the other
  *   force variants; 0 (default) turns it off.  Reset to 0 whenever the
  *   family changes.  Same results bit for bit as the other FP32 kernels
  *   when no critical stretch is within reach (with one, those form bond
@@ -418,11 +424,12 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  *   evaluates every Gauss point with the strain series alone, then a pass
  *   that redoes, with the exact form where needed, only the tiles in which
  *   a point left the series range (one byte per tile, kept by the context).
- * PD_OPT_GATHER_STENCIL: 1 lets the FP32-form gather (one thread per four
- *   points) take every node's MLS contributors from a pattern of id offsets
- *   (nodes whose lists are translates of each other share one; kept with
- *   the context and rebuilt by pd_set_mls) instead of its list, so the
- *   contributor loads no longer wait on an index load from memory.  Same
+ * PD_OPT_GATHER_STENCIL: 1 lets the FP32-form gather take every node's MLS
+ *   contributors from a pattern of id offsets (nodes whose lists are
+ *   translates of each other share one; built when first asked for and again
+ *   with new MLS data) instead of its list, so the contributor loads no longer
+ *   wait on an index load from memory: with 2x2x2 points together with
+ *   PD_OPT_GATHER_SELL from 65,536 nodes on, with other rules always.  Same
  *   contributors in the same order: same results bit for bit.  Refused
  *   (PD_ERR_ARG) when the distinct patterns would hold more than a quarter
  *   of all list entries (at least 4M allowed, at most 64M); 0 (default)

@@ -132,8 +132,7 @@ struct pd_ctx {
     longlong2* fst_boxb = nullptr;
     std::vector<int64_t> box_first;  // pd_set_boxes: node ranges that are complete box lattices
     std::vector<int4> box_dims;
-    int64_t* sell_off = nullptr;  // SELL copy of the FP32 gather's lists
-    int32_t* sell_idx = nullptr;
+    int64_t* sell_off = nullptr;  // SELL copy of the FP32 gather's coefficients
     float* sell_coef = nullptr;
     int64_t* adj_mirror = nullptr;  // mirror entries of the unbroken family and a bond's share (k_vjp_bonds)
     double4* adj_bond = nullptr;
@@ -750,20 +749,17 @@ int pd_sync(pd_ctx* c) {
     return PD_OK;
 }
 
-// The SELL copy of the FP32 gather's contributor lists, in the current work
-// order (rebuilt after pd_set_mls and after a work-order change; freed when
-// the gather cannot use it).
+// The SELL copy of the FP32 gather's coefficients, in the current work order
+// (rebuilt after pd_set_mls and after a work-order change; left out where no
+// gather reads it).
 static int sell_prepare(pd_ctx* c) {
     dfree(c, c->sell_off);
-    dfree(c, c->sell_idx);
     dfree(c, c->sell_coef);
     c->sell_off = nullptr;
-    c->sell_idx = nullptr;
     c->sell_coef = nullptr;
     c->d.sell_off = nullptr;
-    c->d.sell_idx = nullptr;
     c->d.sell_coef = nullptr;
-    if (!c->d.sell_on || !c->have_mls || !c->d.mls || c->npt != 8 || c->n == 0) return PD_OK;
+    if (!c->d.sell_on || !c->have_mls || !c->d.mls || c->npt != 8 || !pd::large_forms(c->d)) return PD_OK;
     const int64_t S = pd::sell_slices(c->d);
     int64_t* width = nullptr;
     PD_TRY(dalloc(c, &width, S));
@@ -774,12 +770,10 @@ static int sell_prepare(pd_ctx* c) {
     if (rc != PD_OK) return fail(PD_ERR_CUDA, "SELL layout: scan");
     int64_t total = 0;
     PD_CUDA_TRY(cudaMemcpy(&total, c->sell_off + S, sizeof(int64_t), cudaMemcpyDeviceToHost));
-    PD_TRY(dalloc(c, &c->sell_idx, total * 16));
     PD_TRY(dalloc(c, &c->sell_coef, total * 16 * 8));
     c->d.sell_off = c->sell_off;
-    c->d.sell_idx = c->sell_idx;
     c->d.sell_coef = c->sell_coef;
-    pd::launch_sell_fill(c->d, c->sell_off, c->sell_idx, c->sell_coef, c->stream);
+    pd::launch_sell_fill(c->d, c->sell_off, c->sell_coef, c->stream);
     PD_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->generation++;
     return PD_OK;
@@ -3116,7 +3110,7 @@ extern "C" int pd_autotune(pd_ctx* c, double dt, int steps, pd_tune_result* out)
         if ((rc = trial(T)) != PD_OK) return done(rc);
         if (!(best.ms < before)) c->d.gather_per_point = gp0;
         out->gather_per_point = c->d.gather_per_point;
-        if (c->npt == 8 && !c->d.gather_per_point) {
+        if (c->npt == 8 && !c->d.gather_per_point && pd::large_forms(c->d)) {
             // every combination of the SELL copy (rebuilt for every later order
             // trial) and the contributor patterns (refused when nothing
             // repeats); both together run the coefficient ring
@@ -3146,7 +3140,7 @@ extern "C" int pd_autotune(pd_ctx* c, double dt, int steps, pd_tune_result* out)
         const int f0 = c->fst_shape;
         int keep = f0;
         const double before = best.ms;
-        for (int sh = 1; sh <= 4; ++sh) {
+        for (int sh = 1; sh <= (pd::large_forms(c->d) ? 4 : 1); ++sh) {  // below, every shape is the lane kernel
             if (pd_set_option(c, PD_OPT_FORCE_STENCIL, sh) != PD_OK) break;  // not a box lattice: skip
             Trial T{best.tile, 0, c->persist_per_sm, c->force_chunk, c->gather_chunk, 0.0};
             const double prev = best.ms;

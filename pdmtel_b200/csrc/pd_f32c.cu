@@ -1591,7 +1591,7 @@ __global__ void k_blocks_to_ug(Dev d, double* __restrict__ ug) {
     }
 }
 
-// SELL layout: the widest contributor list of every slice, then the copy
+// SELL layout: the widest contributor list of every slice, then the coefficients
 __global__ void k_sell_width(Dev d, int64_t* __restrict__ width, int64_t S) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (s >= S) return;
@@ -1605,14 +1605,12 @@ __global__ void k_sell_width(Dev d, int64_t* __restrict__ width, int64_t S) {
     width[s] = w;
 }
 
-__global__ void k_sell_fill(Dev d, const int64_t* __restrict__ off, int32_t* __restrict__ sidx,
-                            float* __restrict__ scoef) {
+__global__ void k_sell_fill(Dev d, const int64_t* __restrict__ off, float* __restrict__ scoef) {
     const int64_t slot = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (slot >= d.n) return;
     const int64_t i = d.order[slot], sl = slot / kSell, l = slot % kSell, base = off[sl];
     const int64_t c0 = d.cbptr[i], nc = d.cbptr[i + 1] - c0;
     for (int64_t k = 0; k < nc; ++k) {
-        sidx[(base + k) * kSell + l] = d.cbidx[c0 + k];
         const float* src = d.coeff32 + (c0 + k) * 8;
         float* dst = scoef + ((base + k) * kSell + l) * 8;
         for (int g = 0; g < 8; ++g) dst[g] = src[g];
@@ -1848,6 +1846,7 @@ inline int force_lanes(const Dev& d) { return d.n < 12288 ? 32 : (d.n < 131072 ?
 // there are (5,500 nodes 296 us against 39, 50,000 238 against 167, 80,000 299
 // against 298, a batch of 97,000 375 against 432).
 constexpr int64_t kStencilFrom = 65536;
+bool large_forms(const Dev& d) { return d.n >= kStencilFrom; }
 
 template <bool CCI>
 void launch_any(const Dev& d, double dts, cudaStream_t s, int stage, double dt) {
@@ -1875,7 +1874,7 @@ bool launch_force_f32c(const Dev& d, double dts, cudaStream_t s, int stage, doub
     const int lanes = force_lanes(d);
     const unsigned nbl = blocks_for(lanes * d.n, 128);
     const size_t shl = 4 * sizeof(float) * (2 * 32 * kTileStride + 32 / lanes * lane_group_words(lanes));
-    if (d.blk_cm && d.sten_mask && d.npt == 8 && d.gc_host && d.n < kStencilFrom) {
+    if (d.blk_cm && d.sten_mask && d.npt == 8 && d.gc_host && !large_forms(d)) {
         const bool bd = d.bdry_on != 0, sf = d.sfac != nullptr;
         const PointPack<8> P = pack_points<8>(d, d.gc_host);
 #define PD_STEN_L(HF, BD, SF)                                                                                  \
@@ -2023,11 +2022,11 @@ void launch_gather_f32c(const Dev& d, const double* us, cudaStream_t s) {
     }
     const int ngrp = (d.npt + 3) / 4;
     const unsigned nb = blocks_for(d.n * ngrp, 256);
-    const bool sell = d.sell_on && d.sell_idx && d.mls && d.npt == 8, pat = d.gpat_id && d.mls;
+    const bool sell = d.sell_on && d.sell_coef && d.mls && d.npt == 8, pat = d.gpat_id && d.mls;
     // the ring wins once its stream of coefficients fills the memory system
     // (640,000 nodes 433 us against 521, a batch of 97,000 121 against 125;
     // 5,500 nodes 37 against 21)
-    const bool ring = sell && pat && d.n >= kStencilFrom;
+    const bool ring = sell && pat && large_forms(d);
     if (d.npt == 8 && d.mls && !ring) {
         k_gather_f32c_lanes<<<blocks_for(8 * d.n, 128), 128, 4 * gather_warp_bytes<float>(kGatherStages), s>>>(d, us);
         return;
@@ -2071,8 +2070,8 @@ void launch_sell_width(const Dev& d, int64_t* width, cudaStream_t s) {
     if (S) k_sell_width<<<blocks_for(S, 256), 256, 0, s>>>(d, width, S);
 }
 
-void launch_sell_fill(const Dev& d, const int64_t* off, int32_t* sidx, float* scoef, cudaStream_t s) {
-    if (d.n) k_sell_fill<<<blocks_for(d.n, 128), 128, 0, s>>>(d, off, sidx, scoef);
+void launch_sell_fill(const Dev& d, const int64_t* off, float* scoef, cudaStream_t s) {
+    if (d.n) k_sell_fill<<<blocks_for(d.n, 128), 128, 0, s>>>(d, off, scoef);
 }
 
 void launch_pack_cci_f32c(const Dev& d, cudaStream_t s) {

@@ -120,7 +120,6 @@ struct Dev {
     // FP32 gather in SELL layout (16 nodes per slice of the work order, 2x2x2 points)
     int sell_on;
     const int64_t* sell_off;  // [slices + 1] first contributor slot of each slice
-    const int32_t* sell_idx;  // [slots][16]
     const float* sell_coef;   // [slots][16][8]
     // FP32 force on the lattice stencil (2x2x2 points, one material, nodes
     // that form complete box lattices: box b holds the nodes first_b ..
@@ -230,8 +229,11 @@ void launch_gather_f32c(const Dev& d, const double* us, cudaStream_t s);
 void launch_pack_cci_f32c(const Dev& d, cudaStream_t s);
 size_t tiled_smem_bytes(const Dev& d);
 int64_t sell_slices(const Dev& d);
+// whether the size allows the stencil force and the ring gather (with its SELL
+// coefficients); smaller problems take the lane kernels whatever the options say
+bool large_forms(const Dev& d);
 void launch_sell_width(const Dev& d, int64_t* width, cudaStream_t s);
-void launch_sell_fill(const Dev& d, const int64_t* off, int32_t* sidx, float* scoef, cudaStream_t s);
+void launch_sell_fill(const Dev& d, const int64_t* off, float* scoef, cudaStream_t s);
 int prepare_tiled_force(size_t smem);
 void launch_family_radius(const Dev& d, int* out, cudaStream_t s);
 // lattice-stencil force setup: offsets present in the families (bitmap over

@@ -112,3 +112,25 @@ def test_stencil_force_and_ring_on_several_boxes():
         ctx.set_option(P.OPT_FORCE_STENCIL, shape)
         assert same(steps(ctx, local, 1e-4), want), shape
     ctx.close()
+
+
+def test_sell_copy_holds_the_coefficients_and_nothing_else():
+    import torch
+
+    def made(ctx):
+        before = torch.cuda.mem_get_info()[0]
+        ctx.set_option(P.OPT_GATHER_SELL, 1)
+        return before - torch.cuda.mem_get_info()[0]
+
+    ctx, _ = context(DIMS)
+    width = np.diff(ctx.get_mls()[0])
+    at = np.stack(np.unravel_index(np.arange(ctx.n), DIMS[::-1]), -1)[:, ::-1]  # x, y, z
+    shift = np.array([3, 2, 2])
+    tile, inner = at >> shift, at & ((1 << shift) - 1)
+    order = np.lexsort((inner[:, 0], inner[:, 1], inner[:, 2], tile[:, 0], tile[:, 1], tile[:, 2]))
+    slices = np.concatenate([width[order], np.zeros(-ctx.n % 16, width.dtype)]).reshape(-1, 16).max(1)
+    assert made(ctx) <= slices.sum() * 16 * 8 * 4 + (8 << 20)
+    ctx.close()
+    ctx, _ = context((40, 30, 20))  # no gather reads it below 65,536 nodes
+    assert made(ctx) <= 2 << 20 and ctx.get_option(P.OPT_GATHER_SELL) == 1
+    ctx.close()
