@@ -987,9 +987,7 @@ def run_ours(args):
         "rel_err_vs_fp64": {"U": err_u, "V": err_v, "after_steps": args.warmup + args.steps},
         "e2e": {"value": ws * evals_step * args.steps / (ms_e2e / 1e3), "unit": UNIT,
                 "h2d_bytes_per_step": 2 * 3 * n * 8, "d2h_bytes_per_step": 2 * 3 * n * 8},
-        # per step: 4 stages x (gather, force, epilogue) + the time advance;
-        # the stencil force is two launches (series pass, exact pass)
-        # begin, four forces (the stencil's two passes), four gathers, and four
+        # per step: begin, four forces (the stencil's two passes), four gathers, and four
         # epilogues where the force does not take them along
         "gpu_launches": (9 + (8 if sten else 0 if force_kernel == "k_force_f32c_lanes" else 4)) * args.steps,
         "roofline": {"bound": "fp32", "kernel": force_kernel, "achieved": force_flops / (force_ms / 1e3) / 1e12,

@@ -309,7 +309,8 @@ __global__ void k_vjp_pack(Dev d, const double* __restrict__ teU, const double* 
 // Two passes of eight lanes per node, a lane per point, evaluated every point
 // twice, gathered 24 displacements per bond in one of them and formed the roots
 // and the division with the library's routines: 0.81 + 0.66 ms for 32,768 nodes
-// (51.1M points); 0.58 ms here and 0.04 in k_vjp_nodes.  FP64 pipe 41 % busy at
+// (51.1M points); 0.66 ms here and 0.04 in k_vjp_nodes (0.58 with roots and
+// quotients left unrounded).  FP64 pipe 43 % busy at
 // eight warps per SM (254 registers; three blocks at 168 spill and measured the
 // same): bound by the latency of its chains.
 template <int L>

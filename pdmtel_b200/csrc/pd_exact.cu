@@ -2,10 +2,12 @@
 //
 // This translation unit is compiled with -fmad=false: every multiply and add
 // is rounded on its own, in the order the reference's C++ evaluates it, and
-// double division and square root are IEEE round-to-nearest.  One thread owns
-// one node and sums its family in ascending id order, which is the order of
-// the reference's loops, so the force, gather and state vectors are bit-for-
-// bit those of the reference CPU path (pdDataManager.cpp:1767-2134).
+// double division and square root are IEEE round-to-nearest (by the compiler's
+// operators, or by pd_rn.cuh inside its range).  A node's lanes take its bonds
+// or contributors side by side; every sum adds its terms one after another in
+// family order, which is the order of the reference's loops, so the force,
+// gather and state vectors are bit-for-bit those of the reference CPU path
+// (pdDataManager.cpp:1767-2134).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -1450,7 +1452,8 @@ int bond_search(const Dev& d, const SearchGrid& g, int64_t ncell, double reach, 
     PD_S_TRY(cudaMalloc(&acol, sizeof(int32_t) * (tot[1] + 1)));
     const int cap = (int)hs[1] + 1;
     const size_t sh = (size_t)wpb * cap * sizeof(uint32_t);
-    // the limit of the buffers of earlier builds (five bytes an entry)
+    // Largest family taken: 10,239 members.  The keys themselves (four bytes)
+    // would allow a quarter more; what is refused does not follow their size.
     if ((size_t)wpb * cap * 5 > 200 * 1024)
         return release(fail(PD_ERR_CAPACITY, "family larger than the search kernel's shared buffer"));
     if (sh > 48 * 1024)

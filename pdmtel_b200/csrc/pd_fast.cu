@@ -333,12 +333,13 @@ __global__ void k_broken_fill(Dev d, const int* __restrict__ map, const int64_t*
 // per node; the operator kernels store them in place of their own.  A cracked
 // box then runs on the stencil, with lists only where the crack cut: 60x40x12
 // with a slit, 65 us per matvec on the family lists, 7 us here and about 15 in
-// k_static_nd; the solve 4.43 -> 4.31 ms, 96x96x96 90 -> 95 ms, against
-// subtracting the broken entries from the whole stencil.  (That difference is
-// rounding noise where a node, or one direction of it, has no stiffness left;
-// the preconditioner weights the noise by 17 orders of magnitude and the solve
-// does not converge.)  Entries in a list: read from acol through the lattice
-// positions and an offset table the same solve took 4.54 ms.
+// k_static_nd.  Subtracting the broken entries from the whole stencil instead
+// leaves rounding noise where a node, or one direction of it, has no stiffness
+// left; the preconditioner weights that noise by 17 orders of magnitude and the
+// solve does not converge.  Solves, subtracted -> listed: 60x40x12 4.46 -> 4.30
+// ms, 46x16x21 3.84 -> 4.05, 96x96x96 90 -> 95.  Bound by the latency of entry
+// -> neighbour: 4.49 ms without the next entry loaded ahead, 4.54 read from acol
+// through the lattice positions and an offset table.
 template <bool SFAC>
 __global__ void __launch_bounds__(128) k_static_rows(Dev d, StencilDev S, const double* __restrict__ xm) {
     const int k = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
@@ -346,8 +347,12 @@ __global__ void __launch_bounds__(128) k_static_rows(Dev d, StencilDev S, const 
     const int64_t N = d.n, i = S.bnode[k];
     const double x0 = xm[i], x1 = xm[N + i], x2 = xm[2 * N + i];
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int64_t p = S.bptr[k] + lane; p < S.bptr[k + 1]; p += 32) {
-        const int2 e = S.bent[p];
+    const int64_t pe = S.bptr[k + 1];
+    int64_t p = S.bptr[k] + lane;
+    int2 next = p < pe ? S.bent[p] : make_int2(0, 0);
+    for (; p < pe; p += 32) {
+        const int2 e = next;
+        if (p + 32 < pe) next = S.bent[p + 32];
         const int64_t j = e.x;
         const double4 g = S.geo[e.y];
         double w = g.w;
