@@ -970,7 +970,7 @@ def run_ours(args):
     tp = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(tp):
         with open(tp) as f:
-            traffic = json.load(f).get("force_f32c_sten_bytes_per_launch" if sten else "force_f32c_bytes_per_launch")
+            traffic = json.load(f).get("force_f32c_sten_bytes_per_launch") if sten else None
     value = replica_throughput(ws, evals_step * args.steps, ms32 / 1e3)
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,

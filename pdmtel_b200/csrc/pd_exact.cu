@@ -152,8 +152,8 @@ __device__ __forceinline__ bool point_rn(const BetaIn& B, double bE, double c, d
 // far nodes' displacements, then reads ue and leaves the next stage's in
 // ue_next.
 //
-// Bound by the FP64 pipe and the latency of its chains: 146 instructions per
-// evaluation, about 71 of them FP64 (pipe 53 % busy), and no faster with more
+// Bound by the FP64 pipe and the latency of its chains: 154 instructions per
+// evaluation, about 71 of them FP64 (pipe 57 % busy), and no faster with more
 // warps (five blocks per SM 1.51 ms, six 1.48, against 1.45 with four; four
 // points side by side at three blocks 1.50, all eight 1.67-1.91).  200x200x4
 // cracked plate, per launch: 3.86 -> 1.45 ms against one thread per node with

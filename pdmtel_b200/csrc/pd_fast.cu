@@ -332,7 +332,7 @@ __global__ void k_broken_fill(Dev d, const int* __restrict__ map, const int64_t*
 // The rows of the nodes with broken bonds from their unbroken entries, a warp
 // per node; the operator kernels store them in place of their own.  A cracked
 // box then runs on the stencil, with lists only where the crack cut: 60x40x12
-// with a slit, 65 us per matvec on the family lists, 7 us here and about 15 in
+// with a slit, 65 us per matvec on the family lists, 9 us here and 22 in
 // k_static_nd.  Subtracting the broken entries from the whole stencil instead
 // leaves rounding noise where a node, or one direction of it, has no stiffness
 // left; the preconditioner weights that noise by 17 orders of magnitude and the
