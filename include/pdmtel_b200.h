@@ -359,7 +359,7 @@ int pd_static_rhs(pd_ctx* ctx, double time, double* b);
  * b - K x whenever it has fallen 100-fold and at convergence ("reliable
  * updates"); convergence is judged on the FP64 true residual.  On a cracked
  * lattice stencil (PD_OPT_STATIC_STENCIL) the FP32C iterations' matvec is the
- * FP64 one.  x [3N] is the initial guess in and the solution out.
+ * FP64 one and the residual is replaced at convergence only.  x [3N] is the initial guess in and the solution out.
  * iters/relres may be NULL. */
 int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int maxit, double* x, int* iters,
                     double* relres);

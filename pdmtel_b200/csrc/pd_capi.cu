@@ -2522,8 +2522,9 @@ int cg_static(pd_ctx* c, const double* b, double* x, double* r, double* p, doubl
         rel = std::sqrt(c->hscalar[pd::CG_RES] / bb);
         if (!std::isfinite(rel)) break;
         since = std::max(since, rel);
-        if (f32 && (rel <= rtol || rel < 1e-2 * since)) {
-            // replace: r = b - K x in FP64; p keeps its direction
+        if (f32 && (rel <= rtol || (f32_below > 0.0 && rel < 1e-2 * since))) {
+            // replace: r = b - K x in FP64; p keeps its direction (FP64 matvecs
+            // alone need it only for the verdict)
             true_residual();
             PD_TRY(read());
             rel = std::sqrt(c->hscalar[pd::CG_RES] / bb);
