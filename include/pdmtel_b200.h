@@ -365,8 +365,8 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
                     double* relres);
 
 /* ---- Tuning options (no counterpart in the reference) ----
- * None of them changes a result (PD_OPT_STATIC_PRECOND: beyond the solve's
- * tolerance); they change launch shapes only.
+ * They change launch shapes, not results: exactly, but for the static options
+ * (within the solve's tolerance) and PD_OPT_ADJOINT_VJP32.
  * PD_OPT_F64_LANES_BELOW: the FP64 force runs a warp per node (same
  *   arithmetic, same order) when the problem has fewer nodes than this and
  *   than 12288, eight lanes per node otherwise.  Default 131072.
@@ -392,7 +392,8 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  *   memory.  Reset to 0 whenever the family changes.
  * PD_OPT_FORCE_QUAD: 1 runs the FP32-form force with four nodes per thread
  *   (nodes on one lattice, one material, no critical stretch within reach;
- *   otherwise ignored); 0 (default) with two.
+ *   otherwise ignored); 0 (default) with a lane per bond, the faster one on
+ *   every problem measured.
  * PD_OPT_GATHER_SELL: 1 keeps a sliced-ELLPACK copy of the FP32 gather's
  *   coefficients (16 nodes of the work order side by side per contributor
  *   slot: coalesced loads; 2x2x2 points), which the gather reads when
@@ -446,9 +447,10 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  *   operator until the relative residual is below 1/v, then with the FP32
  *   one (default 10: below 0.1); 0 uses the FP32 operator from the start.
  * PD_OPT_ADJOINT_VJP32: 1 makes the reverse sweep of an FP32C forward run
- *   (pd_adjoint_backward) evaluate its point terms in FP32 (faster; the
- *   family sums of a smooth adjoint cancel, so its gradient is good to about
- *   1e-3); 0 (default) keeps them FP64 on the FP32C tape. */
+ *   (pd_adjoint_backward) evaluate its point terms in FP32 (the family sums of
+ *   a smooth adjoint cancel, so its gradient is good to about 1e-3; slower
+ *   than 0, which evaluates each point once: 6.1 against 4.7 ms per step on the
+ *   64x64x8 specimen); 0 (default) keeps them FP64 on the FP32C tape. */
 enum {
     PD_OPT_F64_LANES_BELOW = 1,
     PD_OPT_TILE = 2,
