@@ -449,7 +449,7 @@ int pd_static_solve(pd_ctx* ctx, double time, int precision, double rtol, int ma
  * PD_OPT_ADJOINT_VJP32: 1 makes the reverse sweep of an FP32C forward run
  *   (pd_adjoint_backward) evaluate its point terms in FP32 (the family sums of
  *   a smooth adjoint cancel, so its gradient is good to about 1e-3; slower
- *   than 0, which evaluates each point once: 6.1 against 4.7 ms per step on the
+ *   than 0, which evaluates each point once: 6.1 against 4.5 ms per step on the
  *   64x64x8 specimen); 0 (default) keeps them FP64 on the FP32C tape. */
 enum {
     PD_OPT_F64_LANES_BELOW = 1,

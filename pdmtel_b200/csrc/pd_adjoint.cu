@@ -309,10 +309,10 @@ __global__ void k_vjp_pack(Dev d, const double* __restrict__ teU, const double* 
 // Two passes of eight lanes per node, a lane per point, evaluated every point
 // twice, gathered 24 displacements per bond in one of them and formed the roots
 // and the division with the library's routines: 0.81 + 0.66 ms for 32,768 nodes
-// (51.1M points); 0.66 ms here and 0.04 in k_vjp_nodes (0.58 with roots and
-// quotients left unrounded).  FP64 pipe 43 % busy at
-// eight warps per SM (254 registers; three blocks at 168 spill and measured the
-// same): bound by the latency of its chains.
+// (51.1M points); 0.61 ms here and 0.04 in k_vjp_nodes (0.58 with roots and
+// quotients a unit or two off, 0.66 with one more step in each).  FP64 pipe 43 %
+// busy at eight warps per SM (254 registers; three blocks at 168 spill and
+// measured the same): bound by the latency of its chains.
 template <int L>
 __global__ void __launch_bounds__(128, 2) k_vjp_bonds(Dev d, const double* __restrict__ rec,
                                                       const double* __restrict__ teug, double* __restrict__ lam_ug,
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(128, 2) k_vjp_bonds(Dev d, const double* __res
             const double r = r2 * rinv, pl = p2 * ip, sum = pl + r;
             // p - r = eta.(2 xi + eta) / (p + r)
             const double q2 = e0 * (x0 + y0) + e1 * (x1 + y1) + e2 * (x2 + y2);
-            const double ext = rn_quotient(q2, sum);
+            const double ext = quotient_near(q2, sum);
             const double st = ext * rinv;
             const double beta = r <= d.delta - 0.5 * G.dxe ? 1.0
                                 : r <= d.delta + 0.5 * G.dxe ? rn_div(d.delta + 0.5 * G.dxe - r, G.dxe, G.ydxe)

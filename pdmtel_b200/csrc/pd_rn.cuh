@@ -59,18 +59,16 @@ __device__ __forceinline__ double rn_rcp(double b, double y0) {
     return fma(fma(-b, y, 1.0), y, y);
 }
 
-// 1 / sqrt(a) within half a unit in the last place and 2^-49 of one, a in
-// rn_range: with e = 1 - a y^2, the root's reciprocal is y (1 + e/2 + 3 e^2/8 +
-// ...); one step of third order from the 20-bit seed, then one of first order
-// whose e has the rounding of a y taken out.
+// 1 / sqrt(a) within half a unit in the last place and 2^-15 of one, a in
+// rn_range: with e = 1 - a y^2 for the seed y, |e| below 2^-18, it is y (1 + e/2 +
+// 3 e^2/8 + 5 e^3/16 + ...), where e has the rounding of a y taken out and is
+// good to 2^-72, and the terms left out are below 2^-73.
 __device__ __forceinline__ double rsqrt_near(double a) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    double e = fma(-(a * y), y, 1.0);
-    y = fma(y * e, fma(0.375, e, 0.5), y);
     const double g = a * y;
-    e = fma(-fma(a, y, -g), y, fma(-g, y, 1.0));
-    return fma(rn_pow2(y, -1), e, y);
+    const double e = fma(-fma(a, y, -g), y, fma(-g, y, 1.0));
+    return fma(y, e * fma(e, fma(e, 0.3125, 0.375), 0.5), y);
 }
 
 // a / b with y = 1/b, b > 0; a zero or rn_quotient_ok (the quotient of a zero
@@ -79,13 +77,14 @@ __device__ __forceinline__ double rn_div(double a, double b, double y) {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
-// a / b without a reciprocal at hand, b > 0 in rn_range; an a outside
-// rn_quotient_ok may end one unit off
-__device__ __forceinline__ double rn_quotient(double a, double b) {
+// a / b without a reciprocal at hand, b > 0 in rn_range, within half a unit in
+// the last place and 2^-49 of one (rn_div's last step on a reciprocal that is
+// rounded from within 2^-59); an a outside rn_quotient_ok may end one unit off
+__device__ __forceinline__ double quotient_near(double a, double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     const double e = fma(-b, y, 1.0);
-    return rn_div(a, b, rn_rcp(b, fma(y, fma(e, e, e), y)));
+    return rn_div(a, b, fma(y, fma(e, e, e), y));
 }
 // the same as rn_div with the sign of a zero kept (any quotient has the sign of a)
 __device__ __forceinline__ double rn_div_signed(double a, double b, double y) {
