@@ -556,7 +556,7 @@ int pd_ctx_create(const pd_problem* P, pd_ctx** out) {
         (rc = dalloc(c, &nblk, (size_t)N * d.bs)) || (rc = dalloc(c, &sblk, (size_t)N * 8)) ||
         (rc = dalloc(c, &order, N)) || (rc = dalloc(c, &eed, N)) ||
         (rc = dalloc(c, &red, 2 * N + 4 + 2 * 160)) || (rc = dalloc(c, &tdev, 1)) ||
-        (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
+        (rc = dalloc(c, &c->dotpart, 2 * (N + 4096))) || (rc = dalloc(c, &c->scal, pd::CG_NSLOT)))
         return bail(rc);
     if (d.cci) try_dalloc(c, &c->ue, 2 * n3);  // without it the epilogues run apart
     if (c->nslit) {
@@ -2359,7 +2359,8 @@ int stencil_prepare(pd_ctx* c) {
     return PD_OK;
 }
 
-// What the summing kernels leave per block, and their counter.
+// What the summing kernels leave per block (made again if it was given back),
+// and their counter.
 int sums_prepare(pd_ctx* c) {
     if (!c->dotpart) PD_TRY(dalloc(c, &c->dotpart, 2 * (c->n + 4096)));
     if (!c->dot_done) {
